@@ -131,7 +131,7 @@ tc_status Workspace::ensure(int64_t n, int64_t m, int64_t extent) {
     TC_TRY(grow(large, c2, items_for(n, m)));
     item_cap = items_for(n, m);
   }
-  TC_TRY(grow(indp, e_cap, std::max(m, extent) + kIndpPad));
+  TC_TRY(grow(indp, e_cap, std::max(m, extent)));
   if (hubs_for(m) > hub_cap) {
     hub_cap = 0;
     int64_t c1 = 0, c2 = 0, c3 = 0;

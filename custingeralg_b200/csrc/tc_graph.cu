@@ -265,7 +265,7 @@ tc_status tc_graph_validate(tc_graph* g, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   TC_TRY(g->ws.ensure(g->n, g->m, g->pool_cap));
   SlackView view{g->start, g->used, g->pool};
-  TC_TRY(validate_view(view, g->n, g->ws, s));
+  TC_TRY(validate_view(view, g->n, g->m, g->ws, s));
   tc_count_info info;
   return read_info(g->ws, s, &info);
 }

@@ -23,14 +23,12 @@ struct TraceRange {
 
 constexpr int kWarp = 32;
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kHubChunk = 2048;     // orientation: list entries per warp work item of a hub
+constexpr int kHubChunk = 2048;     // orientation: most list entries per warp work item of a hub
+constexpr int kHubChunkMin = 512;   // (on small graphs, where a chunk's chain of steps is the tail) and fewest
 constexpr int kHubMin = 256;        // orientation: lists longer than this are oriented as hubs
 static_assert(kHubMin <= kHubChunk, "a hub has at least one chunk");
 constexpr int kWarpTierMax = 128;   // largest out-degree a single warp counts on its own
-constexpr int kItemRangeMin = 256;  // fewest neighbours of a count work item (queue sizing)
-// The count reads oriented lists in aligned 16-byte units, up to 3 entries past a list's end:
-// every oriented-list array holds this many entries past its capacity.
-constexpr int kIndpPad = 4;
+constexpr int kItemRangeMin = 64;   // fewest neighbours of a count work item (queue sizing)
 
 // ---- error reporting -------------------------------------------------------------------
 
@@ -92,7 +90,7 @@ struct SlackView {
 
 // ---- device-side status of one count ---------------------------------------------------
 
-enum : unsigned { kBadRange = 1u, kBadOrder = 2u, kBadSelfLoop = 4u, kBadCapacity = 8u, kBadTimeout = 16u };
+enum : unsigned { kBadRange = 1u, kBadOrder = 2u, kBadSelfLoop = 4u, kBadCapacity = 8u };
 
 struct DevStatus {
   unsigned long long triangles;          // T
@@ -151,6 +149,11 @@ struct SchedParams {
   int32_t lane_max;        // static: lists of at most this many entries are walked by one lane
   int32_t packed_max;      // static: longer lists up to this many entries are walked packed
   int32_t hub_min;         // streaming: changed edges per longer endpoint for the hub count (0 = off)
+  // static count: how the work is cut (set_work_sizes)
+  int32_t cta_range;       // neighbours of a CTA-tier centre per work item
+  int32_t warp_range;      // and of a warp-tier centre
+  int32_t tile;            // vertices per orientation tile (at most 32)
+  int32_t hub_chunk;       // list entries per orientation work item of a hub
   uint8_t table[16][16];
 };
 
@@ -189,9 +192,9 @@ struct Workspace {
   void release();
   // Hub arrays needed for a graph of m directed edges.
   static int64_t hubs_for(int64_t m) { return m / kHubMin + 1; }
-  static int64_t chunks_for(int64_t m) { return m / kHubMin + m / kHubChunk + 2; }
-  // Count work items of one queue: at most one per vertex plus one per kItemRangeMin neighbours.
-  static constexpr int64_t items_for(int64_t n, int64_t m) { return n + m / kItemRangeMin + 1; }
+  static constexpr int64_t chunks_for(int64_t m) { return m / kHubMin + m / kHubChunkMin + 2; }
+  // Count work items of one queue: at most one per vertex plus one per `range` neighbours.
+  static constexpr int64_t items_for(int64_t n, int64_t m, int64_t range = kItemRangeMin) { return n + m / range + 1; }
 };
 
 // Device properties cached per device.
@@ -209,7 +212,7 @@ tc_status static_count(const View& view, int32_t n, int64_t m, Workspace& ws, in
 
 // Structural check only (the first orientation pass). Stream-ordered; read with read_info.
 template <class View>
-tc_status validate_view(const View& view, int32_t n, Workspace& ws, cudaStream_t stream);
+tc_status validate_view(const View& view, int32_t n, int64_t m, Workspace& ws, cudaStream_t stream);
 
 // Phase events of the calling thread (tc_profile_enable). Each is a no-op when disabled.
 void prof_mark(int point, cudaStream_t stream);   // 0 = start, 1 = orientation done, 2 = count done

@@ -29,16 +29,16 @@ constexpr int64_t kMaxNv = TC_NOALLOC_MAX_NV;
 constexpr int64_t kMaxEdges = TC_NOALLOC_MAX_EDGES;
 
 constexpr int64_t kMaxHubs = kMaxEdges / kHubMin + 1;
-constexpr int64_t kMaxChunks = kMaxEdges / kHubMin + kMaxEdges / kHubChunk + 2;
+constexpr int64_t kMaxChunks = Workspace::chunks_for(kMaxEdges);
 
 // Layout (bytes, each part 256-aligned): DevStatus | offp int64[maxnv+1] | dplus, degv
 // int32[maxnv+1] | large, medium uint64[items] | hub_u, hub_base, hub_done int32[hubs]
-// | hub_cnt, chunk_hub int32[chunks] | indp int32[max_edges + kIndpPad]
+// | hub_cnt, chunk_hub int32[chunks] | indp int32[max_edges]
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kOffStatus = 0;
 constexpr size_t kOffOffp = align256(kOffStatus + sizeof(DevStatus));
 constexpr size_t kOffDplus = align256(kOffOffp + sizeof(int64_t) * (kMaxNv + 1));
-constexpr int64_t kMaxItems = Workspace::items_for(kMaxNv, kMaxEdges);
+constexpr int64_t kMaxItems = Workspace::items_for(kMaxNv, kMaxEdges, 256);
 constexpr size_t kOffDegv = align256(kOffDplus + sizeof(int32_t) * (kMaxNv + 1));
 constexpr size_t kOffLarge = align256(kOffDegv + sizeof(int32_t) * (kMaxNv + 1));
 constexpr size_t kOffMedium = align256(kOffLarge + sizeof(unsigned long long) * kMaxItems);
@@ -48,7 +48,7 @@ constexpr size_t kOffHubDone = align256(kOffHubBase + sizeof(int32_t) * kMaxHubs
 constexpr size_t kOffHubCnt = align256(kOffHubDone + sizeof(int32_t) * kMaxHubs);
 constexpr size_t kOffChunkHub = align256(kOffHubCnt + sizeof(int32_t) * kMaxChunks);
 constexpr size_t kOffIndp = align256(kOffChunkHub + sizeof(int32_t) * kMaxChunks);
-constexpr size_t kScratchBytes = align256(kOffIndp + sizeof(int32_t) * (kMaxEdges + kIndpPad));
+constexpr size_t kScratchBytes = align256(kOffIndp + sizeof(int32_t) * kMaxEdges);
 static_assert(kScratchBytes > (size_t(48) << 20) && kScratchBytes < (size_t(49) << 20),
               "the documented size of the no-alloc scratch (about 48.6 MiB) no longer holds");
 

@@ -23,17 +23,17 @@
 //     work is the sum over edges of min(d+u, d+v). k_count is a persistent grid; a centre walks
 //     its original neighbour list N(c) in groups of 32 and takes the neighbours it is centre
 //     for. Tiers by a = d+(c):
-//       CTA   a > warp_max: one CTA per item of 4096 neighbours, N+(c) staged in the full
-//             2048-slot table (load <= 0.25 up to 512 entries) in passes of at most 1024
-//             entries split evenly; a pass holds a value range of N+(c), and each streamed list
-//             is cut to that range by binary search, so no list entry is probed twice;
-//       warp  1 <= a <= warp_max (at most 128): one warp per centre (items of 256 neighbours for
-//             centres with more), a warp-private set of up to 256 slots.
-//     CTAs of 4 warps, 12 resident per SM (40 registers, 16 KB of shared memory each).
+//       CTA   a > warp_max: one CTA per item of up to 4096 neighbours, N+(c) staged in a 2048-slot
+//             table in passes of at most 768 entries split evenly; a pass holds a value range of
+//             N+(c), and each streamed list is cut to that range by binary search, so no list
+//             entry is probed twice;
+//       warp  1 <= a <= warp_max (at most 128): one warp per centre (items of up to 256 neighbours
+//             for centres with more), a warp-private set of up to 512 slots.
+//     CTAs of 4 warps, 10 resident per SM (48 registers, 16.5 KB of shared memory each).
 //     Per edge, the warp streams N+(o) with coalesced loads (four per lane in flight); or, for
 //     short lists, one lane walks it while the other lanes walk theirs; or, for mid-size lists,
-//     the warp walks all such lists of its group of neighbours concatenated (packed); the
-//     scheduler (thresholds or learned per-degree-cell table) picks.
+//     several such lists are walked at once by a few lanes each (packed); the scheduler
+//     (thresholds or learned per-degree-cell table) picks.
 //  3. Attribution. Per-vertex counts never take a global atomic per triangle: the centre's count
 //     stays in registers, the other endpoint's is reduced once per list (one redux.sync), and
 //     the third vertex's is a shared-memory counter beside the hash slot that the probe found;
@@ -54,17 +54,18 @@ namespace tc {
 
 namespace {
 
-constexpr int kThreads = 128;     // 4 warps: small CTAs keep more warps resident per SM
+constexpr int kThreads = 128;      // 4 warps: a CTA's warps wait for one another at each item's end
+                                   // (256 threads on the same table: 6 % slower on R-MAT 20)
 constexpr int kWarps = kThreads / kWarp;
-constexpr int kChunk = 1024;      // A entries staged per pass for an L-tier vertex
-constexpr int kHashMax = 2048;    // hash slots for such a chunk (load <= 0.5)
-constexpr int kUnroll = 4;        // list elements a lane loads before probing (independent loads)
-constexpr int kWarpRange = 256;   // neighbours of a warp-tier centre per work item
-constexpr int kCtaRange = 4096;   // neighbours of a CTA-tier centre per work item
-static_assert(kWarpRange >= kItemRangeMin && kCtaRange >= kItemRangeMin, "queue sizing");
-constexpr int kMedSlots = 2 * kWarpTierMax;  // warp-private hash slots (load <= 0.25 up to a = 64, else <= 0.5)
-// Hash sets are bucketized: 4 slots per 16-byte bucket, probed with one 128-bit shared load,
-// so a lookup ends after one bucket unless that bucket is full (rare at these loads).
+constexpr int kCtasPerSm = 10;     // k_count: 48 registers a thread (12 CTAs at 40 spill: R-MAT 24 + 19 %,
+                                   // BA n = 2^22 + 24 %; 8 CTAs: R-MAT 20 + 8 %)
+constexpr int kHashMaxBits = 11;
+constexpr int kHashMax = 1 << kHashMaxBits;  // hash slots of the CTA tier's table
+constexpr int kChunk = 768;        // entries of N+(c) staged per pass (load <= 3/8)
+constexpr int kWarpSlots = kHashMax / kWarps;  // of a warp-private table (load <= 0.25)
+static_assert(kWarpSlots >= 4 * kWarpTierMax, "load of the warp tables");
+constexpr int kTableBytes = 2 * 4 * kHashMax;  // keys and counters
+constexpr int kUnroll = 4;         // list elements a lane loads before probing (independent loads)
 constexpr int kScanThreads = 256;
 constexpr int kScanPer = 8;
 constexpr int kScanTile = kScanThreads * kScanPer;
@@ -98,79 +99,68 @@ __device__ unsigned long long* tc_dbg_kern = nullptr;
   } while (0)
 #endif
 
-// Hash sets of staged entries of N+(c). The third-vertex counter of an entry sits beside its
-// slot: cnt[s] counts the triangles found through the key hkeys[s], so a hit adds to the slot
-// it found with no indirection. Warp-private set (warp tier):
-struct WarpTable {
-  alignas(16) int32_t hkeys[kMedSlots];
-  uint32_t cnt[kMedSlots];
-};
+// Hash sets of staged entries of N+(c): every entry sits at one of its two slots (cuckoo hashing, one
+// slot in each half of the table, both from one multiplicative hash), so a lookup reads two 4-byte
+// slots and compares twice, with no loop and no divergence. The third-vertex counter of an entry
+// sits beside its slot: cnt[s] counts the triangles found through the key keys[s], so a hit adds
+// to the slot it found with no indirection. A build that finds no place for an entry in kKicks
+// moves fails (at these loads that takes ids chosen against the hash), and the caller stages half
+// as many entries; two entries always fit.
+//
+// The kernel is bound by the instructions around each lookup and by the shared-memory pipe. On R-MAT
+// 20 (1.97 G lookups, 2 t(v) per vertex): 16-byte buckets of four slots, 62 warp instructions per
+// 32 lookups, 4.46 ms; one 4-byte slot with a scan past collisions, which some lane of nearly every
+// row takes, 4.4 ms; two slots 2.65 G instructions and 632 M shared wavefronts, 3.19 ms (total only:
+// 3.87 -> 2.61 ms; CSR weights: 5.39 -> 3.66 ms). R-MAT 24: 180 -> 124 ms for the whole count.
+constexpr int32_t kFreeSlot = -1;
+constexpr int32_t kNoKey = -2;  // an entry that is not there: equals no slot's key
+constexpr int kKicks = 64;
 
-// CTA-shared set of one chunk of a CTA-tier centre's N+(c) (16 KB):
-struct BlockTable {
-  alignas(16) int32_t hkeys[kHashMax];
-  uint32_t cnt[kHashMax];
-};
-
-// Dynamic shared memory of k_count, laid out as CountSmem.
+// Dynamic shared memory of k_count: the tables, then CountSmem. Tables are addressed by 32-bit
+// shared addresses and read and updated with inline ld.shared / red.shared: through C++ pointers
+// the compiler recomputes the block's shared window (a special-register read and two uniform
+// instructions) next to every few accesses.
+constexpr int kWarpTableBytes = kTableBytes / kWarps;
 extern __shared__ __align__(16) unsigned char smem_raw[];
 
 struct CountSmem {
-  union {
-    BlockTable L;
-    WarpTable W[kWarps];
-  } t;
   unsigned long long tri[kWarps];
   unsigned long long item;
-  uint64_t mbar;  // completion of the bulk copy that stages a CTA-tier chunk
   int gctr;
   // Value range [vlo, vhi) of the CTA-tier pass in flight when its centre takes several passes
   // (ranged = 1; 0 for a centre of one pass). Only the CTA tier reads them.
   int ranged;
   int32_t vlo, vhi;
 };
+constexpr size_t kCountSmem = kTableBytes + sizeof(CountSmem);
 
-// ---- bulk copies into shared memory (cp.async.bulk, completion on an mbarrier) ----------------
-
-// Bound of the wait for a staged chunk: it lands within microseconds; a wait that runs out sets
-// kBadTimeout and the CTA stops (after a second bounded wait for its copy in flight).
-constexpr unsigned long long kStageWaitNs = 1000000000ull;  // 1 s
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+__device__ __forceinline__ uint32_t table_base() {
+  uint32_t base;  // kept in a register: the compiler cannot recompute a volatile result
+  asm volatile("mov.u32 %0, %1;" : "=r"(base) : "r"((uint32_t)__cvta_generic_to_shared(smem_raw)));
+  return base;
 }
-
-// Issue one 1-D bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
-// global to shared memory; the mbarrier's phase completes when the bytes have landed.
-__device__ __forceinline__ void stage_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ int32_t lds(const uint32_t at) {
+  int32_t v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(at));
+  return v;
 }
-
-// Wait (bounded by kStageWaitNs of device time) for the mbarrier phase `parity` to complete.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  unsigned long long t0;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (unsigned it = 0; it < (1u << 26); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > kStageWaitNs) break;
-  }
-  return false;
+__device__ __forceinline__ int4 lds4(const uint32_t at) {
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ void sts4(const uint32_t at, const int32_t v) {
+  asm volatile("st.shared.v4.s32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(v) : "memory");
+}
+__device__ __forceinline__ int32_t exchange(const uint32_t at, const int32_t v) {
+  int32_t old;
+  asm volatile("atom.shared.exch.b32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ int lane_id() {
+  int lane;
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  return lane;
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -194,39 +184,52 @@ __device__ __forceinline__ T warp_sum(T x) {
   return x;
 }
 
-__device__ __forceinline__ uint32_t hash_bucket(int32_t key, int bbits) {
-  return ((uint32_t)key * 0x9E3779B1u) >> (32 - bbits);
+// A set of 2 * 2^bits slots, 2^bits in each half, at the shared address keys; its counters lie kCnt
+// bytes after its keys.
+template <int kCnt>
+struct Set {
+  uint32_t keys;
+  int bits;
+  __device__ __forceinline__ int slots() const { return 2 << bits; }
+  // Addresses of the two slots of a key: the top bits of its hash, and the next ones in the upper
+  // half.
+  __device__ __forceinline__ uint32_t slot1(const uint32_t h) const { return ((h >> (30 - bits)) & ~3u) + keys; }
+  __device__ __forceinline__ uint32_t slot2(const uint32_t h) const {
+    return ((h >> (30 - 2 * bits)) & ((4u << bits) - 4u)) + (keys + (4u << bits));
+  }
+};
+using CtaSet = Set<kHashMax * 4>;
+using WarpSet = Set<kWarpSlots * 4>;
+
+__device__ __forceinline__ uint32_t hash_of(const int32_t key) { return (uint32_t)key * 0x9E3779B1u; }
+
+// Insert a key (concurrently with others): into its first slot, the key found there into its other
+// one, and so on; false when a key is left over after kKicks moves.
+template <class S>
+__device__ __forceinline__ bool insert(const S& t, int32_t key) {
+  uint32_t at = t.slot1(hash_of(key));
+  for (int it = 0; it < kKicks; ++it) {
+    key = exchange(at, key);
+    if (key == kFreeSlot) return true;
+    const uint32_t h = hash_of(key), s1 = t.slot1(h);
+    at = at == s1 ? t.slot2(h) : s1;
+  }
+  return false;
 }
 
-// Insert key (unique) into a table of 2^bbits buckets of 4 slots (load <= 0.5, so a bucket with
-// a free slot is always found within 2^bbits steps). Slots of a bucket fill in order and are
-// never freed, so a key that moved on found every slot before it taken.
-__device__ __forceinline__ void hash_insert(int32_t* keys, int bbits, int32_t key) {
-  const uint32_t bmask = (1u << bbits) - 1;
-  uint32_t b = hash_bucket(key, bbits);
-  for (uint32_t it = 0; it <= bmask; ++it) {
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int32_t prev = atomicCAS(&keys[4 * b + t], -1, key);
-      if (prev == -1 || prev == key) return;
-    }
-    b = (b + 1) & bmask;
+// Free slots and zero counters, by `threads` threads of index `at`.
+template <int kCnt>
+__device__ __forceinline__ void clear_set(const Set<kCnt>& t, const int at, const int threads) {
+  for (int s = at; s < t.slots() / 4; s += threads) {
+    sts4(t.keys + 16 * s, kFreeSlot);
+    sts4(t.keys + kCnt + 16 * s, 0);
   }
 }
 
-// Continue a lookup whose first bucket b was full and lacked key: slot of key, or -1.
-__device__ __forceinline__ int hash_find_after(const int32_t* keys, int bbits, int32_t key, uint32_t b) {
-  const uint32_t bmask = (1u << bbits) - 1;
-  for (uint32_t it = 0; it < bmask; ++it) {
-    b = (b + 1) & bmask;
-    const int4 q = *reinterpret_cast<const int4*>(keys + 4 * b);
-    if (q.x == key) return 4 * b;
-    if (q.y == key) return 4 * b + 1;
-    if (q.z == key) return 4 * b + 2;
-    if (q.w == key) return 4 * b + 3;
-    if (q.w == -1) return -1;
-  }
-  return -1;
+// Add x to the shared counter at `at` where `take` holds.
+__device__ __forceinline__ void count_if(const bool take, const uint32_t at, const uint32_t x) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p red.shared.add.u32 [%1], %2; }" ::"r"((unsigned)take),
+               "r"(at), "r"(x));
 }
 
 __device__ __forceinline__ int log2_cell(int x) {
@@ -234,22 +237,10 @@ __device__ __forceinline__ int log2_cell(int x) {
   return min(c, 15);
 }
 
-// Weights a found triangle (u, v, w) adds to each vertex's per-vertex output.
-// TC_PV_HANDLE: 1 each (doubled at flush: out = 2 t(v)).
-// TC_PV_CSR: the reference's raw-CSR kernel counts a triangle at every edge (x, y) with
-// y > x whose lists share the third vertex, crediting x: the smallest id gets 2, the middle 1.
-template <int PV>
-__device__ __forceinline__ void tri_weights(int32_t u, int32_t v, int32_t w, uint32_t& wu, uint32_t& wv,
-                                            uint32_t& ww) {
-  if (PV == TC_PV_CSR) {
-    wu = (u < v) + (u < w);
-    wv = (v < u) + (v < w);
-    ww = (w < u) + (w < v);
-  } else {
-    wu = wv = ww = 1u;
-  }
-}
-
+// Weights of a found triangle in the per-vertex output. Handle conventions: 1 per vertex, doubled
+// at flush (out = 2 t(v)). TC_PV_CSR: the reference's raw-CSR kernel counts a triangle at every
+// edge (x, y) with y > x whose lists share the third vertex, crediting x: the smallest id gets 2,
+// the middle 1.
 template <int PV>
 __host__ __device__ constexpr uint32_t flush_mult() {
   return PV == TC_PV_HANDLE || PV == TC_PV_HANDLE64 ? 2u : 1u;
@@ -278,97 +269,77 @@ __device__ __forceinline__ bool centre_of(int32_t c, int a, int32_t o, int b) {
   return b < a || (b == a && c < o);
 }
 
-// Probe one entry key of the list owned by o into the hash set; returns 1 on a hit. Per hit, the
-// third vertex's counter cnt[slot] gets its weight; vacc and c_acc collect the weights of
-// o and of the centre c (TC_PV_CSR only: in handle mode all weights are 1 and the caller counts
-// the hits instead).
-template <int PV>
-__device__ __forceinline__ uint32_t probe_one(const int32_t key, const int32_t c, const int32_t o,
-                                              const int32_t* hkeys, const int bits, uint32_t* cnt,
-                                              uint32_t& c_acc, uint32_t& vacc) {
-  // First bucket in one 128-bit load; the common case (a miss in a bucket with a free slot)
-  // ends here without computing a slot.
-  const uint32_t bk = hash_bucket(key, bits);
-  const int4 q = *reinterpret_cast<const int4*>(hkeys + 4 * bk);
-  const bool hit = (q.x == key) | (q.y == key) | (q.z == key) | (q.w == key);
-  if (!(hit | (q.w != -1))) return 0;
-  const int s = hit ? (int)(4 * bk) + (q.x == key ? 0 : q.y == key ? 1 : q.z == key ? 2 : 3)
-                    : hash_find_after(hkeys, bits, key, bk);
-  if (s < 0) return 0;
+// What a walk of (part of) one list found: the hits and, for TC_PV_CSR, how many of the third
+// vertices have smaller ids than the centre and than the list's owner (the weights of a triangle
+// depend on the order of its ids alone).
+struct Hits {
+  uint32_t n = 0, below_c = 0, below_o = 0;
+};
+
+// Look up two entries of the list owned by o (kNoKey where there is none); their slots are read
+// before either is counted.
+template <int PV, int kCnt>
+__device__ __forceinline__ void probe2(const int32_t k0, const int32_t k1, const int32_t c, const int32_t o,
+                                       const Set<kCnt>& t, Hits& h) {
+  const uint32_t x0 = hash_of(k0), x1 = hash_of(k1);
+  const uint32_t a0 = t.slot1(x0), b0 = t.slot2(x0), a1 = t.slot1(x1), b1 = t.slot2(x1);
+  const int32_t p0 = lds(a0), q0 = lds(b0), p1 = lds(a1), q1 = lds(b1);
+  const bool f0 = p0 == k0, f1 = p1 == k1;
+  const bool h0 = f0 | (q0 == k0), h1 = f1 | (q1 == k1);
+  h.n += h0;
+  h.n += h1;
   if (handle_like<PV>()) {
-    atomicAdd(&cnt[s], 1u);
+    count_if(h0, (f0 ? a0 : b0) + kCnt, 1u);
+    count_if(h1, (f1 ? a1 : b1) + kCnt, 1u);
   } else if (PV == TC_PV_CSR) {
-    uint32_t wc, wo, ww;
-    tri_weights<PV>(c, o, key, wc, wo, ww);
-    c_acc += wc;
-    vacc += wo;
-    if (ww) atomicAdd(&cnt[s], ww);
+    const uint32_t c0 = h0 & (k0 < c), c1 = h1 & (k1 < c), o0 = h0 & (k0 < o), o1 = h1 & (k1 < o);
+    h.below_c += c0 + c1;
+    h.below_o += o0 + o1;
+    count_if(c0 | o0, (f0 ? a0 : b0) + kCnt, c0 + o0);
+    count_if(c1 | o1, (f1 ? a1 : b1) + kCnt, c1 + o1);
   }
-  return 1;
 }
 
-// The warp streams the list lst[0 .. len) through the hash set with coalesced loads, kUnroll
-// per lane in flight; returns this lane's hits.
+// The weights of a walk's hits for the centre (added to c_acc) and the owner (returned).
 template <int PV>
-__device__ __forceinline__ uint32_t probe_list(const int32_t* __restrict__ lst, const int len, const int32_t c,
-                                               const int32_t o, const int32_t* hkeys, const int bits,
-                                               uint32_t* cnt, uint32_t& c_acc, uint32_t& vacc) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  uint32_t hits = 0;
-  for (int k0 = lane; k0 < len; k0 += kUnroll * kWarp) {
-    int32_t w[kUnroll];
-#pragma unroll
-    for (int j = 0; j < kUnroll; ++j) {
-      const int k = k0 + j * kWarp;
-      w[j] = k < len ? __ldg(lst + k) : -1;
-    }
-#pragma unroll
-    for (int j = 0; j < kUnroll; ++j) {
-      const int32_t key = w[j];
-      if (key < 0) continue;
-      // First bucket in one 128-bit load; the common case (a miss in a bucket with a free
-      // slot) ends here without computing a slot.
-      const uint32_t bk = hash_bucket(key, bits);
-      const int4 q = *reinterpret_cast<const int4*>(hkeys + 4 * bk);
-      const bool hit = (q.x == key) | (q.y == key) | (q.z == key) | (q.w == key);
-      if (hit | (q.w != -1)) {
-        const int s = hit ? (int)(4 * bk) + (q.x == key ? 0 : q.y == key ? 1 : q.z == key ? 2 : 3)
-                          : hash_find_after(hkeys, bits, key, bk);
-        if (s >= 0) {
-          ++hits;
-          if (handle_like<PV>()) {
-            atomicAdd(&cnt[s], 1u);
-          } else if (PV == TC_PV_CSR) {
-            uint32_t wc, wo, ww;
-            tri_weights<PV>(c, o, key, wc, wo, ww);
-            c_acc += wc;
-            vacc += wo;
-            if (ww) atomicAdd(&cnt[s], ww);
-          }
-        }
-      }
-    }
+__device__ __forceinline__ uint32_t credit(const Hits& h, const int32_t c, const int32_t o, uint32_t& tri,
+                                           uint32_t& c_acc) {
+  tri += h.n;
+  if (handle_like<PV>()) {
+    c_acc += h.n;
+    return h.n;
   }
-  return hits;
+  if (PV == TC_PV_CSR) {  // the smallest id of a triangle gets 2, the middle one 1
+    c_acc += h.n * (1u + (c < o)) - h.below_c;
+    return h.n * (1u + (o < c)) - h.below_o;
+  }
+  return 0;
 }
 
-// One lane walks a whole (short) list lst[0 .. len), kUnroll entries in flight; returns the
-// hits. The lanes of a warp walk different lists at once, so short lists do not leave most of
-// the warp idle.
-template <int PV>
-__device__ __forceinline__ uint32_t walk_list(const int32_t* __restrict__ lst, const int len, const int32_t c,
-                                              const int32_t o, const int32_t* hkeys, const int bits,
-                                              uint32_t* cnt, uint32_t& c_acc, uint32_t& vacc) {
-  uint32_t hits = 0;
-  for (int k0 = 0; k0 < len; k0 += kUnroll) {
+// kLanes lanes walk the list lst[0 .. len) together, lane `at` of them taking every kLanes-th
+// entry, kUnroll per lane in flight: the whole warp with coalesced loads (kLanes = 32), or one lane
+// alone (kLanes = 1; the lanes of a warp then walk different short lists at once).
+template <int PV, int kLanes, int kCnt>
+__device__ __forceinline__ void walk_list(const int32_t* __restrict__ lst, const int len, const int at, const int32_t c,
+                                          const int32_t o, const Set<kCnt>& t, Hits& h) {
+  static_assert(kUnroll == 4, "the last step is cut to half of its rows");
+  lst += at;
+  int left = len;
+  for (; left >= kUnroll * kLanes; left -= kUnroll * kLanes, lst += kUnroll * kLanes) {
     int32_t w[kUnroll];
 #pragma unroll
-    for (int j = 0; j < kUnroll; ++j) w[j] = k0 + j < len ? __ldg(lst + k0 + j) : -1;
+    for (int j = 0; j < kUnroll; ++j) w[j] = __ldg(lst + j * kLanes);
 #pragma unroll
-    for (int j = 0; j < kUnroll; ++j)
-      if (w[j] >= 0) hits += probe_one<PV>(w[j], c, o, hkeys, bits, cnt, c_acc, vacc);
+    for (int j = 0; j < kUnroll; j += 2) probe2<PV>(w[j], w[j + 1], c, o, t, h);
   }
-  return hits;
+  if (left > 0) {
+    const int mine = left - at;
+    int32_t w[kUnroll];
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j) w[j] = mine > j * kLanes ? __ldg(lst + j * kLanes) : kNoKey;
+    probe2<PV>(w[0], w[1], c, o, t, h);
+    if (left > 2 * kLanes) probe2<PV>(w[2], w[3], c, o, t, h);
+  }
 }
 
 // First index of the ascending list lst[0 .. len) whose entry is >= key (one lane, binary search).
@@ -386,34 +357,41 @@ __device__ __forceinline__ int lower_bound_list(const int32_t* __restrict__ lst,
   return lo;
 }
 
+// Lanes that walk one packed list. Handle conventions: 4 (8 lists at a time; 8 lanes: BA n = 2^22
+// + 2.6 %); without per-vertex output or with CSR weights 8 (4 lanes: Erdos-Renyi n = 10^6 total
+// + 6 %, R-MAT 20 + 1.5 %).
+template <int PV>
+__host__ __device__ constexpr int pack_lanes() {
+  return handle_like<PV>() ? 4 : 8;
+}
+
 // Lists at most this long are walked whole in a value-range pass (entries outside the pass's
 // range just miss the hash set); longer ones are first cut to the range by two binary searches.
 constexpr int kRangeSearchMin = 32;
 
 // One warp takes the neighbours o = nbr[0 .. gcount) of centre c (out-degree a) and
 // intersects every edge {c, o} whose centre is c: N+(o), the shorter list (b <= a entries), goes
-// through the hash set of the staged chunk of N+(c) (2^bits buckets, cnt[slot] the counter of
-// the key in that slot). Per edge the scheduler picks how (table cell, else the thresholds
-// b <= lane_max, b <= packed_max):
+// through the hash set of the staged chunk of N+(c). Per edge the scheduler picks how (table cell,
+// else the thresholds b <= lane_max, b <= packed_max):
 //   lane:   each such lane walks its own list, all at once (short lists);
-//   packed: the warp walks all such lists of the group concatenated, 32 entries per step (the
-//           owner of an entry by binary search over the lanes' length prefix), so a group of
-//           mid-size lists takes a few rounds of coalesced loads instead of one per list;
+//   packed: several such lists at a time, pack_lanes() lanes each, so mid-size lists neither leave
+//           most of the warp idle nor need a search for the owner of each entry;
 //   warp:   the lists are taken one at a time and the warp streams each with coalesced loads,
 //           so o, its list and its count stay warp-uniform.
 // When the hash set holds only the entries of N+(c) in [vlo, vhi) (one pass of a centre whose
 // N+(c) is larger than a table), only the part of each N+(o) inside that range is walked: both
 // lists are ascending, so no entry outside it can hit. The range sits in shared memory
-// (CountSmem::ranged, vlo, vhi), so it holds no register across the group loop; kMayRange (the
-// CTA tier) compiles the cut in, the warp tiers (one pass always) leave it out.
-template <int PV, bool kMayRange>
+// (CountSmem::ranged, vlo, vhi), so it holds no register across the group loop; the CTA tier
+// compiles the cut in, the warp tiers leave it out.
+template <int PV, int kCnt>
 __device__ __forceinline__ void process_group(const int32_t n, const int32_t c, const int a,
                                               const int32_t* __restrict__ nbr, const int gcount,
-                                              const int32_t* hkeys, const int bits, uint32_t* cnt, const int32_t* __restrict__ dplus,
+                                              const Set<kCnt>& t, const CountSmem& sm, const int lane,
+                                              const int32_t* __restrict__ dplus,
                                               const int64_t* __restrict__ offp, const int32_t* __restrict__ indp,
                                               uint32_t* __restrict__ out, const SchedParams& sp, uint32_t& tri,
                                               uint32_t& c_acc) {
-  const int lane = threadIdx.x & (kWarp - 1);
+  constexpr bool kMayRange = kCnt == kHashMax * 4;  // the CTA tier
   int32_t o = lane < gcount ? __ldg(nbr + lane) : -1;
   const bool valid = o >= 0 && o < n;  // ids out of range were flagged by the orientation
   if (!valid) o = 0;
@@ -421,136 +399,138 @@ __device__ __forceinline__ void process_group(const int32_t n, const int32_t c, 
   const bool mine = valid && b > 0 && centre_of(c, a, o, b) &&
                     (sp.cell_filter == -1 ||
                      (sp.cell_filter >= 0 && log2_cell(a) * 16 + log2_cell(b) == sp.cell_filter));
-  int64_t base = mine ? __ldg(offp + o) : 0;
+  const int32_t* lst = indp + (mine ? __ldg(offp + o) : 0);
   int strat = !mine ? -1
               : sp.use_table ? sp.table[log2_cell(a)][log2_cell(b)]
                              : (b <= sp.lane_max ? 1 : b <= sp.packed_max ? 2 : 0);
-  int len = b;  // entries of N+(o) walked, from indp[base]
-  const CountSmem& sm = *reinterpret_cast<const CountSmem*>(smem_raw);
+  int len = b;  // entries of N+(o) walked, from lst
   if (kMayRange && sm.ranged) {  // uniform over the CTA
     if (strat >= 0 && b > kRangeSearchMin) {
       const int32_t vlo = sm.vlo, vhi = sm.vhi;
-      const int32_t* lst = indp + base;
       const int p0 = vlo == INT_MIN ? 0 : lower_bound_list(lst, b, vlo);
       const int p1 = vhi == INT_MAX ? b : p0 + lower_bound_list(lst + p0, b - p0, vhi);
-      base += p0;
+      lst += p0;
       len = p1 - p0;
       if (len == 0) strat = -1;
     }
     __syncwarp();
   }
   const bool by_lane = strat == 1;
-  const bool by_pack = strat == 2;
   if (__any_sync(kFull, by_lane)) {
     if (by_lane) {
-      uint32_t vacc = 0;
-      const uint32_t hits = walk_list<PV>(indp + base, len, c, o, hkeys, bits, cnt, c_acc, vacc);
-      tri += hits;
-      if (handle_like<PV>()) {
-        c_acc += hits;
-        vacc = hits;
-      }
+      Hits h;
+      walk_list<PV, 1>(lst, len, 0, c, o, t, h);
+      const uint32_t vacc = credit<PV>(h, c, o, tri, c_acc);
       if (PV != TC_PV_NONE && vacc) out_add<PV>(out, o, vacc);
     }
     __syncwarp();
   }
-  if (__any_sync(kFull, by_pack)) {
-    const int len_l = by_pack ? len : 0;
-    int incl = len_l;
-#pragma unroll
-    for (int d = 1; d < kWarp; d <<= 1) {
-      const int y = __shfl_up_sync(kFull, incl, d);
-      if (lane >= d) incl += y;
-    }
-    const int excl_l = incl - len_l;
-    const int total = __shfl_sync(kFull, incl, kWarp - 1);
-    for (int k0 = 0; k0 < total; k0 += kWarp) {
-      const int k = k0 + lane;
-      const bool in = k < total;
-      int i = 0;  // owner lane: the largest i with excl_i <= k (its list is non-empty)
+  const unsigned packed = __ballot_sync(kFull, strat == 2);
+  if (packed) {
+    // the packed lists' fields, moved to the first lanes: lane r holds the r-th such list
+    const int count = __popc(packed);
+    int from = 0;  // position of the lane-th set bit of packed
+    {
+      int r = lane;
 #pragma unroll
       for (int step = kWarp / 2; step > 0; step >>= 1) {
-        const int e = __shfl_sync(kFull, excl_l, i + step);  // i + step <= 31
-        if (e <= k) i += step;
-      }
-      const int64_t pbase = __shfl_sync(kFull, base, i);
-      const int pos = k - __shfl_sync(kFull, excl_l, i);
-      const int32_t po = __shfl_sync(kFull, o, i);
-      const int32_t key = in ? __ldg(indp + pbase + pos) : -1;
-      uint32_t vw = 0;  // o's weight of this entry's triangle
-      const uint32_t h = key >= 0 ? probe_one<PV>(key, c, po, hkeys, bits, cnt, c_acc, vw) : 0u;
-      tri += h;
-      if (handle_like<PV>()) {
-        c_acc += h;
-        vw = h;
-      }
-      if (PV != TC_PV_NONE) {
-        // o's counter: the first lane of each list's segment in this step adds the segment's sum
-        const bool head = in && (pos == 0 || lane == 0);
-        const unsigned heads = __ballot_sync(kFull, head);
-        const unsigned w0 = __ballot_sync(kFull, vw & 1u);
-        const unsigned w1 = PV == TC_PV_CSR ? __ballot_sync(kFull, vw & 2u) : 0u;
-        if (head && (w0 | w1)) {
-          const unsigned above = heads & ~((2u << lane) - 1u);  // heads of later lanes (lane 31: none)
-          const unsigned seg = (above ? (1u << (__ffs(above) - 1)) - 1u : ~0u) & ~((1u << lane) - 1u);
-          const uint32_t sum = __popc(w0 & seg) + 2u * __popc(w1 & seg);
-          if (sum) out_add<PV>(out, po, sum);
+        const int below = __popc((packed >> from) & ((1u << step) - 1u));
+        if (r >= below) {
+          r -= below;
+          from += step;
         }
+      }
+    }
+    constexpr int kPackLanes = pack_lanes<PV>();
+    const int32_t po_l = __shfl_sync(kFull, o, from);
+    const int plen_l = __shfl_sync(kFull, len, from);
+    const unsigned long long plst_l = __shfl_sync(kFull, (unsigned long long)lst, from);
+    for (int r0 = 0; r0 < count; r0 += kWarp / kPackLanes) {
+      const int r = r0 + lane / kPackLanes;
+      const int32_t po = __shfl_sync(kFull, po_l, r);
+      const int32_t* plst = (const int32_t*)__shfl_sync(kFull, plst_l, r);
+      const int plen_r = __shfl_sync(kFull, plen_l, r);
+      const int plen = r < count ? plen_r : 0;
+      Hits h;
+      walk_list<PV, kPackLanes>(plst, plen, lane % kPackLanes, c, po, t, h);
+      __syncwarp();
+      uint32_t vacc = credit<PV>(h, c, po, tri, c_acc);
+      if (PV != TC_PV_NONE) {
+#pragma unroll
+        for (int d = kPackLanes / 2; d > 0; d >>= 1) vacc += __shfl_xor_sync(kFull, vacc, d);
+        if (lane % kPackLanes == 0 && vacc) out_add<PV>(out, po, vacc);
       }
     }
     __syncwarp();
   }
   unsigned todo = __ballot_sync(kFull, strat == 0);
+  uint32_t o_acc = 0;  // what this lane's neighbour gets from its own list's walk
   while (todo) {
     const int sl = __ffs(todo) - 1;
     todo &= todo - 1;
     const int32_t so = __shfl_sync(kFull, o, sl);
     const int sb = __shfl_sync(kFull, len, sl);
-    const int64_t sbase = __shfl_sync(kFull, base, sl);
-    uint32_t vacc = 0;
-    const uint32_t hits = probe_list<PV>(indp + sbase, sb, c, so, hkeys, bits, cnt, c_acc, vacc);
-    tri += hits;
-    if (handle_like<PV>()) {
-      c_acc += hits;
-      vacc = hits;
-    }
+    const int32_t* slst = (const int32_t*)__shfl_sync(kFull, (unsigned long long)lst, sl);
+    Hits h;
+    walk_list<PV, kWarp>(slst, sb, lane, c, so, t, h);
+    __syncwarp();
+    uint32_t vacc = credit<PV>(h, c, so, tri, c_acc);
     if (PV != TC_PV_NONE) {
       vacc = __reduce_add_sync(kFull, vacc);
-      if (lane == 0 && vacc) out_add<PV>(out, so, vacc);
+      if (lane == sl) o_acc = vacc;
     }
   }
+  if (PV != TC_PV_NONE && o_acc) out_add<PV>(out, o, o_acc);
   __syncwarp();
+}
+
+// Flush a set's counters into the per-vertex output, by `threads` threads of index `at`.
+template <int PV, int kCnt>
+__device__ __forceinline__ void flush_set(const Set<kCnt>& t, const int at, const int threads, uint32_t* __restrict__ out) {
+  for (int s = at; s < t.slots() / 4; s += threads) {
+    const int4 x = lds4(t.keys + kCnt + 16 * s);
+    if (!(x.x | x.y | x.z | x.w)) continue;
+    const int4 k = lds4(t.keys + 16 * s);
+    if (x.x) out_add<PV>(out, k.x, x.x);
+    if (x.y) out_add<PV>(out, k.y, x.y);
+    if (x.z) out_add<PV>(out, k.z, x.z);
+    if (x.w) out_add<PV>(out, k.w, x.w);
+  }
 }
 
 // One warp counts the edges of centre c (out-degree a <= kWarpTierMax) among its neighbours
 // N(c)[k0 .. k1).
 template <int PV>
 __device__ __forceinline__ void warp_centre(const int32_t n, const int32_t c, const int a, const int64_t start,
-                                            const int k0, const int k1, WarpTable& t,
+                                            const int k0, const int k1, const uint32_t table,
+                                            const CountSmem& sm, const int lane,
                                             const int32_t* __restrict__ ind, const int32_t* __restrict__ dplus,
                                             const int64_t* __restrict__ offp, const int32_t* __restrict__ indp,
                                             uint32_t* __restrict__ out, const SchedParams& sp, uint32_t& tri) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  int bits = 4;  // buckets: 4 * 2^bits slots >= 4a (load <= 0.25) while they fit in kMedSlots
-  while ((1 << bits) < a && (8 << bits) <= kMedSlots) ++bits;
-  const int S = 4 << bits;
-  for (int s = lane; s < S; s += kWarp) {
-    t.hkeys[s] = -1;
-    t.cnt[s] = 0;
-  }
-  __syncwarp();
-  for (int j = lane; j < a; j += kWarp) hash_insert(t.hkeys, bits, __ldg(indp + start + j));
-  __syncwarp();
+  int bits = 6;  // 2^(bits + 1) slots, at least 4a (load <= 0.25; one 16-byte store per lane clears 128)
+  while ((2 << bits) < 4 * a && (2 << bits) < kWarpSlots) ++bits;
+  const WarpSet t{table, bits};
   uint32_t c_acc = 0;
-  for (int g = k0; g < k1; g += kWarp)
-    process_group<PV, false>(n, c, a, ind + start + g, min(kWarp, k1 - g), t.hkeys, bits, t.cnt, dplus, offp, indp,
-                             out, sp, tri, c_acc);
-  if (PV != TC_PV_NONE) {
-    for (int s = lane; s < S; s += kWarp) {
-      const uint32_t x = t.cnt[s];
-      if (x) out_add<PV>(out, t.hkeys[s], x);
+  int clen = a;  // entries staged at a time: all of them, fewer only after a failed build
+  for (int cb = 0; cb < a; cb += clen) {
+    clen = min(clen, a - cb);
+    while (true) {
+      clear_set(t, lane, kWarp);
+      __syncwarp();
+      bool ok = true;
+      for (int j = lane; j < clen; j += kWarp) ok &= insert(t, __ldg(indp + start + cb + j));
+      __syncwarp();
+      if (__all_sync(kFull, ok)) break;
+      clen = (clen + 1) / 2;
     }
-    __syncwarp();
+    for (int g = k0; g < k1; g += kWarp)
+      process_group<PV>(n, c, a, ind + start + g, min(kWarp, k1 - g), t, sm, lane, dplus, offp, indp, out, sp, tri, c_acc);
+    if (PV != TC_PV_NONE) {
+      flush_set<PV>(t, lane, kWarp, out);
+      __syncwarp();
+    }
+  }
+  if (PV != TC_PV_NONE) {
     c_acc = __reduce_add_sync(kFull, c_acc);
     if (lane == 0 && c_acc) out_add<PV>(out, c, c_acc);
   }
@@ -563,7 +543,7 @@ __device__ __forceinline__ unsigned long long make_item(int32_t c, int32_t k0) {
 }
 
 template <int PV>
-__global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const int32_t* __restrict__ ind,
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) k_count(const int32_t n, const int32_t* __restrict__ ind,
                                                     const int32_t* __restrict__ degv,
                                                     const int32_t* __restrict__ dplus,
                                                     const int64_t* __restrict__ offp,
@@ -573,22 +553,18 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
                                                     uint32_t* __restrict__ out, DevStatus* __restrict__ st,
                                                     const SchedParams sp) {
   TC_DBG_ENTER(6);
-  CountSmem& sm = *reinterpret_cast<CountSmem*>(smem_raw);
-  const int lane = threadIdx.x & (kWarp - 1);
+  const uint32_t table = table_base();
+  CountSmem& sm = *reinterpret_cast<CountSmem*>(smem_raw + kTableBytes);
+  const int lane = lane_id();
   const int wid = threadIdx.x / kWarp;
   uint32_t tri = 0;
   const unsigned n_large = st->n_large;
   const unsigned n_medium = st->n_medium;
 
-  // CTA tier: one CTA per item (centre with a > warp_max, kCtaRange of its neighbours), over
-  // chunks of kChunk entries of N+(c), each staged into shared memory by one bulk copy.
-  BlockTable& L = sm.t.L;
-  if (threadIdx.x == 0) {
-    mbar_init(&sm.mbar);
-    sm.ranged = 0;
-  }
-  __syncthreads();
-  uint32_t stage_phase = 0;
+  // CTA tier: one CTA per item (centre with a > warp_max, sp.cta_range of its neighbours), over
+  // chunks of kChunk entries of N+(c).
+  const CtaSet L{table, kHashMaxBits - 1};
+  if (threadIdx.x == 0) sm.ranged = 0;
   while (true) {
     if (threadIdx.x == 0) {
       const unsigned q = atomicAdd(&st->q_large, 1u);
@@ -603,50 +579,39 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
     const int32_t k0 = (int32_t)(uint32_t)item;
     const int32_t a = dplus[c];
     const int64_t start = offp[c];
-    const int32_t k1 = min(degv[c], k0 + kCtaRange);
+    const int32_t k1 = min(degv[c], k0 + sp.cta_range);
     uint32_t c_acc = 0;
-    // N+(c) in passes of at most kChunk entries, split evenly; pass pk holds the entries of N+(c)
-    // in [vlo, vhi), and only that part of each streamed list is walked in it.
+    // N+(c) in passes of at most kChunk entries, split evenly; a pass holds the entries of N+(c) in
+    // [vlo, vhi), and only that part of each streamed list is walked in it.
     const int passes = (a + kChunk - 1) / kChunk;
-    for (int pk = 0; pk < passes; ++pk) {
-      const int cb = (int)(((int64_t)pk * a) / passes);
-      const int cb_next = (int)(((int64_t)(pk + 1) * a) / passes);
-      const int clen = cb_next - cb;
-      // the whole table whatever clen: load clen / kHashMax (<= 0.25 up to 512 entries, <= 0.5)
-      constexpr int bits = 9;
-      static_assert((4 << bits) == kHashMax, "CTA table size");
-      const int S = 4 << bits;
-      // Stage N+(c)[cb, cb + clen) in the counter half of the table (cleared after the build):
-      // one bulk copy of the 16-byte units that cover it (at most clen + 3 entries, inside the
-      // list or the array's padding), issued while the threads clear the keys.
-      const int64_t gs = start + cb, ga = gs & ~int64_t(3);
-      const int skip = (int)(gs - ga);
-      static_assert(sizeof(L.cnt) >= sizeof(int32_t) * (kChunk + 4), "staging area");
-      int32_t* stage = reinterpret_cast<int32_t*>(L.cnt);
-      if (threadIdx.x == 0) {
-        sm.gctr = 0;
-        stage_bulk(stage, indp + ga, (uint32_t)(((skip + clen + 3) & ~3) * sizeof(int32_t)), &sm.mbar);
+    int clen = (a + passes - 1) / passes;
+    for (int cb = 0; cb < a; cb += clen) {
+      clen = min(clen, a - cb);
+      while (true) {
+        // this thread's entries, in flight while the table is cleared
+        int32_t mine[kChunk / kThreads];
+#pragma unroll
+        for (int j = 0; j < kChunk / kThreads; ++j) {
+          const int e = (int)threadIdx.x + j * kThreads;
+          mine[j] = e < clen ? __ldg(indp + start + cb + e) : kNoKey;
+        }
+        clear_set(L, threadIdx.x, kThreads);
+        if (threadIdx.x == 0) {
+          sm.gctr = 0;
+          sm.ranged = clen < a;
+          sm.vlo = cb == 0 ? INT_MIN : mine[0];
+          sm.vhi = cb + clen == a ? INT_MAX : __ldg(indp + start + cb + clen);
+        }
+        __syncwarp();
+        __syncthreads();
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < kChunk / kThreads; ++j)
+          if (mine[j] != kNoKey) ok &= insert(L, mine[j]);
+        __syncwarp();
+        if (__syncthreads_and(ok)) break;
+        clen = (clen + 1) / 2;
       }
-      for (int s = threadIdx.x; s < S; s += kThreads) L.hkeys[s] = -1;
-      const bool landed = mbar_wait(&sm.mbar, stage_phase);
-      stage_phase ^= 1u;
-      if (__syncthreads_or(!landed)) {
-        // the copy did not land in time: report it, wait once more for it, stop this CTA
-        if (threadIdx.x == 0) atomicOr(&st->bad_flags, kBadTimeout);
-        mbar_wait(&sm.mbar, stage_phase ^ 1u);
-        return;
-      }
-      if (threadIdx.x == 0) {
-        sm.ranged = passes > 1;
-        sm.vlo = pk == 0 ? INT_MIN : stage[skip];
-        sm.vhi = pk + 1 == passes ? INT_MAX : __ldg(indp + start + cb_next);
-      }
-      for (int j = threadIdx.x; j < clen; j += kThreads) hash_insert(L.hkeys, bits, stage[skip + j]);
-      __syncwarp();
-      __syncthreads();
-      for (int s = threadIdx.x; s < S; s += kThreads) L.cnt[s] = 0;
-      __syncwarp();
-      __syncthreads();
       const int ngroups = (k1 - k0 + kWarp - 1) / kWarp;
       while (true) {
         int g = 0;
@@ -655,17 +620,13 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
         g = __shfl_sync(kFull, g, 0);
         if (g >= ngroups) break;
         const int gk = k0 + g * kWarp;
-        process_group<PV, true>(n, c, a, ind + start + gk, min(kWarp, k1 - gk), L.hkeys, bits, L.cnt, dplus, offp,
-                                indp, out, sp, tri, c_acc);
+        process_group<PV>(n, c, a, ind + start + gk, min(kWarp, k1 - gk), L, sm, lane, dplus, offp, indp, out, sp, tri,
+                                c_acc);
       }
       __syncwarp();
       __syncthreads();
-      if (PV != TC_PV_NONE) {
-        for (int s = threadIdx.x; s < S; s += kThreads) {
-          const uint32_t x = L.cnt[s];
-          if (x) out_add<PV>(out, L.hkeys[s], x);
-        }
-      }
+      if (PV != TC_PV_NONE)
+        flush_set<PV>(L, threadIdx.x, kThreads, out);
       __syncwarp();
       __syncthreads();
     }
@@ -677,9 +638,9 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
   }
 
   // From here every warp works alone, on its own slice of the (now free) staging area.
-  WarpTable& W = sm.t.W[wid];
+  const uint32_t W = table + wid * kWarpTableBytes;
 
-  // Warp tier, centres with many neighbours: one warp per item (kWarpRange neighbours).
+  // Warp tier, centres with many neighbours: one warp per item (sp.warp_range neighbours).
   while (true) {
     unsigned long long item = ~0ull;
     if (lane == 0) {
@@ -693,11 +654,11 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
     const int32_t k0 = (int32_t)(uint32_t)item;
     const int a = __ldg(dplus + c);
     const int64_t start = __ldg(offp + c);
-    const int k1 = min(__ldg(degv + c), k0 + kWarpRange);
-    warp_centre<PV>(n, c, a, start, k0, k1, W, ind, dplus, offp, indp, out, sp, tri);
+    const int k1 = min(__ldg(degv + c), k0 + sp.warp_range);
+    warp_centre<PV>(n, c, a, start, k0, k1, W, sm, lane, ind, dplus, offp, indp, out, sp, tri);
   }
 
-  // Warp tier, the rest (1 <= a <= warp_max, degree <= kWarpRange): one warp per centre,
+  // Warp tier, the rest (1 <= a <= warp_max, degree <= sp.warp_range): one warp per centre,
   // claimed in chunks of vertex ids.
   while (true) {
     unsigned long long c0 = 0;
@@ -715,14 +676,14 @@ __global__ void __launch_bounds__(kThreads, 12) k_count(const int32_t n, const i
       const int aa = in ? __ldg(dplus + uu) : 0;
       const int dd = in ? __ldg(degv + uu) : 0;
       unsigned elig = __ballot_sync(
-          kFull, aa >= 1 && aa <= sp.warp_max && dd <= kWarpRange && (!sharded || (uu >= s_lo && uu < s_hi)));
+          kFull, aa >= 1 && aa <= sp.warp_max && dd <= sp.warp_range && (!sharded || (uu >= s_lo && uu < s_hi)));
       while (elig) {
         const int sl = __ffs(elig) - 1;
         elig &= elig - 1;
         const int32_t c = ub + sl;
         const int a = __shfl_sync(kFull, aa, sl);
         const int d = __shfl_sync(kFull, dd, sl);
-        warp_centre<PV>(n, c, a, __ldg(offp + c), 0, d, W, ind, dplus, offp, indp, out, sp, tri);
+        warp_centre<PV>(n, c, a, __ldg(offp + c), 0, d, W, sm, lane, ind, dplus, offp, indp, out, sp, tri);
       }
     }
   }
@@ -818,7 +779,8 @@ __global__ void __launch_bounds__(256) k_find_hubs(const View g, const int32_t n
                                                    int32_t* __restrict__ hub_u,
                                                    int32_t* __restrict__ hub_base, int32_t* __restrict__ hub_done,
                                                    int32_t* __restrict__ chunk_hub, const int64_t hub_cap,
-                                                   const int64_t chunk_cap, DevStatus* __restrict__ st) {
+                                                   const int64_t chunk_cap, const int32_t hub_chunk,
+                                                   DevStatus* __restrict__ st) {
   for (int64_t uu = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; uu < n; uu += (int64_t)gridDim.x * blockDim.x) {
     const int32_t u = (int32_t)uu;
     const int32_t d = g.len(u);
@@ -826,7 +788,7 @@ __global__ void __launch_bounds__(256) k_find_hubs(const View g, const int32_t n
     dplus[u] = 0;
     offp[u] = 0;
     degv[u] = 0;
-    const int nch = (d + kHubChunk - 1) / kHubChunk;
+    const int nch = (d + hub_chunk - 1) / hub_chunk;
     const unsigned h = atomicAdd(&st->n_hubs, 1u);
     const unsigned base = atomicAdd(&st->n_hub_chunks, (unsigned)nch);
     const bool ok = h < hub_cap && (int64_t)base + nch <= chunk_cap;
@@ -853,7 +815,8 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
                                                 const int32_t* __restrict__ hub_u,
                                                 const int32_t* __restrict__ hub_base, int32_t* __restrict__ hub_cnt,
                                                 int32_t* __restrict__ hub_done, const int32_t* __restrict__ chunk_hub,
-                                                const int64_t hub_cap, const int64_t chunk_cap, DevStatus* __restrict__ st) {
+                                                const int64_t hub_cap, const int64_t chunk_cap, const int32_t hub_chunk,
+                                                const int32_t tile, DevStatus* __restrict__ st) {
   const int lane = threadIdx.x & (kWarp - 1);
   const unsigned nchunks = (unsigned)min((long long)st->n_hub_chunks, (long long)chunk_cap);
   const unsigned nhubs = (unsigned)min((long long)st->n_hubs, (long long)hub_cap);
@@ -874,14 +837,14 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
     const int32_t u = hub_u[h];
     const int64_t s = g.start(u);
     const int32_t d = g.len(u);
-    const int nch = (d + kHubChunk - 1) / kHubChunk;
+    const int nch = (d + hub_chunk - 1) / hub_chunk;
     const int c = (int)q - hb;
     if (c < 0 || c >= nch) continue;
     if (s < 0 || s + d > e_cap) {
       bad |= kBadCapacity;
       continue;
     }
-    const int32_t k_begin = c * kHubChunk, k_end = min(d, k_begin + kHubChunk);
+    const int32_t k_begin = c * hub_chunk, k_end = min(d, k_begin + hub_chunk);
     const int cnt = orient_range<View, kWrite>(g, n, u, d, s, k_begin, k_end, indp, s + k_begin, chk, bad);
     // Publish this chunk (entries written by every lane, then its count), then count it done.
     if (lane == 0) hub_cnt[q] = cnt;
@@ -899,7 +862,7 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
     for (int cc = 0; cc < nch; ++cc) {
       const int cn = __ldcg(hub_cnt + hb + cc);
       if (kWrite && cc > 0 && cn > 0) {
-        const int64_t src = s + (int64_t)cc * kHubChunk, dst = s + a;
+        const int64_t src = s + (int64_t)cc * hub_chunk, dst = s + a;
         for (int k0 = 0; k0 < cn; k0 += kWarp) {
           const int k = k0 + lane;
           const int32_t x = k < cn ? __ldcg(indp + src + k) : 0;
@@ -914,7 +877,7 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
   }
 
   // Vertex tiles (hubs skipped: done above). The warp walks the concatenated lists of a tile's
-  // 32 vertices, 32 entries per step: short lists leave no lane idle, and a step is one round of
+  // vertices (at most 32), 32 entries per step: short lists leave no lane idle, and a step is one round of
   // coalesced loads instead of one dependent round per vertex. Lane i keeps vertex t0 + i; the
   // owner of entry k is the last vertex whose list starts at or before k (a binary search over
   // the lanes' exclusive prefix of the lengths). An out-neighbour's rank in N+(u) is its vertex's
@@ -925,12 +888,12 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
   const unsigned lt = lanemask_lt();
   while (true) {
     unsigned t0 = 0;
-    if (lane == 0) t0 = atomicAdd(&st->q_orient_vtx, (unsigned)kTile);
+    if (lane == 0) t0 = atomicAdd(&st->q_orient_vtx, (unsigned)tile);
     __syncwarp();
     t0 = __shfl_sync(kFull, t0, 0);
     if (t0 >= (unsigned)n) break;
     const int32_t u_l = (int32_t)t0 + lane;
-    const bool in_t = u_l < n;
+    const bool in_t = lane < tile && u_l < n;
     const int32_t d_l = in_t ? g.len(u_l) : 0;
     const int64_t s_l = in_t ? g.start(u_l) : 0;
     const bool own_l = in_t && d_l <= kHubMin;  // hubs were completed by the chunk loop
@@ -1022,17 +985,17 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
 }
 
 // The count's work queues, filled after the orientation. A centre with out-degree a > warp_max
-// gets CTA items of kCtaRange neighbours; one with a <= warp_max and more than kWarpRange
-// neighbours gets warp items of kWarpRange (the other centres are claimed by id ranges). The CTA
+// gets CTA items of cta_range neighbours; one with a <= warp_max and more than warp_range
+// neighbours gets warp items of warp_range (the other centres are claimed by id ranges). The CTA
 // queue is ordered by estimated item work, largest first, so the persistent grid does not end
-// on a few long items: the work class of a centre's items is log2(a * min(d, kCtaRange)), and
+// on a few long items: the work class of a centre's items is log2(a * min(d, cta_range)), and
 // classes are laid out in decreasing order, each in vertex-id order (which on R-MAT keeps
 // centres with shared neighbours together). k_push_items counts the items per class and fills
 // the warp queue; k_fill_items places the CTA items.
 constexpr int kWorkClasses = 32;
 
-__device__ __forceinline__ int work_class(const int32_t a, const int32_t d) {
-  const unsigned long long w = (unsigned long long)a * (unsigned long long)min(d, kCtaRange);
+__device__ __forceinline__ int work_class(const int32_t a, const int32_t d, const int32_t range) {
+  const unsigned long long w = (unsigned long long)a * (unsigned long long)min(d, range);
   return min(kWorkClasses - 1, 63 - __clzll(max(w, 1ull)));
 }
 
@@ -1049,7 +1012,8 @@ __device__ __forceinline__ bool cta_centre(const DevStatus* __restrict__ st, con
 __global__ void __launch_bounds__(256) k_push_items(const int32_t n, const int32_t* __restrict__ dplus,
                                                     const int32_t* __restrict__ degv,
                                                     unsigned long long* __restrict__ medium, const int64_t item_cap,
-                                                    DevStatus* __restrict__ st, const int warp_max) {
+                                                    DevStatus* __restrict__ st, const int warp_max,
+                                                    const int cta_range, const int warp_range) {
   const int lane = threadIdx.x & (kWarp - 1);
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) / kWarp;
   unsigned bad = 0;
@@ -1060,9 +1024,9 @@ __global__ void __launch_bounds__(256) k_push_items(const int32_t n, const int32
     const int32_t a = in ? dplus[u] : 0;
     const int32_t d = in ? degv[u] : 0;
     if (in && cta_centre(st, u, a, warp_max))
-      atomicAdd(&st->cls_cnt[work_class(a, d)], (unsigned)((d + kCtaRange - 1) / kCtaRange));
-    const bool wrp = in && a > 0 && a <= warp_max && d > kWarpRange && in_shard(st, u);
-    const int x = wrp ? (d + kWarpRange - 1) / kWarpRange : 0;
+      atomicAdd(&st->cls_cnt[work_class(a, d, cta_range)], (unsigned)((d + cta_range - 1) / cta_range));
+    const bool wrp = in && a > 0 && a <= warp_max && d > warp_range && in_shard(st, u);
+    const int x = wrp ? (d + warp_range - 1) / warp_range : 0;
     int incl = x;
 #pragma unroll
     for (int o = 1; o < kWarp; o <<= 1) {
@@ -1078,7 +1042,7 @@ __global__ void __launch_bounds__(256) k_push_items(const int32_t n, const int32
       bad |= kBadCapacity;
       continue;
     }
-    for (int j = 0; j < x; ++j) medium[base + (incl - x) + j] = make_item(u, j * kWarpRange);
+    for (int j = 0; j < x; ++j) medium[base + (incl - x) + j] = make_item(u, j * warp_range);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) bad |= __shfl_xor_sync(kFull, bad, o);
@@ -1088,7 +1052,8 @@ __global__ void __launch_bounds__(256) k_push_items(const int32_t n, const int32
 __global__ void __launch_bounds__(256) k_fill_items(const int32_t n, const int32_t* __restrict__ dplus,
                                                     const int32_t* __restrict__ degv,
                                                     unsigned long long* __restrict__ large, const int64_t item_cap,
-                                                    DevStatus* __restrict__ st, const int warp_max) {
+                                                    DevStatus* __restrict__ st, const int warp_max,
+                                                    const int cta_range, const int warp_range) {
   __shared__ unsigned cls_base[kWorkClasses];
   __shared__ unsigned total;
   if (threadIdx.x < kWarp) {
@@ -1115,11 +1080,11 @@ __global__ void __launch_bounds__(256) k_fill_items(const int32_t n, const int32
     const int32_t a = dplus[u];
     if (!cta_centre(st, u, a, warp_max)) continue;
     const int32_t d = degv[u];
-    const int cls = work_class(a, d);
-    const int nit = (d + kCtaRange - 1) / kCtaRange;
+    const int cls = work_class(a, d, cta_range);
+    const int nit = (d + cta_range - 1) / cta_range;
     const unsigned at = cls_base[cls] + atomicAdd(&st->cls_pos[cls], (unsigned)nit);
     if ((int64_t)at + nit > (int64_t)n_items) continue;  // only past a capacity error
-    for (int j = 0; j < nit; ++j) large[at + j] = make_item(u, j * kCtaRange);
+    for (int j = 0; j < nit; ++j) large[at + j] = make_item(u, j * cta_range);
   }
 }
 
@@ -1277,7 +1242,7 @@ tc_status launch_count(int32_t n, const int32_t* ind, const Workspace& ws, uint3
                        cudaStream_t stream) {
   constexpr int kMaxDev = 64;
   static int blocks_per_sm[kMaxDev] = {};  // 0 = not configured on that device yet
-  const size_t smem = sizeof(CountSmem);
+  const size_t smem = kCountSmem;
   int dev = 0;
   TC_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDev) return fail(TC_ERR_INVALID_ARG, "device %d out of range", dev);
@@ -1318,7 +1283,7 @@ tc_status resident_grid(int threads, int* grid) {
 template <class View>
 tc_status orient(const View& view, int32_t n, Workspace& ws, const SchedParams& sp, bool write, cudaStream_t stream) {
   k_find_hubs<View><<<hubs_grid(n), 256, 0, stream>>>(view, n, ws.dplus, ws.offp, ws.degv, ws.hub_u, ws.hub_base,
-                                                      ws.hub_done, ws.chunk_hub, ws.hub_cap, ws.chunk_cap, ws.st);
+                                                      ws.hub_done, ws.chunk_hub, ws.hub_cap, ws.chunk_cap, sp.hub_chunk, ws.st);
   TC_CUDA_TRY(cudaGetLastError());
   int grid = 0;
   if (write) TC_TRY((resident_grid<k_orient<View, true>>(256, &grid)));
@@ -1326,11 +1291,11 @@ tc_status orient(const View& view, int32_t n, Workspace& ws, const SchedParams& 
   if (write)
     k_orient<View, true><<<grid, 256, 0, stream>>>(view, n, ws.dplus, ws.offp, ws.degv, ws.indp, ws.e_cap,
                                                    ws.hub_u, ws.hub_base, ws.hub_cnt, ws.hub_done, ws.chunk_hub,
-                                                   ws.hub_cap, ws.chunk_cap, ws.st);
+                                                   ws.hub_cap, ws.chunk_cap, sp.hub_chunk, sp.tile, ws.st);
   else
     k_orient<View, false><<<grid, 256, 0, stream>>>(view, n, ws.dplus, ws.offp, ws.degv, ws.indp, ws.e_cap,
                                                     ws.hub_u, ws.hub_base, ws.hub_cnt, ws.hub_done, ws.chunk_hub,
-                                                    ws.hub_cap, ws.chunk_cap, ws.st);
+                                                    ws.hub_cap, ws.chunk_cap, sp.hub_chunk, sp.tile, ws.st);
   TC_CUDA_TRY(cudaGetLastError());
   if (write) {
     if (sp.nshards > 1) {
@@ -1344,9 +1309,11 @@ tc_status orient(const View& view, int32_t n, Workspace& ws, const SchedParams& 
       TC_CUDA_TRY(cudaGetLastError());
     }
     // the count's work queues (only a count reads them)
-    k_push_items<<<hubs_grid(n), 256, 0, stream>>>(n, ws.dplus, ws.degv, ws.medium, ws.item_cap, ws.st, sp.warp_max);
+    k_push_items<<<hubs_grid(n), 256, 0, stream>>>(n, ws.dplus, ws.degv, ws.medium, ws.item_cap, ws.st, sp.warp_max,
+                                              sp.cta_range, sp.warp_range);
     TC_CUDA_TRY(cudaGetLastError());
-    k_fill_items<<<hubs_grid(n), 256, 0, stream>>>(n, ws.dplus, ws.degv, ws.large, ws.item_cap, ws.st, sp.warp_max);
+    k_fill_items<<<hubs_grid(n), 256, 0, stream>>>(n, ws.dplus, ws.degv, ws.large, ws.item_cap, ws.st, sp.warp_max,
+                                              sp.cta_range, sp.warp_range);
     TC_CUDA_TRY(cudaGetLastError());
   }
   return TC_OK;
@@ -1391,9 +1358,34 @@ SchedParams to_params(const tc_sched* s) {
   return p;
 }
 
+// How a count's work is cut. On a graph that keeps every warp busy for long the pieces are large
+// (fewer grabs and table builds); on a small one (below 2^23 directed edges, where a count takes
+// under about half a millisecond) a large piece is the tail: one warp's chain of dependent steps.
+// Measured on R-MAT 16 (1.8 M directed edges): centres claimed 5 instead of 64 at a time 527 -> 291 us
+// for the whole count, items of 512 and 64 edges instead of 4096 and 256 -> 264 us, orientation tiles
+// of 8 vertices instead of 32 and hub chunks of 512 entries -> 222 us. On R-MAT 20 the same small items
+// cost 1 % and tiles of 8 nothing, on Barabasi-Albert n = 2^22 3 % and 2 %.
+void set_work_sizes(SchedParams& sp, int64_t n, int64_t m, int64_t item_cap) {
+  const bool small = m < (int64_t)1 << 23;
+  sp.cta_range = small ? 512 : 4096;
+  sp.warp_range = small && item_cap >= Workspace::items_for(n, m, 64) ? 64 : 256;
+  sp.hub_chunk = small ? kHubChunkMin : kHubChunk;
+  // Vertices claimed at a time: at least two claims per warp, at most 16 (64: R-MAT 20 + 2 %,
+  // Erdos-Renyi n = 2^20 + 6 %; 1: 16384 vertices + 2 %, 90601 + 25 %).
+  const int64_t warps = (int64_t)device_info().sms * kCtasPerSm * kWarps;
+  sp.chunk = (int32_t)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sp.chunk, 16, n / (2 * warps)}));
+  // Orientation tiles: 32 vertices, or on a graph of fewer tiles than warps as many as hold about 128
+  // entries (four steps).
+  sp.tile = kWarp;
+  if (n < kWarp * warps)
+    while (sp.tile > 4 && (int64_t)sp.tile / 2 * m >= 128 * n) sp.tile /= 2;
+}
+
 template <class View>
 tc_status static_count(const View& view, int32_t n, int64_t m, Workspace& ws, int pv_mode, int32_t* per_vertex,
-                       int64_t* triangles_dev, const SchedParams& sp, cudaStream_t stream) {
+                       int64_t* triangles_dev, const SchedParams& sp0, cudaStream_t stream) {
+  SchedParams sp = sp0;
+  set_work_sizes(sp, n, m, ws.item_cap);
   if (sp.nshards > 1 && n > 0) TC_TRY(ws.ensure_shards(n));
   TC_CUDA_TRY(cudaMemsetAsync(ws.st, 0, sizeof(DevStatus), stream));
   if (pv_mode != TC_PV_NONE && n > 0)
@@ -1450,10 +1442,6 @@ tc_status read_info(const Workspace& ws, cudaStream_t stream, tc_count_info* inf
     info->status = TC_ERR_CAPACITY;
     return fail(TC_ERR_CAPACITY, "oriented graph exceeded its workspace");
   }
-  if (h.bad_flags & kBadTimeout) {
-    info->status = TC_ERR_TIMEOUT;
-    return fail(TC_ERR_TIMEOUT, "a staged copy of the count kernel did not land in time; the count is incomplete");
-  }
   if (h.sym_checksum != 0) {
     info->status = TC_ERR_NOT_SYMMETRIC;
     return fail(TC_ERR_NOT_SYMMETRIC, "adjacency is not symmetric");
@@ -1508,14 +1496,16 @@ tc_status cell_stats(int32_t n, Workspace& ws, double* out_host, cudaStream_t st
 }
 
 template <class View>
-tc_status validate_view(const View& view, int32_t n, Workspace& ws, cudaStream_t stream) {
+tc_status validate_view(const View& view, int32_t n, int64_t m, Workspace& ws, cudaStream_t stream) {
   TC_CUDA_TRY(cudaMemsetAsync(ws.st, 0, sizeof(DevStatus), stream));
-  if (n > 0) TC_TRY(orient(view, n, ws, to_params(nullptr), false, stream));
+  SchedParams sp = to_params(nullptr);
+  set_work_sizes(sp, n, m, ws.item_cap);
+  if (n > 0) TC_TRY(orient(view, n, ws, sp, false, stream));
   return TC_OK;
 }
 
-template tc_status validate_view<SlackView>(const SlackView&, int32_t, Workspace&, cudaStream_t);
-template tc_status validate_view<Csr64View>(const Csr64View&, int32_t, Workspace&, cudaStream_t);
+template tc_status validate_view<SlackView>(const SlackView&, int32_t, int64_t, Workspace&, cudaStream_t);
+template tc_status validate_view<Csr64View>(const Csr64View&, int32_t, int64_t, Workspace&, cudaStream_t);
 
 }  // namespace tc
 

@@ -66,7 +66,8 @@ typedef struct tc_sched {
                                into the longer one when 16 d_long > ratio * d_short (log2 d_long + 1),
                                else merges */
   int32_t blocks_per_sm;  /* persistent grid = SMs x blocks_per_sm (0 = occupancy limit) */
-  int32_t chunk;          /* vertices a warp claims per work-queue grab */
+  int32_t chunk;          /* most vertices a warp claims per work-queue grab (graphs with few
+                             vertices per warp, and all at 16, use fewer) */
   int32_t use_table;      /* 1 = the per-degree-cell strategy table below overrides the rules */
   uint8_t table[16][16];  /* strategy per cell [log2 d_a][log2 d_b]. Static count (a = the centre's
                              out-degree, b = the other endpoint's): 0 = the warp streams N+(b)
@@ -86,8 +87,8 @@ typedef struct tc_sched {
   int32_t lane_max_deg;   /* static count rule without a table: lists of at most this many entries
                              are walked by one lane each (several lists per warp step) */
   int32_t packed_max_deg; /* static count rule without a table: lists longer than lane_max_deg and
-                             of at most this many entries are packed: the warp walks all such lists
-                             of a group of 32 neighbours concatenated, 32 entries per step
+                             of at most this many entries are packed: the warp walks several such
+                             lists of a group of 32 neighbours at once, a few lanes each
                              (0 = never); longer lists are streamed one at a time */
   int32_t stream_hub_min; /* streaming delta count (tc_apply_batch, tc_pipeline): changed edges whose
                              longer-list endpoint holds at least this many of a batch phase's
