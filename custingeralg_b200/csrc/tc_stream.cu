@@ -31,12 +31,12 @@ namespace {
 constexpr int kThreads = 256;
 constexpr uint64_t kSentinel = ~0ull;
 constexpr int kLongList = 2048;  // lists longer than this are rewritten by a whole CTA
-// Tile shape of the delta count (defaults; the pipeline's autotuner picks per batch-size bin):
+// Tile shape of the cuStinger-style delta count (tc_count_batch):
 constexpr int kDeltaSplit = 2048;   // intersections whose shorter list is longer are split ...
 constexpr int kDeltaChunk = 1024;   // ... into items of this many entries of the shorter list
 constexpr int64_t kDeltaItems = 1 << 20;  // capacity of the split-item queue
 constexpr unsigned long long kNoItem = ~0ull;
-constexpr int kGrab = 4;  // changed edges a warp takes per grab from the delta kernel's queue
+constexpr int kGrab = 4;  // most changed edges a warp takes per grab from the delta kernel's queue
 // Bound of the persistent delta kernel's waits for queued split items (a wait that runs out
 // reports kErrTimeout and the warp leaves the item pass).
 constexpr unsigned long long kSpinNs = 2000000000ull;  // 2 s
@@ -75,6 +75,7 @@ struct BatchStatus {
   unsigned long long hub_total[2];  // changed edges placed in hub groups
   unsigned long long hub_q[2];    // work-queue heads of the hub kernel
   unsigned long long hub_items[2];  // hub work items queued
+  unsigned long long n_desc[2];   // changed edges left to the per-edge kernel
   unsigned long long e_next[2];   // work-queue heads of the delta kernel's entry and item passes
   unsigned long long i_next[2];
 };
@@ -833,6 +834,12 @@ struct BatchLists {
   const int32_t* dup;
 };
 
+// A changed edge as the per-edge kernel takes it: its lists, the shorter one first.
+struct __align__(16) DeltaDesc {
+  int32_t oa, ob, la, lb;  // owners and lengths
+  int64_t sa, sb;          // starts
+};
+
 struct DeltaArgs {
   SlackView g;
   const uint8_t* mark;
@@ -869,11 +876,12 @@ struct DeltaArgs {
   unsigned bar_extra;
   unsigned long long spin_ns;
   // hub-centred counting (k_delta_hub): changed edges whose longer endpoint holds at least
-  // hub_min of the phase's changed edges are counted at that endpoint (0 = never); hubbed[e] = 1
-  // marks them for the per-edge kernel to skip (NULL = no hub groups)
+  // hub_min of the phase's changed edges are counted at that endpoint (0 = never)
   int hub_min;
-  const uint8_t* hubbed;
-  // dynamic work queues of k_delta_fused's two passes (zero at launch; NULL = warp-strided)
+  // the changed edges not counted at a hub (k_hub_place) and their number
+  const DeltaDesc* desc;
+  const unsigned long long* n_desc;
+  // dynamic work queues of k_delta_fused's two passes (zero at launch)
   unsigned long long* e_next;
   unsigned long long* i_next;
   int stage_ok;      // the launch has kStageSmem of dynamic shared memory: staged cells may stage
@@ -938,6 +946,21 @@ struct DeltaPair {
   int cell;
 };
 
+// How the pair's lists are intersected. With marks (PRED = kPredMark) every cell that does not stage
+// searches: a merge's lanes each walk a chain of dependent loads, and searching was never slower
+// (whole streaming passes, ratio rule -> search everywhere: 3-1000 updates on R-MAT 22
+// 14.1 -> 6.7 ms, 20,011 on BA n = 2^20 3.8 -> 2.0 ms, 10^6 on R-MAT 22 16.3 -> 14.4 ms).
+template <int PRED>
+__device__ __forceinline__ int pair_strategy(const DeltaArgs& A, const DeltaPair& P) {
+  const int t = A.use_table ? A.table[P.cell] : -1;
+  if (t == kStratStage && A.stage_ok) return kStratStage;
+  if (PRED == kPredMark || t == kStratSearch) return kStratSearch;
+  if (t >= 0) return kStratMerge;
+  const int lg = 32 - __clz(P.lb);
+  return 16LL * P.lb > (long long)A.search_ratio_x16 * P.la * lg ? kStratSearch : kStratMerge;
+}
+
+template <int PRED>
 __device__ __forceinline__ DeltaPair delta_pair(const DeltaArgs& A, int32_t x, int32_t y, int32_t lx, int32_t ly,
                                                 int64_t sx, int64_t sy) {
   DeltaPair P;
@@ -950,13 +973,7 @@ __device__ __forceinline__ DeltaPair delta_pair(const DeltaArgs& A, int32_t x, i
   P.lb = xs ? ly : lx;
   P.key = ekey(x, y);
   P.cell = cell_of(P.la, P.lb);
-  const int lg = 32 - __clz(P.lb);
-  if (A.use_table) {
-    const int t = A.table[P.cell];
-    P.strat = t == kStratSearch ? kStratSearch : (t == kStratStage && A.stage_ok) ? kStratStage : kStratMerge;
-  } else {
-    P.strat = 16LL * P.lb > (long long)A.search_ratio_x16 * P.la * lg ? kStratSearch : kStratMerge;
-  }
+  P.strat = pair_strategy<PRED>(A, P);
   return P;
 }
 
@@ -969,8 +986,7 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
   const int lane = threadIdx.x & 31;
   const int32_t* L = A.g.ind;
   uint32_t c = 0;
-  auto on_match = [&](int64_t ia, int64_t ib, int32_t w) {
-    const bool ca = changed<PRED>(A, P.oa, P.sa + ia, w);
+  auto match = [&](const bool ca, int64_t ib, int32_t w) {
     const bool cb = changed<PRED>(A, P.ob, P.sb + ib, w);
     const bool keep = (!ca || P.key < ekey(P.oa, w)) && (!cb || P.key < ekey(P.ob, w));
     if (keep) {
@@ -978,6 +994,7 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
       atomicAdd(&pv[w], A.weight * (uint32_t)A.sign);
     }
   };
+  auto on_match = [&](int64_t ia, int64_t ib, int32_t w) { match(changed<PRED>(A, P.oa, P.sa + ia, w), ib, w); };
   const int64_t sb = P.sb, eb = P.sb + P.lb;
   if (P.strat == kStratStage) {
     // The part of the longer list that can meet entries [i_begin, i_end) of the shorter one,
@@ -1042,6 +1059,9 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
       const bool in = i < i_end, in2 = i2 < i_end;
       const int32_t w = in ? L[P.sa + i] : INT32_MAX;
       const int32_t w2 = in2 ? L[P.sa + i2] : INT32_MAX;
+      // the shorter list's marks are read beside its entries, not after a match
+      const bool ca = PRED == kPredMark && in && A.mark[P.sa + i] != 0;
+      const bool ca2 = PRED == kPredMark && in2 && A.mark[P.sa + i2] != 0;
       int64_t lo, hi, lo2, hi2;
       bucket(w, lo, hi);
       bucket(w2, lo2, hi2);
@@ -1059,8 +1079,14 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
           else hi2 = mid;
         }
       }
-      if (in && lo < eb && L[lo] == w) on_match(i, lo - sb, w);
-      if (in2 && lo2 < eb && L[lo2] == w2) on_match(i2, lo2 - sb, w2);
+      const bool m = in && lo < eb && L[lo] == w, m2 = in2 && lo2 < eb && L[lo2] == w2;
+      if (PRED == kPredMark) {
+        if (m) match(ca, lo - sb, w);
+        if (m2) match(ca2, lo2 - sb, w2);
+      } else {
+        if (m) on_match(i, lo - sb, w);
+        if (m2) on_match(i2, lo2 - sb, w2);
+      }
     }
   } else {
     const int32_t len = i_end - i_begin;
@@ -1111,45 +1137,25 @@ __device__ __forceinline__ int edge_shard(int32_t x, int32_t y, int nshards) {
   return (int)((z ^ (z >> 31)) % (uint64_t)nshards);
 }
 
-// The triangle delta of the changed edges, one warp per edge (warp-strided; with shards, only
-// this rank's edges). An edge whose shorter list is longer than A.split_min (two hubs) would be one
-// warp's serial tail of the whole launch: when A.split_items is set it is queued instead as
-// items of A.chunk entries of its shorter list, which the item pass spreads over all warps (a
-// full queue leaves the edge to this warp). Lane 0 of each warp accumulates the kept triangles
-// and the edge's algorithmic bytes.
-template <int PRED>
-__device__ __forceinline__ void delta_entries(const DeltaArgs& A, uint32_t* __restrict__ pv, const int64_t gw,
+// The cuStinger-style count (tc_count_batch): the triangle delta of the batch's edges, one warp per
+// edge (warp-strided; with shards, only this rank's edges). An edge whose shorter list is longer
+// than A.split_min (two hubs) would be one warp's serial tail of the whole launch: it is queued
+// instead as items of A.chunk entries of its shorter list, which the second launch spreads over
+// all warps (a full queue leaves the edge to this warp). Lane 0 of each warp accumulates the kept
+// triangles and the edge's algorithmic bytes.
+__device__ __forceinline__ void batch_entries(const DeltaArgs& A, uint32_t* __restrict__ pv, const int64_t gw,
                                               const int64_t nw, unsigned long long& tri_acc,
                                               unsigned long long& bytes_acc) {
   const int lane = threadIdx.x & 31;
-  const int64_t cnt = A.count_dev ? (int64_t)(*A.count_dev) : A.count_host;
-  const unsigned epoch = A.item_tag ? *A.item_epoch : 0u;
-  int64_t next = gw, next_end = 0;
-  for (;;) {
-    // the next entry: warp-strided, or from runs of kGrab entries taken from the queue
-    if (A.e_next) {
-      if (next >= next_end) {
-        unsigned long long g = 0;
-        if (lane == 0) g = atomicAdd(A.e_next, (unsigned long long)kGrab);
-        g = __shfl_sync(kFull, g, 0);
-        if ((int64_t)g >= cnt) break;
-        next = (int64_t)g;
-        next_end = min(cnt, next + kGrab);
-      }
-    } else if (next >= cnt) {
-      break;
-    }
-    const int64_t e = next;
-    next += A.e_next ? 1 : nw;
-    if (A.hubbed && A.hubbed[e]) continue;  // counted at its hub (k_delta_hub)
+  for (int64_t e = gw; e < A.count_host; e += nw) {
     int32_t x, y;
     bool count_total;
-    if (!delta_entry<PRED>(A, e, x, y, count_total)) continue;
+    if (!delta_entry<kPredBatch>(A, e, x, y, count_total)) continue;
     if (A.nshards > 1 && edge_shard(x, y, A.nshards) != A.shard) continue;
     const int32_t lx = A.g.len(x), ly = A.g.len(y);
     if (lx < 2 || ly < 2) continue;
     const int64_t sx = A.g.start(x), sy = A.g.start(y);
-    if (PRED == kPredBatch && A.only_present) {
+    if (A.only_present) {
       // the edge must exist for its triangles to be destroyed
       bool pres = false;
       if (lane == 0) {
@@ -1159,23 +1165,21 @@ __device__ __forceinline__ void delta_entries(const DeltaArgs& A, uint32_t* __re
       __syncwarp();
       if (!__shfl_sync(kFull, pres, 0)) continue;
     }
-    const DeltaPair P = delta_pair(A, x, y, lx, ly, sx, sy);
+    const DeltaPair P = delta_pair<kPredBatch>(A, x, y, lx, ly, sx, sy);
     if (A.cell_filter == -2 || (A.cell_filter >= 0 && P.cell != A.cell_filter)) continue;
     if (lane == 0 && count_total) bytes_acc += 4ull * (unsigned long long)(lx + ly) + 8ull;
-    if (A.split_items && P.la > A.split_min) {
+    if (P.la > A.split_min) {
       const int nch = (P.la + A.chunk - 1) / A.chunk;
       unsigned long long at = 0;
       if (lane == 0) at = atomicAdd(A.split_cnt, (unsigned long long)nch);
       at = __shfl_sync(kFull, at, 0);
       const bool fits = at + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
       for (int j = lane; j < nch; j += 32)
-        if (at + j < (unsigned long long)kDeltaItems) {
+        if (at + j < (unsigned long long)kDeltaItems)
           A.split_items[at + j] = fits ? ((unsigned long long)e << 24) | (unsigned long long)j : kNoItem;
-          if (A.item_tag) st_release(A.item_tag + at + j, epoch);  // the slot is ready
-        }
       if (fits) continue;
     }
-    const uint32_t c = delta_range<PRED>(A, P, 0, P.la, pv);
+    const uint32_t c = delta_range<kPredBatch>(A, P, 0, P.la, pv);
     if (lane == 0 && c) {
       atomicAdd(&pv[x], c * A.weight * (uint32_t)A.sign);
       atomicAdd(&pv[y], c * A.weight * (uint32_t)A.sign);
@@ -1184,53 +1188,103 @@ __device__ __forceinline__ void delta_entries(const DeltaArgs& A, uint32_t* __re
   }
 }
 
-// One queued chunk of a split intersection, run by the warp. The item's edge passed every check
-// of the entry pass already; its endpoints' per-vertex updates and the total add up per chunk.
-template <int PRED>
-__device__ __forceinline__ void delta_item_run(const DeltaArgs& A, uint32_t* __restrict__ pv,
-                                               const unsigned long long item, const int64_t cnt,
-                                               unsigned long long& tri_acc) {
-  const int lane = threadIdx.x & 31;
-  if (item == kNoItem) return;
-  const int64_t e = (int64_t)(item >> 24);
-  const int32_t k = (int32_t)(item & 0xffffffu);
-  if (e >= cnt) return;  // only an item of an abandoned pass could hold one
-  int32_t x, y;
-  bool count_total;
-  if (!delta_entry<PRED>(A, e, x, y, count_total)) return;
-  const int32_t lx = A.g.len(x), ly = A.g.len(y);
-  const int64_t sx = A.g.start(x), sy = A.g.start(y);
-  const DeltaPair P = delta_pair(A, x, y, lx, ly, sx, sy);
-  const int32_t i0 = k * A.chunk;
-  if (i0 >= P.la) return;
-  const uint32_t c = delta_range<PRED>(A, P, i0, min(P.la, i0 + A.chunk), pv);
-  if (lane == 0 && c) {
-    atomicAdd(&pv[x], c * A.weight * (uint32_t)A.sign);
-    atomicAdd(&pv[y], c * A.weight * (uint32_t)A.sign);
-    if (count_total) tri_acc += c;
-  }
-}
-
-// The queued chunks of the split intersections after the entry pass has finished (the second
-// launch of the cuStinger-style count), one warp per item: warp-strided, or one at a time from
-// the queue.
-template <int PRED>
-__device__ __forceinline__ void delta_items(const DeltaArgs& A, uint32_t* __restrict__ pv, const int64_t gw,
+// Its queued chunks, one warp per item (the second launch). An item's edge passed every check of
+// the entry pass; its endpoints' per-vertex updates and the total add up per chunk.
+__device__ __forceinline__ void batch_items(const DeltaArgs& A, uint32_t* __restrict__ pv, const int64_t gw,
                                             const int64_t nw, unsigned long long& tri_acc) {
   const int lane = threadIdx.x & 31;
   const int64_t n_items = (int64_t)min(*A.split_cnt, (unsigned long long)kDeltaItems);
-  const int64_t cnt = A.count_dev ? (int64_t)(*A.count_dev) : A.count_host;
-  for (int64_t q0 = gw;;) {
-    int64_t q = q0;
-    if (A.i_next) {
-      unsigned long long g = 0;
-      if (lane == 0) g = atomicAdd(A.i_next, 1ull);
-      q = (int64_t)__shfl_sync(kFull, g, 0);
-    } else {
-      q0 += nw;
+  for (int64_t q = gw; q < n_items; q += nw) {
+    const unsigned long long item = A.split_items[q];
+    if (item == kNoItem) continue;
+    const int64_t e = (int64_t)(item >> 24);
+    int32_t x, y;
+    bool count_total;
+    if (!delta_entry<kPredBatch>(A, e, x, y, count_total)) continue;
+    const DeltaPair P =
+        delta_pair<kPredBatch>(A, x, y, A.g.len(x), A.g.len(y), A.g.start(x), A.g.start(y));
+    const int32_t i0 = (int32_t)(item & 0xffffffu) * A.chunk;
+    if (i0 >= P.la) continue;
+    const uint32_t c = delta_range<kPredBatch>(A, P, i0, min(P.la, i0 + A.chunk), pv);
+    if (lane == 0 && c) {
+      atomicAdd(&pv[x], c * A.weight * (uint32_t)A.sign);
+      atomicAdd(&pv[y], c * A.weight * (uint32_t)A.sign);
+      if (count_total) tri_acc += c;
     }
-    if (q >= n_items) break;
-    delta_item_run<PRED>(A, pv, A.split_items[q], cnt, tri_acc);
+  }
+}
+
+// The pair of a described edge.
+__device__ __forceinline__ DeltaPair described_pair(const DeltaArgs& A, const DeltaDesc& d) {
+  DeltaPair P;
+  P.oa = d.oa;
+  P.ob = d.ob;
+  P.la = d.la;
+  P.lb = d.lb;
+  P.sa = d.sa;
+  P.sb = d.sb;
+  P.key = ekey(d.oa, d.ob);
+  P.cell = A.use_table ? cell_of(d.la, d.lb) : 0;
+  P.strat = pair_strategy<kPredMark>(A, P);
+  return P;
+}
+
+// Entries [i0, i1) of a described edge's shorter list, run by the warp.
+__device__ __forceinline__ void delta_part(const DeltaArgs& A, uint32_t* __restrict__ pv, const DeltaDesc& d,
+                                           const int32_t i0, const int32_t i1, unsigned long long& tri_acc) {
+  const uint32_t c = delta_range<kPredMark>(A, described_pair(A, d), i0, i1, pv);
+  if ((threadIdx.x & 31) == 0 && c) {
+    atomicAdd(&pv[d.oa], c * A.weight * (uint32_t)A.sign);
+    atomicAdd(&pv[d.ob], c * A.weight * (uint32_t)A.sign);
+    tri_acc += c;
+  }
+}
+
+// The entry pass of the persistent kernel: the described edges, one warp per edge, taken from a queue
+// up to kGrab at a time (the descriptions of a grab are read together; a batch of fewer edges
+// than warps goes out one by one). An edge whose shorter list is longer than A.split_min is queued
+// as items of A.chunk entries of it, published one by one (a full queue leaves the edge to this
+// warp).
+__device__ __forceinline__ void delta_entries(const DeltaArgs& A, uint32_t* __restrict__ pv,
+                                              unsigned long long& tri_acc, unsigned long long& bytes_acc) {
+  const int lane = threadIdx.x & 31;
+  const int64_t cnt = (int64_t)*A.n_desc;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int grab = (int)max((int64_t)1, min((int64_t)kGrab, cnt / (2 * nw)));
+  const unsigned epoch = *A.item_epoch;
+  for (;;) {
+    unsigned long long g = 0;
+    if (lane == 0) g = atomicAdd(A.e_next, (unsigned long long)grab);
+    g = __shfl_sync(kFull, g, 0);
+    if ((int64_t)g >= cnt) break;
+    const int have = (int)min((int64_t)grab, cnt - (int64_t)g);
+    DeltaDesc mine = {};
+    if (lane < have) mine = A.desc[g + lane];
+    __syncwarp();
+    for (int k = 0; k < have; ++k) {
+      DeltaDesc d;
+      d.oa = __shfl_sync(kFull, mine.oa, k);
+      d.ob = __shfl_sync(kFull, mine.ob, k);
+      d.la = __shfl_sync(kFull, mine.la, k);
+      d.lb = __shfl_sync(kFull, mine.lb, k);
+      d.sa = __shfl_sync(kFull, mine.sa, k);
+      d.sb = __shfl_sync(kFull, mine.sb, k);
+      if (lane == 0) bytes_acc += 4ull * ((unsigned long long)d.la + (unsigned long long)d.lb) + 8ull;
+      if (d.la > A.split_min) {
+        const int nch = (d.la + A.chunk - 1) / A.chunk;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(A.split_cnt, (unsigned long long)nch);
+        at = __shfl_sync(kFull, at, 0);
+        const bool fits = at + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
+        for (int j = lane; j < nch; j += 32)
+          if (at + j < (unsigned long long)kDeltaItems) {
+            A.split_items[at + j] = fits ? ((g + k) << 24) | (unsigned long long)j : kNoItem;
+            st_release(A.item_tag + at + j, epoch);  // the slot is ready
+          }
+        if (fits) continue;
+      }
+      delta_part(A, pv, d, 0, d.la, tri_acc);
+    }
   }
 }
 
@@ -1261,13 +1315,12 @@ __device__ __forceinline__ int wait_item(const DeltaArgs& A, const unsigned long
 // while other warps may still queue items. Slots are taken in order from the queue head; a slot
 // is read once its tag carries this launch's epoch (items written by other CTAs are read past
 // the non-coherent L1 after the acquire).
-template <int PRED>
 __device__ __forceinline__ void delta_items_stream(const DeltaArgs& A, uint32_t* __restrict__ pv,
                                                    unsigned long long& tri_acc) {
   const int lane = threadIdx.x & 31;
   const unsigned epoch = *A.item_epoch;
   const unsigned total = (unsigned)(((int64_t)gridDim.x * blockDim.x) >> 5) + A.bar_extra;
-  const int64_t cnt = (int64_t)__ldcg(A.count_dev);
+  const unsigned long long cnt = *A.n_desc;
   for (;;) {
     unsigned long long q = 0;
     int state = 0;
@@ -1279,28 +1332,30 @@ __device__ __forceinline__ void delta_items_stream(const DeltaArgs& A, uint32_t*
     state = __shfl_sync(kFull, state, 0);
     q = __shfl_sync(kFull, q, 0);
     if (state != 1) break;
-    delta_item_run<PRED>(A, pv, __ldcg(A.split_items + q), cnt, tri_acc);
+    const unsigned long long item = __ldcg(A.split_items + q);
+    if (item == kNoItem || (item >> 24) >= cnt) continue;
+    const DeltaDesc d = A.desc[item >> 24];
+    const int32_t i0 = (int32_t)(item & 0xffffffu) * A.chunk;
+    if (i0 < d.la) delta_part(A, pv, d, i0, min(d.la, i0 + A.chunk), tri_acc);
   }
 }
 
 // Two launches: the entry pass, then the item pass (the cuStinger-style count, tc_count_batch).
-template <int PRED>
 __global__ void __launch_bounds__(kThreads, 6) k_delta(const DeltaArgs A, uint32_t* __restrict__ pv,
                                                     unsigned long long* __restrict__ tri_out) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long tri_acc = 0, bytes_acc = 0;
-  delta_entries<PRED>(A, pv, gw, nw, tri_acc, bytes_acc);
+  batch_entries(A, pv, gw, nw, tri_acc, bytes_acc);
   delta_flush(tri_acc, bytes_acc, tri_out, A.bytes_out);
 }
 
-template <int PRED>
 __global__ void __launch_bounds__(kThreads, 6) k_delta_split(const DeltaArgs A, uint32_t* __restrict__ pv,
                                                           unsigned long long* __restrict__ tri_out) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long tri_acc = 0;
-  delta_items<PRED>(A, pv, gw, nw, tri_acc);
+  batch_items(A, pv, gw, nw, tri_acc);
   delta_flush(tri_acc, 0ull, tri_out, nullptr);
 }
 
@@ -1312,16 +1367,13 @@ __global__ void __launch_bounds__(kThreads, 6) k_delta_split(const DeltaArgs A, 
 // epoch (bumped before it) marks the slots published in this launch. A wait that runs out (the
 // grid was not resident, or a test forces it) sets kErrTimeout and the warp leaves the item
 // pass: the batch's count is then incomplete and the host reports TC_ERR_TIMEOUT.
-template <int PRED>
 #ifndef TC_DELTA_MIN_BLOCKS
 #define TC_DELTA_MIN_BLOCKS 6
 #endif
 __global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(const DeltaArgs A, uint32_t* __restrict__ pv,
                                                           unsigned long long* __restrict__ tri_out) {
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long tri_acc = 0, bytes_acc = 0;
-  delta_entries<PRED>(A, pv, gw, nw, tri_acc, bytes_acc);
+  delta_entries(A, pv, tri_acc, bytes_acc);
   // this warp's items are published: count it done (its lanes' releases before lane 0's add)
   __threadfence();
   __syncwarp();
@@ -1329,7 +1381,7 @@ __global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(c
     __threadfence();
     atomicAdd(A.entry_done, 1u);
   }
-  delta_items_stream<PRED>(A, pv, tri_acc);
+  delta_items_stream(A, pv, tri_acc);
   delta_flush(tri_acc, bytes_acc, tri_out, A.bytes_out);
 }
 
@@ -1354,7 +1406,8 @@ __global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(c
 // edge whichever kernel counts it. Grouping takes three passes over the changed edges: count the
 // edges, units and partner entries per longer endpoint, where a vertex becomes a hub when its
 // edge count reaches hub_min; give each hub a range of unit slots and its items; place the units
-// and flag the edges hubbed. A hub whose units or items do not fit is left to the per-edge kernel.
+// and describe the other edges for the per-edge kernel. A hub whose units or items do not fit is left
+// to that kernel.
 
 #ifndef TC_HUB_THREADS
 #define TC_HUB_THREADS 512
@@ -1392,7 +1445,10 @@ struct HubWs {
   int32_t* fill;     // [cap]
   int2* units;       // [unit_cap] (partner s, unit r: entries [r kHubUnit, (r + 1) kHubUnit) of N(s))
   int64_t unit_cap;
-  uint8_t* hubbed;   // [cap] 1 = counted at its hub
+  DeltaDesc* desc;   // [cap] the edges not counted at a hub
+  unsigned long long* n_desc;
+  unsigned* item_epoch;
+  int on;            // hub groups are formed (0: every edge is described)
   unsigned long long* items;  // [item_cap] (hub id << 32 | item index within the hub)
   int64_t item_cap;
   unsigned long long* n_hubs;
@@ -1401,9 +1457,10 @@ struct HubWs {
   unsigned long long* q;
 };
 
-// Changed edge e as the hub count sees it: false unless this rank counts it and both lists have
-// at least two entries (the per-edge kernel's filters); h = the endpoint with the longer list.
-__device__ __forceinline__ bool hub_entry(const DeltaArgs& A, int64_t e, int32_t& h, int32_t& s, int32_t& ls) {
+// Changed edge e as the delta count sees it: false unless this rank counts it and both lists have
+// at least two entries; h = the endpoint with the longer list, s = the other one.
+__device__ __forceinline__ bool hub_entry(const DeltaArgs& A, int64_t e, int32_t& h, int32_t& s, int32_t& lh,
+                                          int32_t& ls) {
   int32_t x, y;
   bool count_total;
   if (!delta_entry<kPredMark>(A, e, x, y, count_total)) return false;
@@ -1413,6 +1470,7 @@ __device__ __forceinline__ bool hub_entry(const DeltaArgs& A, int64_t e, int32_t
   const bool x_long = lx > ly || (lx == ly && x < y);
   h = x_long ? x : y;
   s = x_long ? y : x;
+  lh = x_long ? lx : ly;
   ls = x_long ? ly : lx;
   return true;
 }
@@ -1420,8 +1478,8 @@ __device__ __forceinline__ bool hub_entry(const DeltaArgs& A, int64_t e, int32_t
 __global__ void __launch_bounds__(kThreads) k_hub_count(const DeltaArgs A, const HubWs H) {
   const int64_t cnt = (int64_t)*A.count_dev;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-    int32_t h, s, ls;
-    if (!hub_entry(A, e, h, s, ls)) continue;
+    int32_t h, s, lh, ls;
+    if (!hub_entry(A, e, h, s, lh, ls)) continue;
     atomicAdd(reinterpret_cast<unsigned long long*>(&H.sum[h]), (unsigned long long)ls);
     atomicAdd(&H.uni[h], (ls + kHubUnit - 1) / kHubUnit);
     if (atomicAdd(&H.cnt[h], 1) + 1 == A.hub_min) {  // exactly one edge sees the count reach hub_min
@@ -1471,26 +1529,38 @@ __global__ void __launch_bounds__(kThreads) k_hub_alloc(const DeltaArgs A, const
   }
 }
 
-// Place the units of every hub edge in its hub's range and flag the edge; clears the per-vertex
-// counts.
+// Place the units of every hub edge in its hub's range and describe every other edge for the per-edge
+// kernel (its lists looked up here once, by a thread per edge, so that a warp of that kernel starts
+// with one load); clears the per-vertex counts and opens the per-edge kernel's launch epoch.
 __global__ void __launch_bounds__(kThreads) k_hub_place(const DeltaArgs A, const HubWs H) {
   const int64_t cnt = (int64_t)*A.count_dev;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-    uint8_t f = 0;
-    int32_t h, s, ls;
-    if (hub_entry(A, e, h, s, ls)) {
+  const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *H.item_epoch += 1u;
+  for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); e0 < cnt;
+       e0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e = e0 + lane;
+    int32_t h = 0, s = 0, lh = 0, ls = 0;
+    bool left = e < cnt && hub_entry(A, e, h, s, lh, ls);  // counted by the per-edge kernel
+    if (left && H.on) {
       const int32_t hid1 = H.of[h];
       if (hid1 > 0) {
         const int32_t u = (ls + kHubUnit - 1) / kHubUnit;
         const int32_t pos = H.off[hid1 - 1] + atomicAdd(&H.fill[hid1 - 1], u);
         for (int32_t r = 0; r < u; ++r) H.units[pos + r] = make_int2(s, r);
-        f = 1;
+        left = false;
       }
       H.cnt[h] = 0;
       H.uni[h] = 0;
       H.sum[h] = 0;
     }
-    H.hubbed[e] = f;
+    if (A.cell_filter != -1 && (A.cell_filter == -2 || cell_of(ls, lh) != A.cell_filter)) left = false;
+    __syncwarp();
+    const unsigned m = __ballot_sync(kFull, left);
+    if (m == 0) continue;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(H.n_desc, (unsigned long long)__popc(m));
+    at = __shfl_sync(kFull, at, 0);
+    if (left) H.desc[at + __popc(m & ((1u << lane) - 1u))] = DeltaDesc{s, h, ls, lh, A.g.start(s), A.g.start(h)};
   }
 }
 
@@ -1837,7 +1907,7 @@ struct StreamWs {
   int32_t* hub_fill = nullptr;    // [b]
   int32_t* hub_chunks = nullptr;  // [b]
   int2* hub_units = nullptr;      // [kHubUnitsPerUpdate * b]
-  uint8_t* hubbed = nullptr;      // [b]
+  DeltaDesc* desc = nullptr;      // [b] changed edges of the per-edge kernel
   unsigned long long* hub_items = nullptr;  // [kHubItemsPerUpdate * b]
   void release();
 };
@@ -1851,7 +1921,7 @@ void StreamWs::release() {
   cudaFree(vlist); cudaFree(claim); cudaFree(first_del); cudaFree(d_epoch); cudaFree(cub_tmp); cudaFree(st); cudaFreeHost(st_host); cudaFree(counter);
   cudaFree(cnt); cudaFree(scan64); cudaFree(tiles); cudaFree(split_items); cudaFree(item_tag); cudaFree(item_epoch);
   cudaFree(hub_cnt); cudaFree(hub_sum); cudaFree(hub_uni); cudaFree(hub_of); cudaFree(hub_list); cudaFree(hub_off);
-  cudaFree(hub_len); cudaFree(hub_fill); cudaFree(hub_chunks); cudaFree(hub_units); cudaFree(hubbed);
+  cudaFree(hub_len); cudaFree(hub_fill); cudaFree(hub_chunks); cudaFree(hub_units); cudaFree(desc);
   cudaFree(hub_items);
   *this = StreamWs();
 }
@@ -1946,12 +2016,12 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
     cudaFree(w.long_cnt); cudaFree(w.long_plan); cudaFree(w.cmp_plan);
     w.long_cnt = nullptr; w.long_plan = nullptr; w.cmp_plan = nullptr;
     cudaFree(w.hub_list); cudaFree(w.hub_off); cudaFree(w.hub_len); cudaFree(w.hub_fill); cudaFree(w.hub_chunks);
-    cudaFree(w.hub_units); cudaFree(w.hubbed); cudaFree(w.hub_items);
+    cudaFree(w.hub_units); cudaFree(w.desc); cudaFree(w.hub_items);
     w.src = nullptr; w.dst = nullptr; w.isdel = nullptr; w.keys = nullptr; w.keys2 = nullptr; w.head = nullptr;
     w.dlist = nullptr; w.ilist = nullptr; w.dk = nullptr; w.dk2 = nullptr; w.run_start = nullptr;
     w.long_runs = nullptr; w.ins_slot = nullptr; w.vlist = nullptr; w.cub_tmp = nullptr;
     w.hub_list = nullptr; w.hub_off = nullptr; w.hub_len = nullptr; w.hub_fill = nullptr; w.hub_chunks = nullptr;
-    w.hub_units = nullptr; w.hubbed = nullptr; w.hub_items = nullptr;
+    w.hub_units = nullptr; w.desc = nullptr; w.hub_items = nullptr;
     w.b_cap = 0;
     w.cub_bytes = 0;
   };
@@ -1981,7 +2051,7 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
             ::tc::dev_malloc(&w.hub_fill, sizeof(int32_t) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.hub_chunks, sizeof(int32_t) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.hub_units, sizeof(int2) * kHubUnitsPerUpdate * nb) == cudaSuccess &&
-            ::tc::dev_malloc(&w.hubbed, nb) == cudaSuccess &&
+            ::tc::dev_malloc(&w.desc, sizeof(DeltaDesc) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.hub_items, sizeof(unsigned long long) * kHubItemsPerUpdate * nb) == cudaSuccess &&
             cub::DeviceRadixSort::SortKeys(nullptr, t1, w.keys, w.keys2, (int)(2 * nb)) == cudaSuccess &&
             cub::DeviceRadixSort::SortKeys(nullptr, t2, w.dk, w.dk2, (int)(2 * nb)) == cudaSuccess &&
@@ -2089,6 +2159,22 @@ DeltaArgs delta_args(tc_graph* g, const SchedParams& sp) {
   return A;
 }
 
+struct PipeCand {
+  int ctas;       // persistent delta kernel CTAs per SM (0 = the occupancy limit)
+  int chunk;      // split-item size: entries of the shorter list
+  int split_min;  // intersections whose shorter list is longer than this are split
+};
+constexpr int kPipeCands = 5;
+constexpr PipeCand kPipeCand[kPipeCands] = {
+    {0, 1024, 2048}, {0, 512, 1024}, {0, 256, 512}, {0, 128, 256}, {0, 64, 128}};
+
+// The shape without tuning, for a phase of about `edges` changed edges: small items where few edges
+// share the chip (a warp searching 1024 entries into a hub's list is a chain of hundreds of
+// dependent loads: batches of 3-1000 updates on R-MAT 22 6.7 ms with items of 1024, 3.2 ms with 64,
+// a pass of 12 batches), larger ones where the items' own look-ups count (10^6 updates: 13.4 ms a
+// pass with 256, 14.1 with 64, 14.4 with 1024).
+int default_cand(int64_t edges) { return edges <= ((int64_t)1 << 15) ? 4 : 2; }
+
 // Dynamic shared memory of a delta-kernel launch with these arguments.
 size_t delta_smem(const DeltaArgs& A) { return A.stage_ok ? kStageSmem : 0; }
 
@@ -2133,7 +2219,7 @@ tc_status fused_grid(int ctas_per_sm, size_t smem, int* grid) {
   const int k = smem > 0 ? 1 : 0;
   if (occ[dev][k] == 0) {
     int b = 0;
-    TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_delta_fused<kPredMark>, kThreads, k ? kStageSmem : 0));
+    TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_delta_fused, kThreads, k ? kStageSmem : 0));
     occ[dev][k] = std::max(1, b);
   }
   const int per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, occ[dev][k]) : occ[dev][k];
@@ -2161,13 +2247,11 @@ tc_status hub_grid(int* grid) {
 }
 
 // Hub groups and their count for one phase of a batch (deletions: phase 0, insertions: 1) on a
-// grid of `grid` hub CTAs; `cap` bounds the phase's changed edges. Sets A.hubbed for the
-// per-edge kernel that follows (NULL when the hub count is off: hub_min <= 0, or a timing run of
-// one degree cell). Launches only (it can run inside a stream capture).
+// grid of `grid` hub CTAs, and the descriptions of the edges left to the per-edge kernel that
+// follows (all of them when the hub count is off: hub_min <= 0, or a timing run of one degree
+// cell); `cap` bounds the phase's changed edges. Launches only (it can run inside a stream capture).
 void hub_kernels(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, int grid, uint32_t* pv,
                  unsigned long long* tri_out, cudaStream_t s) {
-  A.hubbed = nullptr;
-  if (A.hub_min <= 0 || A.cell_filter != -1) return;
   HubWs H;
   H.cnt = w.hub_cnt;
   H.sum = w.hub_sum;
@@ -2180,19 +2264,25 @@ void hub_kernels(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, int grid, ui
   H.fill = w.hub_fill;
   H.units = w.hub_units;
   H.unit_cap = kHubUnitsPerUpdate * w.b_cap;
-  H.hubbed = w.hubbed;
+  H.desc = w.desc;
+  H.n_desc = &w.st->n_desc[phase];
+  H.item_epoch = w.item_epoch;
+  H.on = A.hub_min > 0 && A.cell_filter == -1;
   H.items = w.hub_items;
   H.item_cap = kHubItemsPerUpdate * w.b_cap;
   H.n_hubs = &w.st->n_hubs[phase];
   H.total = &w.st->hub_total[phase];
   H.n_items = &w.st->hub_items[phase];
   H.q = &w.st->hub_q[phase];
+  A.desc = w.desc;
+  A.n_desc = H.n_desc;
   const int gb = grid_for(cap, kThreads);
-  k_hub_count<<<gb, kThreads, 0, s>>>(A, H);
-  k_hub_alloc<<<gb, kThreads, 0, s>>>(A, H);
+  if (H.on) {
+    k_hub_count<<<gb, kThreads, 0, s>>>(A, H);
+    k_hub_alloc<<<gb, kThreads, 0, s>>>(A, H);
+  }
   k_hub_place<<<gb, kThreads, 0, s>>>(A, H);
-  k_delta_hub<<<grid, kHubThreads, kHubSmem, s>>>(A, H, pv, tri_out);
-  A.hubbed = w.hubbed;
+  if (H.on) k_delta_hub<<<grid, kHubThreads, kHubSmem, s>>>(A, H, pv, tri_out);
 }
 
 tc_status launch_hub(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, uint32_t* pv, unsigned long long* tri_out,
@@ -2206,8 +2296,11 @@ tc_status launch_hub(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, uint32_t
 
 // The persistent delta kernel of one phase of a batch (deletions: phase 0, insertions: 1) on
 // the batch workspace's counters, after the hub groups' count.
-tc_status launch_delta_fused(DeltaArgs A, StreamWs& w, int phase, uint32_t* pv, unsigned long long* tri_out,
-                             int ctas_per_sm, cudaStream_t s) {
+tc_status launch_delta_fused(DeltaArgs A, StreamWs& w, int phase, int64_t edges, uint32_t* pv,
+                             unsigned long long* tri_out, cudaStream_t s) {
+  const PipeCand& shape = kPipeCand[default_cand(edges)];
+  A.chunk = shape.chunk;
+  A.split_min = shape.split_min;
   A.split_items = w.split_items;
   A.split_cnt = &w.st->n_split[phase];
   A.entry_done = &w.st->entry_done[phase];
@@ -2217,11 +2310,10 @@ tc_status launch_delta_fused(DeltaArgs A, StreamWs& w, int phase, uint32_t* pv, 
   A.bytes_out = &w.st->delta_bytes;
   A.e_next = &w.st->e_next[phase];
   A.i_next = &w.st->i_next[phase];
-  TC_TRY(launch_hub(A, w, phase, w.b_cap, pv, tri_out, s));
+  TC_TRY(launch_hub(A, w, phase, edges, pv, tri_out, s));
   int grid = 0;
-  TC_TRY(fused_grid(ctas_per_sm, delta_smem(A), &grid));
-  k_bump_epoch<<<1, 32, 0, s>>>(w.item_epoch);  // marks the item slots this launch publishes
-  k_delta_fused<kPredMark><<<grid, kThreads, delta_smem(A), s>>>(A, pv, tri_out);
+  TC_TRY(fused_grid(shape.ctas, delta_smem(A), &grid));
+  k_delta_fused<<<grid, kThreads, delta_smem(A), s>>>(A, pv, tri_out);
   return TC_OK;
 }
 
@@ -2303,7 +2395,7 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
     A.count_dev = &w.st->n_del;
     A.sign = -1;
     A.weight = 2;
-    TC_TRY(launch_delta_fused(A, w, 0, pv_use, &w.st->tri_removed, 0, s));
+    TC_TRY(launch_delta_fused(A, w, 0, (int64_t)h.n_del, pv_use, &w.st->tri_removed, s));
     k_endpoints<<<gd, kThreads, 0, s>>>(w.dlist, w.st, w.vlist);
     k_bump_epoch<<<1, 32, 0, s>>>(w.d_epoch);
     k_compact_marked<<<grid_for(2 * (int64_t)h.n_del * 32, kThreads), kThreads, 0, s>>>(
@@ -2323,7 +2415,7 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
     A.count_dev = &w.st->n_ins;
     A.sign = 1;
     A.weight = 2;
-    TC_TRY(launch_delta_fused(A, w, 1, pv_use, &w.st->tri_added, 0, s));
+    TC_TRY(launch_delta_fused(A, w, 1, (int64_t)h.n_ins, pv_use, &w.st->tri_added, s));
     k_clear_slots<<<grid_for(2 * (int64_t)h.n_ins, kThreads), kThreads, 0, s>>>(w.ins_slot, 2 * (int64_t)h.n_ins,
                                                                                   nullptr, g->mark);
     TC_CUDA_TRY(cudaGetLastError());
@@ -2484,9 +2576,9 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
     A.split_items = w.split_items;
     A.split_cnt = &w.st->n_split[0];
     TC_CUDA_TRY(cudaMemsetAsync(A.split_cnt, 0, sizeof(unsigned long long), s));
-    k_delta<kPredBatch><<<delta_grid(), kThreads, delta_smem(A), s>>>(A, reinterpret_cast<uint32_t*>(per_vertex),
+    k_delta<<<delta_grid(), kThreads, delta_smem(A), s>>>(A, reinterpret_cast<uint32_t*>(per_vertex),
                                                                      w.counter);
-    k_delta_split<kPredBatch><<<delta_grid(), kThreads, delta_smem(A), s>>>(A, reinterpret_cast<uint32_t*>(per_vertex),
+    k_delta_split<<<delta_grid(), kThreads, delta_smem(A), s>>>(A, reinterpret_cast<uint32_t*>(per_vertex),
                                                                            w.counter);
     TC_CUDA_TRY(cudaGetLastError());
   }
@@ -2528,15 +2620,6 @@ namespace tc {
 namespace {
 constexpr int kPipeBins = 16;
 constexpr int64_t kPipeMinBin = 1 << 10;
-struct PipeCand {
-  int ctas;       // persistent delta kernel CTAs per SM (0 = the occupancy limit)
-  int chunk;      // split-item size: entries of the shorter list
-  int split_min;  // intersections whose shorter list is longer than this are split
-};
-constexpr int kPipeCands = 5;
-constexpr PipeCand kPipeCand[kPipeCands] = {
-    {0, kDeltaChunk, kDeltaSplit}, {0, kDeltaChunk / 2, kDeltaSplit / 2}, {0, kDeltaChunk / 4, kDeltaSplit / 4},
-    {0, kDeltaChunk / 8, kDeltaSplit / 8}, {0, kDeltaChunk / 16, kDeltaSplit / 16}};
 constexpr int kPipeArms = kPipeCands + 1;  // + the default shape in the next bin's graph
 constexpr double kMergeSlack = 1.03;
 }  // namespace
@@ -2726,8 +2809,7 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
     A.i_next = &w.st->i_next[0];
     if (p->profile) cudaEventRecordWithFlags(p->pev[0], s, cudaEventRecordExternal);
     hub_kernels(A, w, 0, cap, ghub, pv, &w.st->tri_removed, s);
-    k_bump_epoch<<<1, 32, 0, s>>>(w.item_epoch);
-    k_delta_fused<kPredMark><<<gdelta, kThreads, dsm, s>>>(A, pv, &w.st->tri_removed);
+    k_delta_fused<<<gdelta, kThreads, dsm, s>>>(A, pv, &w.st->tri_removed);
     if (p->profile) cudaEventRecordWithFlags(p->pev[1], s, cudaEventRecordExternal);
     k_endpoints<<<gb, kThreads, 0, s>>>(w.dlist, w.st, w.vlist);
     k_bump_epoch<<<1, 32, 0, s>>>(w.d_epoch);
@@ -2749,8 +2831,7 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
     B.i_next = &w.st->i_next[1];
     if (p->profile) cudaEventRecordWithFlags(p->pev[2], s, cudaEventRecordExternal);
     hub_kernels(B, w, 1, cap, ghub, pv, &w.st->tri_added, s);
-    k_bump_epoch<<<1, 32, 0, s>>>(w.item_epoch);
-    k_delta_fused<kPredMark><<<gdelta, kThreads, dsm, s>>>(B, pv, &w.st->tri_added);
+    k_delta_fused<<<gdelta, kThreads, dsm, s>>>(B, pv, &w.st->tri_added);
     if (p->profile) cudaEventRecordWithFlags(p->pev[3], s, cudaEventRecordExternal);
     k_clear_slots<<<g2, kThreads, 0, s>>>(w.ins_slot, 0, &w.st->n_ins, g->mark);
     k_add_delta<<<1, 32, 0, s>>>(delta, &w.st->tri_added, &w.st->tri_removed);
@@ -2833,7 +2914,7 @@ tc_status tc_pipeline_create(tc_graph* g, int64_t max_batch, const tc_sched* sch
   }
   p->b_max = p->bin_cap[p->nbins - 1];
   for (int i = 0; i < kPipeBins; ++i) {
-    p->cand[i] = 0;
+    p->cand[i] = i < p->nbins ? default_cand(p->bin_cap[i]) : 0;
     p->serve[i] = i;
   }
   tc_status rc = TC_OK;
