@@ -1414,7 +1414,8 @@ __global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(c
 #endif
 constexpr int kHubThreads = TC_HUB_THREADS;
 constexpr int kHubCtasPerSm = 1536 / kHubThreads;
-constexpr int kHubBucketsMax = 2048 * kHubThreads / 256;  // 64 KB of int32 keys for 512 threads
+// log2 of the slots of each half of the largest table: 32 slots a thread, 64 KB of keys for 512 threads
+constexpr int kHubSlotBits = kHubThreads <= 256 ? 12 : kHubThreads <= 512 ? 13 : 14;
 #ifndef TC_HUB_UNIT
 #define TC_HUB_UNIT 512
 #endif
@@ -1422,7 +1423,7 @@ constexpr int kHubBucketsMax = 2048 * kHubThreads / 256;  // 64 KB of int32 keys
 // item for the warp with the last unit; on the streaming workload 512 entries measured 5 % less
 // time than 1024 over the whole run (prefetching the next 128 entries changed nothing).
 constexpr int kHubUnit = TC_HUB_UNIT;
-constexpr int kHubPass = 2 * kHubBucketsMax;  // entries of N(h) per pass (load <= 0.5)
+constexpr int kHubPass = 3 << (kHubSlotBits - 2);  // entries of N(h) per pass (load <= 3/8)
 constexpr int32_t kHubMarkBit = INT32_MIN;    // bit 31 of a stored key: the edge (h, key) is changed
 constexpr int64_t kHubSearchCost = 64;        // an item's estimate of one range search, in probes
 #ifndef TC_HUB_ITEM_LOG2
@@ -1564,41 +1565,46 @@ __global__ void __launch_bounds__(kThreads) k_hub_place(const DeltaArgs A, const
   }
 }
 
-__device__ __forceinline__ uint32_t hub_bucket(int32_t w, int bits) {
-  return ((uint32_t)w * 0x9E3779B1u) >> (32 - bits);
-}
-
-// Insert a key (id, with kHubMarkBit when the edge to it is changed) into 2^bits buckets of 4
-// slots (load <= 0.5: a bucket with a free slot is always found).
-__device__ __forceinline__ void hub_insert(int32_t* keys, int bits, int32_t id, int32_t key) {
-  const uint32_t bmask = (1u << bits) - 1;
-  uint32_t b = hub_bucket(id, bits);
-  for (uint32_t it = 0; it <= bmask; ++it) {
-#pragma unroll
-    for (int t = 0; t < 4; ++t)
-      if (atomicCAS(&keys[4 * b + t], -1, key) == -1) return;
-    b = (b + 1) & bmask;
+// A hub's hash set in shared memory: 2 * 2^bits slots of 4 bytes, every key (an id, with kHubMarkBit
+// when the edge to it is changed) at one of its two slots, one in each half (cuckoo hashing): a
+// lookup is two loads and two comparisons with no loop. Addressed by 32-bit shared addresses.
+struct HubSet {
+  uint32_t base;
+  int bits;
+  __device__ __forceinline__ uint32_t slot1(const uint32_t x) const { return ((x >> (30 - bits)) & ~3u) + base; }
+  __device__ __forceinline__ uint32_t slot2(const uint32_t x) const {
+    return ((x >> (30 - 2 * bits)) & ((4u << bits) - 4u)) + (base + (4u << bits));
   }
+};
+constexpr int32_t kHubFree = -1;  // no key: ids are below INT32_MAX
+constexpr int32_t kHubNone = -2;  // an entry that is not there: equals no id
+constexpr int kHubKicks = 64;
+
+__device__ __forceinline__ uint32_t hub_hash(const int32_t id) { return (uint32_t)id * 0x9E3779B1u; }
+__device__ __forceinline__ int32_t hub_lds(const uint32_t at) {
+  int32_t v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(at));
+  return v;
 }
 
-// Is id in the table? If so, `changed` = its stored mark bit (the edge (h, id) is changed).
-__device__ __forceinline__ bool hub_find(const int32_t* keys, int bits, int32_t id, bool& changed) {
-  const uint32_t bmask = (1u << bits) - 1;
-  uint32_t b = hub_bucket(id, bits);
-  for (uint32_t it = 0; it <= bmask; ++it) {
-    const int4 q = *reinterpret_cast<const int4*>(keys + 4 * b);
-    if ((q.x & INT32_MAX) == id) { changed = q.x < 0; return true; }
-    if ((q.y & INT32_MAX) == id) { changed = q.y < 0; return true; }
-    if ((q.z & INT32_MAX) == id) { changed = q.z < 0; return true; }
-    if ((q.w & INT32_MAX) == id) { changed = q.w < 0; return true; }
-    if (q.w == -1) return false;  // slots fill in order: a free slot ends the probe
-    b = (b + 1) & bmask;
+// Insert a key (concurrently with others): into its first slot, the key found there into its other
+// one, and so on; false when a key is left over.
+__device__ __forceinline__ bool hub_insert(const HubSet& t, int32_t key) {
+  uint32_t at = t.slot1(hub_hash(key & INT32_MAX));
+  for (int it = 0; it < kHubKicks; ++it) {
+    asm volatile("atom.shared.exch.b32 %0, [%1], %0;" : "+r"(key) : "r"(at) : "memory");
+    if (key == kHubFree) return true;
+    const uint32_t x = hub_hash(key & INT32_MAX), s1 = t.slot1(x);
+    at = at == s1 ? t.slot2(x) : s1;
   }
   return false;
 }
 
 // Work items of the hubs from one queue: item (hub, j) is pass j / C over unit chunk j % C of the
-// hub's C chunks; its warps walk one unit each.
+// hub's C chunks; its warps walk one unit each. A pass whose table cannot be built (ids chosen
+// against the hash) is taken in halves. Bound by its instructions and the partner lists' loads: with
+// 16-byte buckets of four keys and the marks read after a hit, a pass of 2 x 10^6 updates on R-MAT 22
+// spent 6.98 ms here, with two-slot sets and the marks beside the entries 4.96 ms.
 __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const DeltaArgs A, const HubWs H,
                                                                           uint32_t* __restrict__ pv,
                                                                           unsigned long long* __restrict__ tri_out) {
@@ -1606,6 +1612,8 @@ __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const 
   __shared__ unsigned long long s_item;
   __shared__ int s_next;
   __shared__ unsigned long long s_red[kHubThreads / 32][2];
+  uint32_t table;
+  asm volatile("mov.u32 %0, %1;" : "=r"(table) : "r"((uint32_t)__cvta_generic_to_shared(hub_keys)));
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t n_items = (int64_t)min(*H.n_items, (unsigned long long)H.item_cap);
   const uint32_t inc = A.weight * (uint32_t)A.sign;
@@ -1614,7 +1622,6 @@ __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const 
     if (threadIdx.x == 0) {
       const unsigned long long q = atomicAdd(H.q, 1ull);
       s_item = q < (unsigned long long)n_items ? H.items[q] : ~1ull;
-      s_next = 0;
     }
     __syncthreads();
     const unsigned long long item = s_item;
@@ -1631,81 +1638,94 @@ __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const 
     const int pk = j / C, ci = j % C;
     const int32_t per = (k + C - 1) / C;
     const int32_t e0 = ci * per, e1 = min(k, e0 + per);
-    const int cb = (int)(((int64_t)pk * lh) / P);
-    const int cb_next = (int)(((int64_t)(pk + 1) * lh) / P);
-    const int clen = cb_next - cb;
-    int bits = 4;  // buckets >= clen (load <= 0.25) while they fit, else load <= 0.5
-    while ((1 << bits) < clen && (1 << bits) < kHubBucketsMax) ++bits;
-    const int S = 4 << bits;
-    for (int i = threadIdx.x; i < S; i += kHubThreads) hub_keys[i] = -1;
-    __syncthreads();
-    for (int i = threadIdx.x; i < clen; i += kHubThreads) {
-      const int32_t w = A.g.ind[sh + cb + i];
-      hub_insert(hub_keys, bits, w, A.mark[sh + cb + i] ? (w | kHubMarkBit) : w);
-    }
-    const int32_t vlo = pk == 0 ? INT32_MIN : A.g.ind[sh + cb];
-    const int32_t vhi = pk + 1 == P ? INT32_MAX : A.g.ind[sh + cb_next];
-    __syncthreads();
+    const int cb_end = (int)(((int64_t)(pk + 1) * lh) / P);
     uint32_t hub_c = 0;  // triangles kept at h in this item (lane 0 of each warp)
-    while (true) {
-      int i = 0;
-      if (lane == 0) i = atomicAdd(&s_next, 1);
-      i = e0 + __shfl_sync(kFull, i, 0);
-      if (i >= e1) break;
-      const int2 un = H.units[base + i];
-      const int32_t s = un.x;
-      const int32_t ls = A.g.len(s);
-      const int64_t ss = A.g.start(s);
-      const uint64_t key_hs = ekey(h, s);
-      if (pk == 0 && un.y == 0 && lane == 0) bytes_acc += 4ull * (unsigned long long)(lh + ls) + 8ull;
-      const int32_t c0 = un.y * kHubUnit, c1 = min(ls, c0 + kHubUnit);
-      int32_t cur = c0;
-      if (P > 1) {  // the unit's part in [vlo, vhi), if any
-        const int32_t first = A.g.ind[ss + c0], last = A.g.ind[ss + c1 - 1];
-        if (last < vlo || first >= vhi) continue;
-        if (first < vlo) cur = c0 + warp_lower_bound(A.g.ind + ss + c0, c1 - c0, vlo);
-      }
-      uint32_t c = 0;
-      // N(s)[cur, c1) up to the first entry >= vhi, 128 entries per step (four loads per lane)
-      while (cur < c1) {
-        int32_t w[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int32_t q = cur + lane + 32 * t;
-          w[t] = q < c1 ? A.g.ind[ss + q] : INT32_MAX;
+    int cb = (int)(((int64_t)pk * lh) / P);
+    int clen = cb_end - cb;
+    HubSet t{table, 4};
+    while ((3 << t.bits) < 4 * clen && t.bits < kHubSlotBits) ++t.bits;  // load <= 3/8
+    for (; cb < cb_end; cb += clen) {
+      clen = min(clen, cb_end - cb);
+      while (true) {
+        for (int i = threadIdx.x; i < (2 << t.bits) / 4; i += kHubThreads)
+          reinterpret_cast<int4*>(hub_keys)[i] = make_int4(kHubFree, kHubFree, kHubFree, kHubFree);
+        if (threadIdx.x == 0) s_next = 0;
+        __syncthreads();
+        bool ok = true;
+        for (int i = threadIdx.x; i < clen; i += kHubThreads) {
+          const int32_t w = A.g.ind[sh + cb + i];
+          ok &= hub_insert(t, A.mark[sh + cb + i] ? (w | kHubMarkBit) : w);
         }
-        int n_in = 0;
+        if (__syncthreads_and(ok)) break;
+        clen = (clen + 1) / 2;
+      }
+      const bool ranged = clen < lh;
+      const int32_t vlo = cb == 0 ? INT32_MIN : A.g.ind[sh + cb];
+      const int32_t vhi = cb + clen == lh ? INT32_MAX : A.g.ind[sh + cb + clen];
+      while (true) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&s_next, 1);
+        i = e0 + __shfl_sync(kFull, i, 0);
+        if (i >= e1) break;
+        const int2 un = H.units[base + i];
+        const int32_t s = un.x;
+        const int32_t ls = A.g.len(s);
+        const int64_t ss = A.g.start(s);
+        if (cb == 0 && un.y == 0 && lane == 0) bytes_acc += 4ull * (unsigned long long)(lh + ls) + 8ull;
+        int32_t cur = un.y * kHubUnit, end = min(ls, cur + kHubUnit);
+        if (ranged) {  // the unit's part in [vlo, vhi), if any
+          const int32_t* const u = A.g.ind + ss + cur;
+          const int32_t len = end - cur, first = u[0], last = u[len - 1];
+          if (last < vlo || first >= vhi) continue;
+          if (last >= vhi) end = cur + warp_lower_bound(u, len, vhi);
+          if (first < vlo) cur += warp_lower_bound(u, len, vlo);
+        }
+        const int32_t* lst = A.g.ind + ss + cur + lane;
+        const uint8_t* mrk = A.mark + ss + cur + lane;
+        uint32_t c = 0;
+        // N(s)[cur, end), 128 entries per step: four loads per lane, and the entries' marks beside them
+        for (int32_t left = end - cur - lane; left > -lane; left -= 128, lst += 128, mrk += 128) {
+          int32_t w[4];
+          uint32_t m[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const bool in = w[t] < vhi;
-          n_in += __popc(__ballot_sync(kFull, in));
-          bool ch = false;
-          if (in && hub_find(hub_keys, bits, w[t], ch)) {
-            const bool cs = A.mark[ss + cur + lane + 32 * t] != 0;
-            if ((!ch || key_hs < ekey(h, w[t])) && (!cs || key_hs < ekey(s, w[t]))) {
+          for (int r = 0; r < 4; ++r) {
+            w[r] = left > 32 * r ? lst[32 * r] : kHubNone;
+            m[r] = left > 32 * r ? mrk[32 * r] : 0;
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const uint32_t x = hub_hash(w[r]);
+            const int32_t q1 = hub_lds(t.slot1(x)), q2 = hub_lds(t.slot2(x));
+            const bool f = (q1 & INT32_MAX) == w[r], g = (q2 & INT32_MAX) == w[r];
+            bool keep = f | g;
+            const bool ch = (f ? q1 : q2) < 0;  // (h, w) is changed
+            if (keep && (ch || m[r])) {         // or (s, w) is: the triangle is the smallest changed edge's
+              const uint64_t key_hs = ekey(h, s);
+              keep = (!ch || key_hs < ekey(h, w[r])) && (!m[r] || key_hs < ekey(s, w[r]));
+            }
+            if (keep) {
               ++c;
-              atomicAdd(&pv[w[t]], inc);
+              atomicAdd(&pv[w[r]], inc);
             }
           }
           __syncwarp();
         }
-        cur += n_in;  // the entries below vhi are a prefix of the step (the list ascends)
-        if (n_in < 128) break;
+        c = __reduce_add_sync(kFull, c);
+        if (lane == 0 && c) {
+          atomicAdd(&pv[s], c * inc);
+          hub_c += c;
+          tri_acc += c;
+        }
       }
-      c = warp_sum(c);
-      if (lane == 0 && c) {
-        atomicAdd(&pv[s], c * inc);
-        hub_c += c;
-        tri_acc += c;
-      }
+      __syncthreads();
     }
     // h's per-vertex count: one atomic per item
     if (lane == 0) s_red[wid][0] = hub_c;
     __syncthreads();
     if (threadIdx.x == 0) {
-      unsigned long long t = 0;
-      for (int w = 0; w < kHubThreads / 32; ++w) t += s_red[w][0];
-      if (t) atomicAdd(&pv[h], (uint32_t)t * inc);
+      unsigned long long sum = 0;
+      for (int w = 0; w < kHubThreads / 32; ++w) sum += s_red[w][0];
+      if (sum) atomicAdd(&pv[h], (uint32_t)sum * inc);
       if (j == 0) H.of[h] = 0;  // zero between phases (k_hub_place, its last reader, is done)
     }
     __syncthreads();
@@ -2227,7 +2247,7 @@ tc_status fused_grid(int ctas_per_sm, size_t smem, int* grid) {
   return TC_OK;
 }
 
-constexpr size_t kHubSmem = sizeof(int32_t) * 4 * kHubBucketsMax;
+constexpr size_t kHubSmem = sizeof(int32_t) * (2 << kHubSlotBits);
 
 // Grid of the hub kernel: its occupancy limit of CTAs per SM (64 KB of shared memory each).
 tc_status hub_grid(int* grid) {
