@@ -37,8 +37,8 @@ constexpr int kDeltaChunk = 1024;   // ... into items of this many entries of th
 constexpr int64_t kDeltaItems = 1 << 20;  // capacity of the split-item queue
 constexpr unsigned long long kNoItem = ~0ull;
 constexpr int kGrab = 4;  // most changed edges a warp takes per grab from the delta kernel's queue
-// Bound of the persistent delta kernel's waits for queued split items (a wait that runs out
-// reports kErrTimeout and the warp leaves the item pass).
+// Bound of the wait in which the persistent delta kernel's CTAs meet (a wait that runs out reports
+// kErrTimeout).
 constexpr unsigned long long kSpinNs = 2000000000ull;  // 2 s
 constexpr unsigned kSpinMaxIters = 1u << 24;
 
@@ -48,7 +48,6 @@ constexpr int32_t kNoDel = 0x7f7f7f7f;
 constexpr unsigned long long kNoLongItem = ~0ull;
 
 struct BatchStatus {
-  unsigned long long n_uniq;      // unique undirected edges
   unsigned long long n_del;       // effective deletions
   unsigned long long n_ins;       // effective insertions
   unsigned long long n_dir;       // directed insert entries (2 n_ins)
@@ -68,7 +67,7 @@ struct BatchStatus {
   unsigned long long cmp_items;
   unsigned long long n_split[2];  // split-intersection items queued (deletions, insertions)
   unsigned long long delta_bytes; // algorithmic bytes of the batch's intersections (4(deg x + deg y) + 8 each)
-  unsigned int entry_done[2];     // warps of the persistent delta kernel done with the entry pass
+  unsigned int arrived[2];        // CTAs of the persistent delta kernel done with the count
   unsigned int err;
   unsigned int pad;
   unsigned long long n_hubs[2];   // hub groups of the delta count (deletions, insertions)
@@ -130,18 +129,10 @@ __device__ __forceinline__ void cp_async4(int32_t* smem_dst, const int32_t* gsrc
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// GPU-scope release store and acquire loads (publication of work items between CTAs).
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+// GPU-scope relaxed load (a poll of another CTA's arrival).
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
   unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -152,47 +143,122 @@ int grid_for(int64_t items, int per_block) {
 
 // ---- batch preparation (canonical undirected updates) --------------------------------------
 
-// key = (min << (L+1)) | (max << 1) | is_insert; self-loops and bad ids become the sentinel.
-__global__ void k_make_keys(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
-                            const uint8_t* __restrict__ is_del, const int64_t b, const int32_t n, const int L,
-                            uint64_t* __restrict__ keys, BatchStatus* __restrict__ st) {
+// key = (min << (L+1)) | (max << 1) | is_insert; self-loops and bad ids become the sentinel
+// (1 << (2L+1)) - 1, and so do the entries [b, cap) of a padded batch.
+__device__ __forceinline__ uint64_t update_key(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+                                               const uint8_t* __restrict__ is_del, const int64_t i, const int64_t b,
+                                               const int32_t n, const int L, BatchStatus* __restrict__ st) {
   const uint64_t sent = (1ull << (2 * L + 1)) - 1;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t s = src[i], d = dst[i];
-    uint64_t k = sent;
-    if (s < 0 || s >= n || d < 0 || d >= n) {
-      atomicOr(&st->err, kErrRange);
-    } else if (s != d) {
-      const uint64_t lo = (uint64_t)min(s, d), hi = (uint64_t)max(s, d);
-      k = (lo << (L + 1)) | (hi << 1) | (uint64_t)((is_del && is_del[i]) ? 0 : 1);
-    }
-    keys[i] = k;
+  if (i >= b) return sent;
+  const int32_t s = src[i], d = dst[i];
+  if (s < 0 || s >= n || d < 0 || d >= n) {
+    atomicOr(&st->err, kErrRange);
+    return sent;
+  }
+  if (s == d) return sent;
+  const uint64_t lo = (uint64_t)min(s, d), hi = (uint64_t)max(s, d);
+  return (lo << (L + 1)) | (hi << 1) | (uint64_t)((is_del && is_del[i]) ? 0 : 1);
+}
+
+// The keys of a batch of b updates, padded to cap entries, and the directed keys' padding.
+__global__ void __launch_bounds__(kThreads) k_load_keys(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+                                                        const uint8_t* __restrict__ is_del, const int64_t b,
+                                                        const int64_t cap, const int32_t n, const int L,
+                                                        uint64_t* __restrict__ keys, uint64_t* __restrict__ dirkeys,
+                                                        BatchStatus* __restrict__ st) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (int64_t)gridDim.x * blockDim.x) {
+    keys[i] = update_key(src, dst, is_del, i, b, n, L, st);
+    reinterpret_cast<ulonglong2*>(dirkeys)[i] = make_ulonglong2(kSentinel, kSentinel);
   }
 }
 
-__global__ void k_run_heads(const uint64_t* __restrict__ keys, const int64_t b, const uint64_t sent,
-                            int32_t* __restrict__ head) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
-    head[i] = (k != sent) && (i == 0 || (keys[i - 1] >> 1) != (k >> 1));
+// ---- small batches: sorted by one CTA ------------------------------------------------------
+//
+// A batch of at most kSmallBatch updates is bound by its launches: each of the library sort's is 13 us
+// or more here, between kernels of a few dependent loads. One CTA sorts its keys in shared memory
+// instead, in the kernels that make them and use them.
+constexpr int64_t kSmallBatch = 2048;
+constexpr int kSortThreads = 1024;
+
+// Ascending bitonic sort of P (a power of two) keys in shared memory by the CTA.
+__device__ __forceinline__ void cta_sort(uint64_t* __restrict__ k, const int P) {
+  for (int size = 2; size <= P; size <<= 1) {
+    for (int h = size >> 1; h > 0; h >>= 1) {
+      for (int p = threadIdx.x; p < P / 2; p += kSortThreads) {
+        const int i = ((p & ~(h - 1)) << 1) | (p & (h - 1)), j = i | h;
+        const uint64_t x = k[i], y = k[j];
+        if ((x > y) == ((i & size) == 0)) {
+          k[i] = y;
+          k[j] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+__device__ __forceinline__ int pow2_at_least(const int64_t n) {
+  int P = 32;
+  while (P < n) P <<= 1;
+  return P;
+}
+
+// The sorted keys of a batch of b <= cap <= kSmallBatch updates, padded to cap.
+__global__ void __launch_bounds__(kSortThreads) k_load_sorted(const int32_t* __restrict__ src,
+                                                              const int32_t* __restrict__ dst,
+                                                              const uint8_t* __restrict__ is_del, const int64_t b,
+                                                              const int64_t cap, const int32_t n, const int L,
+                                                              uint64_t* __restrict__ sorted, BatchStatus* __restrict__ st) {
+  __shared__ uint64_t k[kSmallBatch];
+  const int P = pow2_at_least(b);
+  for (int i = threadIdx.x; i < P; i += kSortThreads) k[i] = update_key(src, dst, is_del, i, b, n, L, st);
+  __syncthreads();
+  cta_sort(k, P);
+  const uint64_t sent = (1ull << (2 * L + 1)) - 1;
+  for (int i = threadIdx.x; i < cap; i += kSortThreads) sorted[i] = i < P ? k[i] : sent;
+}
+
+// ---- classification ------------------------------------------------------------------------
+
+// The run of equal edges starting at i, if one does: does it delete, does it insert.
+__device__ __forceinline__ bool edge_run(const uint64_t* __restrict__ keys, const int64_t i, const int64_t b, const int L,
+                                         bool& del_any, bool& ins_any) {
+  const uint64_t k = keys[i], e = k >> 1;
+  if (k == (1ull << (2 * L + 1)) - 1 || (i > 0 && (keys[i - 1] >> 1) == e)) return false;
+  int64_t j = i;
+  while (j + 1 < b && (keys[j + 1] >> 1) == e) ++j;
+  del_any = (k & 1ull) == 0;        // deletions sort before insertions of the same edge
+  ins_any = (keys[j] & 1ull) == 1;
+  return true;
+}
+
+// Append an effective deletion (the edge's places in both lists) or insertion (its directed keys,
+// (src << L) | dst).
+__device__ __forceinline__ void append_change(const bool is_del, const int32_t x, const int32_t y, const int32_t px,
+                                              const int32_t py, const int L, int4* __restrict__ dlist,
+                                              int2* __restrict__ ilist, uint64_t* __restrict__ dirkeys,
+                                              BatchStatus* __restrict__ st) {
+  if (is_del) {
+    dlist[atomicAdd(&st->n_del, 1ull)] = make_int4(x, y, px, py);
+  } else {
+    const unsigned long long at = atomicAdd(&st->n_ins, 1ull);
+    ilist[at] = make_int2(x, y);
+    dirkeys[2 * at] = ((uint64_t)(uint32_t)x << L) | (uint32_t)y;
+    dirkeys[2 * at + 1] = ((uint64_t)(uint32_t)y << L) | (uint32_t)x;
   }
 }
 
 // Each unique undirected edge: classify against the graph and append to the deletion or the
-// insertion list. A deletion records the slots of the edge in both lists.
+// insertion list. A thread per key; a deletion records the edge's places in both lists.
 __global__ void k_classify(const SlackView g, const uint64_t* __restrict__ keys, const int64_t b, const int L,
-                           const int32_t* __restrict__ head, int4* __restrict__ dlist, int2* __restrict__ ilist,
-                           uint64_t* __restrict__ dirkeys, BatchStatus* __restrict__ st) {
+                           int4* __restrict__ dlist, int2* __restrict__ ilist, uint64_t* __restrict__ dirkeys,
+                           BatchStatus* __restrict__ st) {
   const uint64_t maxmask = (1ull << L) - 1;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
-    if (!head[i]) continue;
+    bool del_any, ins_any;
+    if (!edge_run(keys, i, b, L, del_any, ins_any)) continue;
     const uint64_t e = keys[i] >> 1;
-    int64_t j = i;
-    while (j + 1 < b && (keys[j + 1] >> 1) == e) ++j;
-    const bool del_any = (keys[i] & 1ull) == 0;  // deletions sort before insertions of the same edge
-    const bool ins_any = (keys[j] & 1ull) == 1;
     const int32_t x = (int32_t)(e >> L), y = (int32_t)(e & maxmask);
-    atomicAdd(&st->n_uniq, 1ull);
     // presence: search the shorter list
     const int32_t lx = g.len(x), ly = g.len(y);
     const int64_t sx = g.start(x), sy = g.start(y);
@@ -208,277 +274,94 @@ __global__ void k_classify(const SlackView g, const uint64_t* __restrict__ keys,
     if (del_any && !ins_any && present) {
       if (px < 0) px = lower_bound(g.ind, sx, sx + lx, y) - sx;
       if (py < 0) py = lower_bound(g.ind, sy, sy + ly, x) - sy;
-      const unsigned long long at = atomicAdd(&st->n_del, 1ull);
-      dlist[at] = make_int4(x, y, (int32_t)px, (int32_t)py);
+      append_change(true, x, y, (int32_t)px, (int32_t)py, L, dlist, ilist, dirkeys, st);
     } else if (ins_any && !present) {
-      const unsigned long long at = atomicAdd(&st->n_ins, 1ull);
-      ilist[at] = make_int2(x, y);
-      dirkeys[2 * at] = ((uint64_t)(uint32_t)x << 32) | (uint32_t)y;
-      dirkeys[2 * at + 1] = ((uint64_t)(uint32_t)y << 32) | (uint32_t)x;
+      append_change(false, x, y, 0, 0, L, dlist, ilist, dirkeys, st);
     }
+  }
+}
+
+// The same, a warp per key: 32 samples a round, so a list of 10^5 entries takes four dependent loads
+// instead of seventeen. For batches that leave most warps idle otherwise.
+__global__ void k_classify_warp(const SlackView g, const uint64_t* __restrict__ keys, const int64_t b, const int L,
+                                int4* __restrict__ dlist, int2* __restrict__ ilist, uint64_t* __restrict__ dirkeys,
+                                BatchStatus* __restrict__ st) {
+  const uint64_t maxmask = (1ull << L) - 1;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < b; i += nw) {
+    bool del_any, ins_any;
+    if (!edge_run(keys, i, b, L, del_any, ins_any)) continue;
+    const uint64_t e = keys[i] >> 1;
+    const int32_t x = (int32_t)(e >> L), y = (int32_t)(e & maxmask);
+    const int32_t lx = g.len(x), ly = g.len(y);
+    const int32_t* const nx = g.ind + g.start(x);
+    const int32_t* const ny = g.ind + g.start(y);
+    const bool x_short = lx <= ly;
+    const int32_t ps = x_short ? warp_lower_bound(nx, lx, y) : warp_lower_bound(ny, ly, x);
+    const bool present = x_short ? ps < lx && nx[ps] == y : ps < ly && ny[ps] == x;
+    if (del_any && !ins_any && present) {
+      const int32_t pl = x_short ? warp_lower_bound(ny, ly, x) : warp_lower_bound(nx, lx, y);
+      if (lane == 0) append_change(true, x, y, x_short ? ps : pl, x_short ? pl : ps, L, dlist, ilist, dirkeys, st);
+    } else if (ins_any && !present) {
+      if (lane == 0) append_change(false, x, y, 0, 0, L, dlist, ilist, dirkeys, st);
+    }
+    __syncwarp();
   }
 }
 
 // ---- insertion planning / application ------------------------------------------------------
 
-// Heads of source-vertex runs in the sorted directed entries, and the pool slots the lists that
-// must move could take (computed on the pre-deletion lengths, an upper bound).
-// A run whose list will be long (used + new > kLongList) is stored as -1 - start and also listed
-// (start, length) in long_runs / long_cnt for the long-list insertion; the warp kernel skips it.
-__global__ void k_dir_runs(const uint64_t* __restrict__ dk, const int64_t nd_cap, const int32_t* __restrict__ used,
-                           const int32_t* __restrict__ cap, const int32_t slack_q10, int32_t* __restrict__ run_start,
-                           int32_t* __restrict__ long_runs, int32_t* __restrict__ long_cnt,
-                           BatchStatus* __restrict__ st) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd_cap; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = dk[i];
-    if (k == kSentinel) continue;
-    const uint32_t v = (uint32_t)(k >> 32);
-    if (i > 0 && (uint32_t)(dk[i - 1] >> 32) == v) continue;
-    int64_t j = i;
-    while (j + 1 < nd_cap && dk[j + 1] != kSentinel && (uint32_t)(dk[j + 1] >> 32) == v) ++j;
-    const int32_t c = (int32_t)(j - i + 1);
-    const unsigned long long r = atomicAdd(&st->n_runs, 1ull);
-    const int32_t need = used[v] + c;
-    if (need > kLongList) {
-      run_start[r] = -1 - (int32_t)i;
-      const unsigned long long q = atomicAdd(&st->n_long, 1ull);
-      long_runs[q] = (int32_t)i;
-      long_cnt[q] = c;
-    } else {
-      run_start[r] = (int32_t)i;
-    }
-    if (need > cap[v]) atomicAdd(&st->demand, (unsigned long long)slack_capacity(need, max(slack_q10, 256)));
-  }
+__device__ __forceinline__ int32_t dir_src(const uint64_t k, const int L) { return (int32_t)(k >> L); }
+__device__ __forceinline__ int32_t dir_dst(const uint64_t k, const int L) {
+  return (int32_t)((uint32_t)k & (uint32_t)((1ull << L) - 1));
 }
 
-// One warp per affected source vertex: merge its sorted new neighbours into its list, in place
-// (backwards) when the capacity allows, else into a fresh block at the pool top. New slots are
-// marked (mark = 1) when `mark` is given; their absolute slots go to slot[].
-__global__ void k_insert_runs(const uint64_t* __restrict__ dk, const int64_t nd_cap, const int32_t* __restrict__ run_start,
-                              int64_t* __restrict__ start, int32_t* __restrict__ used, int32_t* __restrict__ cap,
-                              int32_t* __restrict__ pool, const int64_t pool_cap, uint8_t* __restrict__ mark,
-                              int64_t* __restrict__ slot, unsigned long long* __restrict__ pool_top,
-                              const int32_t slack_q10, BatchStatus* __restrict__ st) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t nruns = (int64_t)st->n_runs;
-  for (int64_t r = gw; r < nruns; r += nw) {
-    const int64_t i0 = run_start[r];
-    if (i0 < 0) continue;  // a long list: k_long_plan / k_long_stage / k_long_write
-    const int32_t v = (int32_t)(dk[i0] >> 32);
-    int64_t i1 = i0;  // run end (exclusive), found cooperatively
-    {
-      int64_t k = i0 + lane;
-      while (true) {
-        const bool same = k < nd_cap && dk[k] != kSentinel && (int32_t)(dk[k] >> 32) == v;
-        __syncwarp();
-        const unsigned m = __ballot_sync(kFull, same);
-        if (m != kFull) {
-          i1 = k - lane + __ffs(~m) - 1;
-          break;
-        }
-        k += 32;
-      }
-      i1 = __shfl_sync(kFull, i1, 0);
-    }
-    const int32_t c = (int32_t)(i1 - i0);
-    const int32_t a = used[v];
-    const int64_t s_old = start[v];
-    int64_t s_new = s_old;
-    bool moved = false;
-    if (a + c > cap[v]) {
-      const int32_t nc = slack_capacity(a + c, max(slack_q10, 256));
-      unsigned long long at = 0;
-      if (lane == 0) at = atomicAdd(pool_top, (unsigned long long)nc);
-      __syncwarp();
-      at = __shfl_sync(kFull, at, 0);
-      __syncwarp();
-      if ((int64_t)at + nc > pool_cap) {
-        if (lane == 0) atomicOr(&st->err, kErrPool);
-        for (int64_t j = i0 + lane; j < i1; j += 32) slot[j] = -1;  // nothing to clear later
-        continue;  // cannot happen when the host sized the pool from the demand pass
-      }
-      s_new = (int64_t)at;
-      moved = true;
-      if (lane == 0) {
-        cap[v] = nc;
-        atomicAdd(&st->not_fitting, (unsigned long long)c);
-      }
-    }
-    const int32_t* A = pool + s_old;
-    // New entries first, while A is intact: final position j + #(old < B[j]) (relative). The
-    // first five levels of each search come from 32 evenly spaced samples of A held in the lanes.
-    int32_t first_new = a;  // old entries below the smallest new entry keep their slots
-    {
-      const int32_t step = (a + 31) / 32;
-      const int32_t smp = lane * step < a ? A[lane * step] : INT32_MAX;
-      const int32_t s31 = __shfl_sync(kFull, smp, 31);
-      for (int64_t jb = i0; jb < i1; jb += 32) {
-        const int64_t j = jb + lane;
-        const bool act = j < i1;
-        const int32_t val = act ? (int32_t)(uint32_t)dk[j] : INT32_MAX;
-        int pos = 0;  // samples below val (they ascend with the lane)
-#pragma unroll
-        for (int st = 16; st > 0; st >>= 1)
-          if (__shfl_sync(kFull, smp, pos + st - 1) < val) pos += st;
-        if (pos == 31 && s31 < val) pos = 32;
-        int32_t lo = pos > 0 ? (pos - 1) * step + 1 : 0;
-        int32_t hi = pos < 32 ? min(pos * step, a) : a;
-        if (act) {
-          while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
-            if (A[mid] < val) lo = mid + 1;
-            else hi = mid;
-          }
-          slot[j] = (j - i0) + lo;
-          if (j == i0) first_new = lo;
-        }
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-    // In place, old entries below the first new entry do not move; relocated, all of them do.
-    const int32_t keep_below = moved ? 0 : __shfl_sync(kFull, first_new, 0);
-    // Old entries: final position i + #(new < A[i]); backwards in chunks so that, in place, no
-    // unread entry is overwritten (targets never precede sources). Each chunk's entries are read
-    // one chunk ahead: the writes of a chunk go to slots at or above its own.
-    const int32_t low = (keep_below / 32) * 32;
-    int32_t base = a > 0 ? ((a - 1) / 32) * 32 : -1;
-    int32_t ahead = (base >= low && base + lane < a && base + lane >= keep_below) ? A[base + lane] : 0;
-    for (; base >= low; base -= 32) {
-      const int32_t i = base + lane;
-      const bool act = i < a && i >= keep_below;
-      const int32_t val = ahead;
-      const int32_t inext = i - 32;
-      ahead = (base - 32 >= low && inext >= keep_below) ? A[inext] : 0;
-      int64_t pos = 0;
-      if (act) {
-        int64_t lo = i0, hi = i1;
-        while (lo < hi) {
-          const int64_t mid = (lo + hi) >> 1;
-          if ((int32_t)(uint32_t)dk[mid] < val) lo = mid + 1;
-          else hi = mid;
-        }
-        pos = i + (lo - i0);
-      }
-      __syncwarp();
-      if (act) {
-        pool[s_new + pos] = val;
-        if (mark) mark[s_new + pos] = 0;
-      }
-      __syncwarp();
-    }
-    // New entries into the holes.
-    for (int64_t j = i0 + lane; j < i1; j += 32) {
-      const int64_t pos = s_new + slot[j];
-      pool[pos] = (int32_t)(uint32_t)dk[j];
-      if (mark) mark[pos] = 1;
-      slot[j] = pos;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      used[v] = a + c;
-      if (moved) start[v] = s_new;
-      atomicAdd(&st->dir_added, (unsigned long long)c);
-    }
-  }
+// Heads of source-vertex runs in the sorted directed entries ((src << L) | dst), and the pool slots
+// the lists that must move could take (computed on the pre-deletion lengths, an upper bound).
+// A run whose list will be long (used + new > kLongList) is stored as -1 - start.
+__device__ __forceinline__ void dir_run(const uint64_t* __restrict__ dk, const int64_t i, const int64_t nd_cap, const int L,
+                                        const int32_t* __restrict__ used, const int32_t* __restrict__ cap,
+                                        const int32_t slack_q10, int32_t* __restrict__ run_start,
+                                        BatchStatus* __restrict__ st) {
+  const uint64_t k = dk[i];
+  if (k == kSentinel) return;
+  const uint32_t v = (uint32_t)(k >> L);
+  if (i > 0 && (uint32_t)(dk[i - 1] >> L) == v) return;
+  int64_t j = i;
+  while (j + 1 < nd_cap && dk[j + 1] != kSentinel && (uint32_t)(dk[j + 1] >> L) == v) ++j;
+  const int32_t c = (int32_t)(j - i + 1);
+  const unsigned long long r = atomicAdd(&st->n_runs, 1ull);
+  const int32_t need = used[v] + c;
+  run_start[r] = need > kLongList ? -1 - (int32_t)i : (int32_t)i;
+  if (need > cap[v]) atomicAdd(&st->demand, (unsigned long long)slack_capacity(need, max(slack_q10, 256)));
 }
 
-// Clear the marks of the inserted slots: n_host entries, or 2 * (*n_dev) when n_dev is given.
-__global__ void k_clear_slots(const int64_t* __restrict__ slot, const int64_t n_host,
-                              const unsigned long long* __restrict__ n_dev, uint8_t* __restrict__ mark) {
-  const int64_t n = n_dev ? 2 * (int64_t)(*n_dev) : n_host;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = slot[i];
-    if (s >= 0) mark[s] = 0;
-  }
+__global__ void k_dir_runs(const uint64_t* __restrict__ dk, const int64_t nd_cap, const int L,
+                           const int32_t* __restrict__ used, const int32_t* __restrict__ cap, const int32_t slack_q10,
+                           int32_t* __restrict__ run_start, BatchStatus* __restrict__ st) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd_cap; i += (int64_t)gridDim.x * blockDim.x)
+    dir_run(dk, i, nd_cap, L, used, cap, slack_q10, run_start, st);
 }
 
-// ---- deletion -------------------------------------------------------------------------------
-
-// Mark the slots of the batch's deletions and keep each list's smallest marked slot (the
-// compaction leaves the entries below it in place).
-__global__ void k_mark_deletions(const int4* __restrict__ dlist, const BatchStatus* __restrict__ st,
-                                 const int64_t* __restrict__ start, uint8_t* __restrict__ mark,
-                                 int32_t* __restrict__ first_del) {
-  const int64_t nd = (int64_t)st->n_del;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
-    const int4 d = dlist[i];
-    mark[start[d.x] + d.z] = 1;
-    mark[start[d.y] + d.w] = 1;
-    atomicMin(&first_del[d.x], d.z);
-    atomicMin(&first_del[d.y], d.w);
-  }
+// A small batch's directed keys sorted by one CTA (padded with sentinels to 2 * cap), and their runs.
+__global__ void __launch_bounds__(kSortThreads) k_sort_runs(const uint64_t* __restrict__ dk, const int64_t cap, const int L,
+                                                            uint64_t* __restrict__ sorted, const int32_t* __restrict__ used,
+                                                            const int32_t* __restrict__ vcap, const int32_t slack_q10,
+                                                            int32_t* __restrict__ run_start,
+                                                            BatchStatus* __restrict__ st) {
+  __shared__ uint64_t k[2 * kSmallBatch];
+  const int64_t n = 2 * (int64_t)st->n_ins;
+  const int P = pow2_at_least(n);
+  for (int i = threadIdx.x; i < P; i += kSortThreads) k[i] = i < n ? dk[i] : kSentinel;
+  __syncthreads();
+  cta_sort(k, P);
+  for (int i = threadIdx.x; i < 2 * cap; i += kSortThreads) sorted[i] = i < P ? k[i] : kSentinel;
+  for (int i = threadIdx.x; i < n; i += kSortThreads)
+    dir_run(k, i, n, L, used, vcap, slack_q10, run_start, st);
 }
 
-// Remove marked slots from the lists of the vertices in vlist (each vertex once: the first warp
-// to claim it with this epoch compacts it), then clear the marks of the old range. The entries
-// below the list's first marked slot (first_del, reset here to kNoDel) stay where they are.
-__global__ void k_compact_marked(const int32_t* __restrict__ vlist, const int64_t nv_list, const int stride,
-                                 const unsigned long long* __restrict__ nv_dev, const int64_t* __restrict__ start,
-                                 int32_t* __restrict__ used, int32_t* __restrict__ pool, uint8_t* __restrict__ mark,
-                                 unsigned* __restrict__ claim, const unsigned* __restrict__ epoch_dev,
-                                 int32_t* __restrict__ first_del, BatchStatus* __restrict__ st) {
-  const int lane = threadIdx.x & 31;
-  const unsigned epoch = *epoch_dev;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t cnt = nv_dev ? (int64_t)(*nv_dev) * stride : nv_list;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int64_t k = gw; k < cnt; k += nw) {
-    const int32_t v = vlist[k];
-    if (used[v] > kLongList) continue;  // a long list: k_cmp_plan / stage / prefix / write
-    unsigned old = 0;
-    if (lane == 0) old = atomicMax(&claim[v], epoch);
-    __syncwarp();
-    old = __shfl_sync(kFull, old, 0);
-    if (old >= epoch) continue;
-    const int64_t s = start[v];
-    const int32_t a = used[v];
-    const int32_t f = min(first_del[v], a);
-    __syncwarp();
-    if (lane == 0) first_del[v] = kNoDel;
-    int32_t wp = f;
-    for (int32_t base = f; base < a; base += 32) {
-      const int32_t i = base + lane;
-      int32_t val = 0;
-      bool keep = false;
-      if (i < a) {
-        val = pool[s + i];
-        keep = mark[s + i] == 0;
-      }
-      __syncwarp();
-      const unsigned m = __ballot_sync(kFull, keep);
-      __syncwarp();
-      if (keep) pool[s + wp + __popc(m & lt)] = val;
-      wp += __popc(m);
-      __syncwarp();
-    }
-    for (int32_t i = f + lane; i < a; i += 32) mark[s + i] = 0;
-    if (lane == 0) {
-      used[v] = wp;
-      atomicAdd(&st->dir_removed, (unsigned long long)(a - wp));
-    }
-  }
-}
-
-
-// Insertion into long lists (more than kLongList entries after the batch), in three launches
-// over all of the batch's long runs at once:
-//   k_long_plan   one thread per run: relocation (when the list outgrows its capacity) or the
-//                 in-place merge's first moving entry (the first new entry's slot), the list's
-//                 new length, a range of the scratch buffer and work items of kLongChunk entries;
-//   k_long_stage  one CTA per item: each moving old entry and each new entry computes its place
-//                 in the merged suffix (an old entry shifts by the number of new entries below it,
-//                 a new entry lands after the old entries below it) and writes there in scratch;
-//   k_long_write  one CTA per item: the merged suffix back into the list, with the new entries'
-//                 marks.
-// The launch boundary between staging and writing takes the place of an in-place merge's block
-// barriers: every source is read before any target is written, so a hub list of 10^5 entries is
-// spread over many CTAs instead of being one CTA's chain of steps.
-constexpr int kLongChunk = 4096;
-
+// The long-list insertion's plan of one run (see k_long_stage).
 struct LongPlan {
   int64_t s_old;   // list start before the batch
   int64_t s_new;   // list start after it (s_old unless relocated)
@@ -490,71 +373,369 @@ struct LongPlan {
   int32_t i0;      // the run's first entry in the sorted directed keys
   int32_t pad;
 };
+constexpr int kLongChunk = 4096;  // entries per work item of the long-list kernels
 
-__global__ void __launch_bounds__(kThreads) k_long_plan(
-    const uint64_t* __restrict__ dk, const int32_t* __restrict__ long_runs, const int32_t* __restrict__ long_cnt,
-    int64_t* __restrict__ start, int32_t* __restrict__ used, int32_t* __restrict__ cap,
-    const int32_t* __restrict__ pool, const int64_t pool_cap, int64_t* __restrict__ slot,
-    unsigned long long* __restrict__ pool_top, const int32_t slack_q10, LongPlan* __restrict__ plan,
-    unsigned long long* __restrict__ items, const int64_t item_cap, const int64_t scr_cap,
-    BatchStatus* __restrict__ st) {
-  const int64_t nlong = (int64_t)st->n_long;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nlong; r += (int64_t)gridDim.x * blockDim.x) {
-    LongPlan P;
-    P.i0 = long_runs[r];
-    P.c = long_cnt[r];
-    P.pad = 0;
-    const int32_t v = (int32_t)(dk[P.i0] >> 32);
-    P.a = used[v];
-    P.s_old = start[v];
-    P.s_new = P.s_old;
+struct InsertArgs {
+  const uint64_t* dk;        // sorted directed keys, nd_cap of them
+  int64_t nd_cap;
+  int L;
+  const int32_t* run_start;
+  int64_t* start;
+  int32_t* used;
+  int32_t* cap;
+  int32_t* pool;
+  int64_t pool_cap;
+  uint8_t* mark;             // new slots are marked when given
+  int64_t* slot;             // absolute slots of the new entries
+  unsigned long long* pool_top;
+  int32_t slack_q10;
+  LongPlan* plan;            // long runs: their plans and work items
+  unsigned long long* items;
+  int64_t item_cap;
+  int64_t scr_cap;
+};
+
+// A long run's plan, by the warp: relocation (done by insert_runs) or the first moving entry, the
+// list's new length, a range of the scratch buffer and work items of kLongChunk entries.
+__device__ __forceinline__ void plan_long_run(const InsertArgs& I, const int32_t v, const int64_t i0, const int32_t a,
+                                              const int32_t c, const int64_t s_old, const int64_t s_new,
+                                              BatchStatus* __restrict__ st) {
+  const int lane = threadIdx.x & 31;
+  LongPlan P;
+  P.s_old = s_old;
+  P.s_new = s_new;
+  P.a = a;
+  P.c = c;
+  P.i0 = (int32_t)i0;
+  P.pad = 0;
+  P.first = s_new == s_old ? warp_lower_bound(I.pool + s_old, a, dir_dst(I.dk[i0], I.L)) : 0;
+  P.len = a - P.first + c;
+  const int32_t nch = (P.len + kLongChunk - 1) / kLongChunk;
+  unsigned long long so = 0, ib = 0, r = 0;
+  if (lane == 0) {
+    so = atomicAdd(&st->long_scr, (unsigned long long)P.len);
+    ib = atomicAdd(&st->long_items, (unsigned long long)nch);
+    r = atomicAdd(&st->n_long, 1ull);
+  }
+  so = __shfl_sync(kFull, so, 0);
+  ib = __shfl_sync(kFull, ib, 0);
+  r = __shfl_sync(kFull, r, 0);
+  const bool ok = (int64_t)(so + P.len) <= I.scr_cap && (int64_t)(ib + nch) <= I.item_cap;
+  for (int32_t j = lane; j < nch; j += 32)
+    if ((int64_t)(ib + j) < I.item_cap) I.items[ib + j] = ok ? (r << 32) | (unsigned)j : kNoLongItem;
+  if (!ok) {  // unreachable while the scratch follows the pool's size
+    for (int32_t j = lane; j < c; j += 32) I.slot[i0 + j] = -1;
     P.len = 0;
-    P.soff = 0;
-    P.first = 0;
-    bool ok = true;
-    if (P.a + P.c > cap[v]) {
-      const int32_t nc = slack_capacity(P.a + P.c, max(slack_q10, 256));
-      const unsigned long long at = atomicAdd(pool_top, (unsigned long long)nc);
-      if ((int64_t)at + nc > pool_cap) {
-        atomicOr(&st->err, kErrPool);
-        ok = false;
-      } else {
-        P.s_new = (int64_t)at;
-        start[v] = P.s_new;
-        cap[v] = nc;
-        atomicAdd(&st->not_fitting, (unsigned long long)P.c);
-      }
-    } else {
-      P.first = (int32_t)(lower_bound(pool, P.s_old, P.s_old + P.a, (int32_t)(uint32_t)dk[P.i0]) - P.s_old);
-    }
+  }
+  P.soff = (int64_t)so;
+  if (lane == 0) {
     if (ok) {
-      P.len = P.a - P.first + P.c;
-      const int32_t nch = (P.len + kLongChunk - 1) / kLongChunk;
-      const unsigned long long so = atomicAdd(&st->long_scr, (unsigned long long)P.len);
-      const unsigned long long ib = atomicAdd(&st->long_items, (unsigned long long)nch);
-      if ((int64_t)(so + P.len) > scr_cap || (int64_t)(ib + nch) > item_cap) {
-        atomicOr(&st->err, kErrScratch);  // unreachable while the scratch follows the pool's size
-        ok = false;
-        for (int32_t j = 0; j < nch && (int64_t)(ib + j) < item_cap; ++j) items[ib + j] = kNoLongItem;
-      } else {
-        P.soff = (int64_t)so;
-        for (int32_t j = 0; j < nch; ++j) items[ib + j] = ((unsigned long long)r << 32) | (unsigned)j;
-        used[v] = P.a + P.c;
-        atomicAdd(&st->dir_added, (unsigned long long)P.c);
+      I.used[v] = a + c;
+      atomicAdd(&st->dir_added, (unsigned long long)c);
+    } else {
+      atomicOr(&st->err, kErrScratch);
+    }
+    I.plan[r] = P;
+  }
+  __syncwarp();
+}
+
+// One warp per affected source vertex: merge its sorted new neighbours into its list, in place
+// (backwards) when the capacity allows, else into a fresh block at the pool top. New slots are
+// marked (mark = 1) when `mark` is given; their absolute slots go to slot[]. A list that will be
+// long is planned here and merged by k_long_stage / k_long_write.
+__global__ void __launch_bounds__(kThreads) k_insert_runs(const InsertArgs I, BatchStatus* __restrict__ st) {
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t nruns = (int64_t)st->n_runs;
+  for (int64_t r = gw; r < nruns; r += nw) {
+    const int32_t at_run = I.run_start[r];
+    const bool is_long = at_run < 0;
+    const int64_t i0 = is_long ? -1 - at_run : at_run;
+    const int32_t v = dir_src(I.dk[i0], I.L);
+    int64_t i1 = i0;  // run end (exclusive), found cooperatively
+    {
+      int64_t k = i0 + lane;
+      while (true) {
+        const bool same = k < I.nd_cap && I.dk[k] != kSentinel && dir_src(I.dk[k], I.L) == v;
+        __syncwarp();
+        const unsigned m = __ballot_sync(kFull, same);
+        if (m != kFull) {
+          i1 = k - lane + __ffs(~m) - 1;
+          break;
+        }
+        k += 32;
+      }
+      i1 = __shfl_sync(kFull, i1, 0);
+    }
+    const int32_t c = (int32_t)(i1 - i0);
+    const int32_t a = I.used[v];
+    const int64_t s_old = I.start[v];
+    int64_t s_new = s_old;
+    bool moved = false;
+    if (a + c > I.cap[v]) {
+      const int32_t nc = slack_capacity(a + c, max(I.slack_q10, 256));
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(I.pool_top, (unsigned long long)nc);
+      __syncwarp();
+      at = __shfl_sync(kFull, at, 0);
+      __syncwarp();
+      if ((int64_t)at + nc > I.pool_cap) {
+        if (lane == 0) atomicOr(&st->err, kErrPool);
+        for (int64_t j = i0 + lane; j < i1; j += 32) I.slot[j] = -1;  // nothing to clear later
+        continue;  // cannot happen when the host sized the pool from the demand pass
+      }
+      s_new = (int64_t)at;
+      moved = true;
+      if (lane == 0) {
+        I.cap[v] = nc;
+        I.start[v] = s_new;
+        atomicAdd(&st->not_fitting, (unsigned long long)c);
       }
     }
-    if (!ok) {
-      P.len = 0;
-      for (int32_t j = 0; j < P.c; ++j) slot[P.i0 + j] = -1;
+    if (is_long) {
+      plan_long_run(I, v, i0, a, c, s_old, s_new, st);
+      continue;
     }
-    plan[r] = P;
+    const int32_t* A = I.pool + s_old;
+    // New entries first, while A is intact: final position j + #(old < B[j]) (relative). The
+    // first five levels of each search come from 32 evenly spaced samples of A held in the lanes.
+    int32_t first_new = a;  // old entries below the smallest new entry keep their slots
+    int32_t mine = INT32_MAX;  // this lane's new entry (runs of at most 32)
+    {
+      const int32_t step = (a + 31) / 32;
+      const int32_t smp = lane * step < a ? A[lane * step] : INT32_MAX;
+      const int32_t s31 = __shfl_sync(kFull, smp, 31);
+      for (int64_t jb = i0; jb < i1; jb += 32) {
+        const int64_t j = jb + lane;
+        const bool act = j < i1;
+        const int32_t val = act ? dir_dst(I.dk[j], I.L) : INT32_MAX;
+        mine = val;
+        int pos = 0;  // samples below val (they ascend with the lane)
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+          if (__shfl_sync(kFull, smp, pos + h - 1) < val) pos += h;
+        if (pos == 31 && s31 < val) pos = 32;
+        int32_t lo = pos > 0 ? (pos - 1) * step + 1 : 0;
+        int32_t hi = pos < 32 ? min(pos * step, a) : a;
+        if (act) {
+          while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (A[mid] < val) lo = mid + 1;
+            else hi = mid;
+          }
+          I.slot[j] = (j - i0) + lo;
+          if (j == i0) first_new = lo;
+        }
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    // In place, old entries below the first new entry do not move; relocated, all of them do.
+    const int32_t keep_below = moved ? 0 : __shfl_sync(kFull, first_new, 0);
+    const int32_t m31 = __shfl_sync(kFull, mine, 31);
+    // Old entries: final position i + #(new < A[i]); backwards in steps of 128 entries, each read whole
+    // before its first write, so that, in place, no unread entry is overwritten (targets never
+    // precede sources). The new entries below an old one are counted from the lanes for runs of at
+    // most 32 (the usual case), else by a search of the keys.
+    const int32_t low = (keep_below / 128) * 128;
+    for (int32_t base = a > 0 ? ((a - 1) / 128) * 128 : -1; base >= low; base -= 128) {
+      int32_t val[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int32_t i = base + 32 * q + lane;
+        val[q] = i < a && i >= keep_below ? A[i] : -1;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        int32_t below = 0;
+        if (c <= 32) {
+#pragma unroll
+          for (int h = 16; h > 0; h >>= 1)
+            if (__shfl_sync(kFull, mine, below + h - 1) < val[q]) below += h;
+          if (below == 31 && m31 < val[q]) below = 32;
+        } else if (val[q] >= 0) {
+          int64_t lo = i0, hi = i1;
+          while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (dir_dst(I.dk[mid], I.L) < val[q]) lo = mid + 1;
+            else hi = mid;
+          }
+          below = (int32_t)(lo - i0);
+        }
+        if (val[q] >= 0) {
+          const int64_t pos = s_new + base + 32 * q + lane + below;
+          I.pool[pos] = val[q];
+          if (I.mark) I.mark[pos] = 0;
+        }
+      }
+      __syncwarp();
+    }
+    // New entries into the holes.
+    for (int64_t j = i0 + lane; j < i1; j += 32) {
+      const int64_t pos = s_new + I.slot[j];
+      I.pool[pos] = dir_dst(I.dk[j], I.L);
+      if (I.mark) I.mark[pos] = 1;
+      I.slot[j] = pos;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      I.used[v] = a + c;
+      atomicAdd(&st->dir_added, (unsigned long long)c);
+    }
   }
 }
 
+// ---- deletion -------------------------------------------------------------------------------
+
+// Mark the slots of the batch's deletions and keep each list's smallest marked slot (the
+// compaction leaves the entries below it in place); opens the compaction epoch.
+__global__ void k_mark_deletions(const int4* __restrict__ dlist, const BatchStatus* __restrict__ st,
+                                 const int64_t* __restrict__ start, uint8_t* __restrict__ mark,
+                                 int32_t* __restrict__ first_del, unsigned* __restrict__ epoch) {
+  const int64_t nd = (int64_t)st->n_del;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *epoch += 1u;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
+    const int4 d = dlist[i];
+    mark[start[d.x] + d.z] = 1;
+    mark[start[d.y] + d.w] = 1;
+    atomicMin(&first_del[d.x], d.z);
+    atomicMin(&first_del[d.y], d.w);
+  }
+}
+
+// The long-list compaction's plan of one list (see k_cmp_stage).
+struct CmpPlan {
+  int64_t s;       // list start
+  int64_t soff;    // the list's range in the scratch buffer (chunks j0 on)
+  int64_t ib;      // its first work item
+  int32_t v;
+  int32_t a;       // entries before the deletions
+  int32_t nch;     // work items: chunks j0 .. j0 + nch - 1
+  int32_t j0;      // the chunk of the first marked slot; the chunks below it stay in place
+  int32_t done;    // chunks staged so far
+  int32_t pad;
+};
+
+struct CompactArgs {
+  const int64_t* start;
+  int32_t* used;
+  int32_t* pool;
+  uint8_t* mark;
+  unsigned* claim;
+  const unsigned* epoch;
+  int32_t* first_del;
+  CmpPlan* plan;             // long lists: their plans and work items
+  unsigned long long* items;
+  int64_t item_cap;
+  int64_t scr_cap;
+};
+
+// Remove the marked slots from the list of v (each vertex once: the first warp to claim it with this
+// epoch) and clear its marks, by the warp. The entries below the list's first marked slot
+// (first_del, reset here to kNoDel) stay where they are; the rest move down in steps of 128
+// entries, each read whole before its first write. A long list is only planned (k_cmp_stage).
+__device__ __forceinline__ void compact_vertex(const CompactArgs& C, const int32_t v, BatchStatus* __restrict__ st) {
+  const int lane = threadIdx.x & 31;
+  const unsigned epoch = *C.epoch;
+  const int32_t a = C.used[v];
+  unsigned old = 0;
+  if (lane == 0) old = atomicMax(&C.claim[v], epoch);
+  __syncwarp();
+  old = __shfl_sync(kFull, old, 0);
+  if (old >= epoch) return;
+  const int64_t s = C.start[v];
+  const int32_t f = min(C.first_del[v], a);
+  __syncwarp();
+  if (lane == 0) C.first_del[v] = kNoDel;
+  if (a > kLongList) {
+    CmpPlan P;
+    P.s = s;
+    P.v = v;
+    P.a = a;
+    P.j0 = f / kLongChunk;
+    P.nch = f < a ? (a + kLongChunk - 1) / kLongChunk - P.j0 : 0;
+    P.done = 0;
+    P.pad = 0;
+    const int32_t span = a - P.j0 * kLongChunk;  // entries from chunk j0 on
+    unsigned long long so = 0, ib = 0, r = 0;
+    if (lane == 0) {
+      so = atomicAdd(&st->cmp_scr, (unsigned long long)span);
+      ib = atomicAdd(&st->cmp_items, (unsigned long long)P.nch);
+      r = atomicAdd(&st->n_cmp, 1ull);
+    }
+    so = __shfl_sync(kFull, so, 0);
+    ib = __shfl_sync(kFull, ib, 0);
+    r = __shfl_sync(kFull, r, 0);
+    const bool ok = (int64_t)(so + span) <= C.scr_cap && (int64_t)(ib + P.nch) <= C.item_cap;
+    for (int32_t j = lane; j < P.nch; j += 32)
+      if ((int64_t)(ib + j) < C.item_cap) C.items[ib + j] = ok ? (r << 32) | (unsigned)(P.j0 + j) : kNoLongItem;
+    if (lane == 0) {
+      if (!ok) {  // unreachable while the scratch follows the pool's size
+        atomicOr(&st->err, kErrScratch);
+        P.nch = 0;
+      }
+      P.soff = (int64_t)so;
+      P.ib = (int64_t)ib;
+      C.plan[r] = P;
+    }
+    __syncwarp();
+    return;
+  }
+  const unsigned lt = (1u << lane) - 1u;
+  int32_t wp = f;
+  for (int32_t base = f; base < a; base += 128) {
+    int32_t val[4];
+    bool keep[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int32_t i = base + 32 * q + lane;
+      val[q] = i < a ? C.pool[s + i] : 0;
+      keep[q] = i < a && C.mark[s + i] == 0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int32_t i = base + 32 * q + lane;
+      const unsigned m = __ballot_sync(kFull, keep[q]);
+      if (keep[q]) C.pool[s + wp + __popc(m & lt)] = val[q];
+      else if (i < a) C.mark[s + i] = 0;
+      wp += __popc(m);
+    }
+    __syncwarp();
+  }
+  if (lane == 0) {
+    C.used[v] = wp;
+    atomicAdd(&st->dir_removed, (unsigned long long)(a - wp));
+  }
+  __syncwarp();
+}
+
+// The lists of the vertices vlist[0 .. *nv) (the cuStinger-style deletion).
+__global__ void __launch_bounds__(kThreads) k_compact(const CompactArgs C, const int32_t* __restrict__ vlist,
+                                                      const unsigned long long* __restrict__ nv,
+                                                      BatchStatus* __restrict__ st) {
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < (int64_t)*nv; k += nw)
+    compact_vertex(C, vlist[k], st);
+}
+
+// Insertion into long lists (more than kLongList entries after the batch), over all of the batch's
+// long runs at once, from the plans of k_insert_runs:
+//   k_long_stage  one CTA per item: each moving old entry and each new entry computes its place
+//                 in the merged suffix (an old entry shifts by the number of new entries below it,
+//                 a new entry lands after the old entries below it) and writes there in scratch;
+//   k_long_write  one CTA per item: the merged suffix back into the list, with the new entries'
+//                 marks.
+// The launch boundary between staging and writing takes the place of an in-place merge's block
+// barriers: every source is read before any target is written, so a hub list of 10^5 entries is
+// spread over many CTAs instead of being one CTA's chain of steps.
 __global__ void __launch_bounds__(kThreads) k_long_stage(
-    const uint64_t* __restrict__ dk, const int32_t* __restrict__ pool, const LongPlan* __restrict__ plan,
-    const unsigned long long* __restrict__ items, const int64_t item_cap, int32_t* __restrict__ scr,
-    uint8_t* __restrict__ smark, int64_t* __restrict__ slot, const BatchStatus* __restrict__ st) {
+    const uint64_t* __restrict__ dk, const int L, const int32_t* __restrict__ pool,
+    const LongPlan* __restrict__ plan, const unsigned long long* __restrict__ items, const int64_t item_cap,
+    int32_t* __restrict__ scr, uint8_t* __restrict__ smark, int64_t* __restrict__ slot, const BatchStatus* __restrict__ st) {
   // The new entries whose values fall inside the item's old entries, staged in shared memory,
   // so that each old entry counts the new ones below it there instead of in global memory.
   __shared__ int32_t s_run[kLongChunk];
@@ -576,13 +757,13 @@ __global__ void __launch_bounds__(kThreads) k_long_stage(
         int32_t lo = 0, hi = P.c;
         while (lo < hi) {
           const int32_t mid = (lo + hi) >> 1;
-          if ((int32_t)(uint32_t)dk[P.i0 + mid] < v0) lo = mid + 1;
+          if (dir_dst(dk[P.i0 + mid], L) < v0) lo = mid + 1;
           else hi = mid;
         }
         int32_t lo2 = lo, hi2 = P.c;
         while (lo2 < hi2) {
           const int32_t mid = (lo2 + hi2) >> 1;
-          if ((int32_t)(uint32_t)dk[P.i0 + mid] < v1) lo2 = mid + 1;
+          if (dir_dst(dk[P.i0 + mid], L) < v1) lo2 = mid + 1;
           else hi2 = mid;
         }
         s_lo = lo;
@@ -591,7 +772,7 @@ __global__ void __launch_bounds__(kThreads) k_long_stage(
       __syncthreads();
       run_lo = s_lo;
       run_n = s_n <= kLongChunk ? s_n : -1;
-      for (int32_t t = threadIdx.x; t < run_n; t += kThreads) s_run[t] = (int32_t)(uint32_t)dk[P.i0 + run_lo + t];
+      for (int32_t t = threadIdx.x; t < run_n; t += kThreads) s_run[t] = dir_dst(dk[P.i0 + run_lo + t], L);
       __syncthreads();
     }
     for (int32_t k = k0 + (int32_t)threadIdx.x; k < k1; k += kThreads) {
@@ -614,7 +795,7 @@ __global__ void __launch_bounds__(kThreads) k_long_stage(
           hi = P.c;
           while (lo < hi) {
             const int32_t mid = (lo + hi) >> 1;
-            if ((int32_t)(uint32_t)dk[P.i0 + mid] < val) lo = mid + 1;
+            if (dir_dst(dk[P.i0 + mid], L) < val) lo = mid + 1;
             else hi = mid;
           }
         }
@@ -622,7 +803,7 @@ __global__ void __launch_bounds__(kThreads) k_long_stage(
         mk = 0;
       } else {  // a new entry: lands after the old entries below it
         const int32_t j = k - suffix;
-        val = (int32_t)(uint32_t)dk[P.i0 + j];
+        val = dir_dst(dk[P.i0 + j], L);
         pos = j + (int32_t)(lower_bound(pool, P.s_old, P.s_old + P.a, val) - P.s_old) - P.first;
         slot[P.i0 + j] = P.s_new + P.first + pos;
         mk = 1;
@@ -652,72 +833,22 @@ __global__ void __launch_bounds__(kThreads) k_long_write(
   }
 }
 
-// Deletions from long lists (more than kLongList entries), in four launches over all of the
-// batch's long lists at once, through the insertion's scratch buffer:
-//   k_cmp_plan    one thread per vertex of the deletions: claims the list (the epoch) and gives it
-//                 work items of kLongChunk entries and a range of the scratch;
+// Deletions from long lists (more than kLongList entries), over all of the batch's long lists at
+// once, from the plans of compact_vertex and through the insertion's scratch buffer:
 //   k_cmp_stage   one CTA per item: the chunk's kept entries, compacted within the chunk, into
-//                 scratch, and their count; the chunk's marks cleared;
-//   k_cmp_prefix  one thread per list: its chunks' output offsets (a prefix of the counts) and
-//                 its new length;
+//                 scratch, and their count; the chunk's marks cleared. The CTA that stages a list's
+//                 last chunk turns the counts into output offsets and sets the new length;
 //   k_cmp_write   one CTA per item: the chunk's kept entries from scratch to their place.
 // The scratch keeps sources and targets apart, so chunks of one list proceed on many CTAs.
-struct CmpPlan {
-  int64_t s;       // list start
-  int64_t soff;    // the list's range in the scratch buffer (chunks j0 on)
-  int64_t ib;      // its first work item
-  int32_t v;
-  int32_t a;       // entries before the deletions
-  int32_t nch;     // work items: chunks j0 .. j0 + nch - 1
-  int32_t j0;      // the chunk of the first marked slot; the chunks below it stay in place
-};
-
-__global__ void __launch_bounds__(kThreads) k_cmp_plan(
-    const int32_t* __restrict__ vlist, const int64_t nv_list, const int stride,
-    const unsigned long long* __restrict__ nv_dev, const int64_t* __restrict__ start,
-    const int32_t* __restrict__ used, unsigned* __restrict__ claim, const unsigned* __restrict__ epoch_dev,
-    int32_t* __restrict__ first_del, CmpPlan* __restrict__ plan, unsigned long long* __restrict__ items,
-    const int64_t item_cap, const int64_t scr_cap, BatchStatus* __restrict__ st) {
-  const unsigned epoch = *epoch_dev;
-  const int64_t cnt = nv_dev ? (int64_t)(*nv_dev) * stride : nv_list;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = vlist[k];
-    const int32_t a = used[v];
-    if (a <= kLongList) continue;  // k_compact_marked's
-    if (atomicMax(&claim[v], epoch) >= epoch) continue;  // claimed by another entry of v
-    CmpPlan P;
-    P.v = v;
-    P.a = a;
-    P.s = start[v];
-    const int32_t f = min(first_del[v], a);
-    first_del[v] = kNoDel;
-    P.j0 = f / kLongChunk;
-    P.nch = f < a ? (a + kLongChunk - 1) / kLongChunk - P.j0 : 0;
-    const int32_t span = a - P.j0 * kLongChunk;  // entries from chunk j0 on
-    const unsigned long long so = atomicAdd(&st->cmp_scr, (unsigned long long)span);
-    const unsigned long long ib = atomicAdd(&st->cmp_items, (unsigned long long)P.nch);
-    const unsigned long long r = atomicAdd(&st->n_cmp, 1ull);
-    if ((int64_t)(so + span) > scr_cap || (int64_t)(ib + P.nch) > item_cap) {
-      atomicOr(&st->err, kErrScratch);  // unreachable while the scratch follows the pool's size
-      for (int32_t j = 0; j < P.nch && (int64_t)(ib + j) < item_cap; ++j) items[ib + j] = kNoLongItem;
-      P.nch = 0;
-    } else {
-      for (int32_t j = 0; j < P.nch; ++j) items[ib + j] = (r << 32) | (unsigned)(P.j0 + j);
-    }
-    P.soff = (int64_t)so;
-    P.ib = (int64_t)ib;
-    plan[r] = P;
-  }
-}
 
 // Each thread holds kCmpPer consecutive entries of the chunk (256 threads x 16 = kLongChunk).
 constexpr int kCmpPer = kLongChunk / kThreads;
 static_assert(kCmpPer % 4 == 0, "a thread's run of entries is whole 16-byte units");
 
 __global__ void __launch_bounds__(kThreads) k_cmp_stage(
-    const CmpPlan* __restrict__ plan, const unsigned long long* __restrict__ items, const int64_t item_cap,
+    CmpPlan* __restrict__ plan, const unsigned long long* __restrict__ items, const int64_t item_cap,
     const int32_t* __restrict__ pool, uint8_t* __restrict__ mark, int32_t* __restrict__ scr,
-    int2* __restrict__ chunk, const BatchStatus* __restrict__ st) {
+    int2* __restrict__ chunk, int32_t* __restrict__ used, BatchStatus* __restrict__ st) {
   __shared__ int32_t sh_wsum[kThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t n_items = min((int64_t)st->cmp_items, item_cap);
@@ -786,25 +917,22 @@ __global__ void __launch_bounds__(kThreads) k_cmp_stage(
 #pragma unroll
     for (int t = 0; t < kCmpPer; ++t)
       if (keepm >> t & 1u) scr[P.soff + r0 + at++] = val[t];
-    if (threadIdx.x == 0) chunk[P.ib + (j - P.j0)] = make_int2(0, total);
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_cmp_prefix(const CmpPlan* __restrict__ plan, int2* __restrict__ chunk,
-                                                         int32_t* __restrict__ used, BatchStatus* __restrict__ st) {
-  const int64_t n = (int64_t)st->n_cmp;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    const CmpPlan P = plan[r];
-    if (P.nch == 0) continue;
-    int32_t off = P.j0 * kLongChunk;  // the chunks below j0 keep their entries in place
-    for (int32_t j = 0; j < P.nch; ++j) {
-      const int32_t c = chunk[P.ib + j].y;
-      chunk[P.ib + j].x = off;
-      off += c;
+    if (threadIdx.x == 0) {
+      __stcg(&chunk[P.ib + (j - P.j0)], make_int2(0, total));
+      __threadfence();
+      if (atomicAdd(&plan[item >> 32].done, 1) == P.nch - 1) {
+        __threadfence();
+        int32_t off = P.j0 * kLongChunk;  // the chunks below j0 keep their entries in place
+        for (int32_t x = 0; x < P.nch; ++x) {
+          const int32_t c = __ldcg(&chunk[P.ib + x]).y;
+          __stcg(&chunk[P.ib + x], make_int2(off, c));
+          off += c;
+        }
+        used[P.v] = off;
+        atomicAdd(&st->dir_removed, (unsigned long long)(P.a - off));
+      }
     }
-    used[P.v] = off;
-    atomicAdd(&st->dir_removed, (unsigned long long)(P.a - off));
+    __syncthreads();
   }
 }
 
@@ -834,7 +962,9 @@ struct BatchLists {
   const int32_t* dup;
 };
 
-// A changed edge as the per-edge kernel takes it: its lists, the shorter one first.
+// A changed edge as the per-edge kernel takes it: its lists, the shorter one first. kSplitFlag in la:
+// its intersection is queued as split items.
+constexpr int32_t kSplitFlag = INT32_MIN;
 struct __align__(16) DeltaDesc {
   int32_t oa, ob, la, lb;  // owners and lengths
   int64_t sa, sb;          // starts
@@ -855,23 +985,19 @@ struct DeltaArgs {
   int only_present;  // skip entries whose edge is absent (cuStinger deletion count)
   int use_table;     // per-cell strategy table: 0 = search, 1 = merge
   int cell_filter;   // -1 all, -2 none, c >= 0 only edges of cell c (timing mode)
-  // split queue: (entry << 24 | chunk) items of long intersections (NULL = no splitting)
+  // split queue: (edge << 24 | chunk) items of long intersections
   unsigned long long* split_items;
-  unsigned long long* split_cnt;  // zero before the first pass
+  unsigned long long* split_cnt;  // zero before the items are queued
   int split_min;     // intersections whose shorter list is longer than this are split ...
   int chunk;         // ... into items of this many entries of the shorter list
   int shard;         // this rank counts the entries e with e % nshards == shard
   int nshards;
   unsigned long long* bytes_out;  // algorithmic bytes of the intersections run (NULL = not kept)
-  // persistent kernel (k_delta_fused): its warps take split items while other warps still run
-  // the entry pass. An item slot is published by writing the launch's epoch (*item_epoch, bumped
-  // before each launch) into item_tag[slot]; entry_done counts the warps done with the entry
-  // pass (zero at launch). A wait for an item that runs out reports kErrTimeout in err; bar_extra
-  // is added to the warps the item pass waits for (0; a test sets 1 to make the wait run out);
-  // spin_ns bounds each wait.
-  unsigned* entry_done;
-  unsigned* item_tag;
-  const unsigned* item_epoch;
+  // persistent kernel (k_delta_fused): its CTAs meet once, between the count and the update that
+  // needs the count done. arrived counts them (zero at launch). A wait that runs out reports
+  // kErrTimeout in err; bar_extra is added to the CTAs waited for (0; a test sets 1 to make the wait
+  // run out); spin_ns bounds the wait.
+  unsigned* arrived;
   unsigned* err;
   unsigned bar_extra;
   unsigned long long spin_ns;
@@ -1240,104 +1366,92 @@ __device__ __forceinline__ void delta_part(const DeltaArgs& A, uint32_t* __restr
   }
 }
 
-// The entry pass of the persistent kernel: the described edges, one warp per edge, taken from a queue
-// up to kGrab at a time (the descriptions of a grab are read together; a batch of fewer edges
-// than warps goes out one by one). An edge whose shorter list is longer than A.split_min is queued
-// as items of A.chunk entries of it, published one by one (a full queue leaves the edge to this
-// warp).
-__device__ __forceinline__ void delta_entries(const DeltaArgs& A, uint32_t* __restrict__ pv,
-                                              unsigned long long& tri_acc, unsigned long long& bytes_acc) {
-  const int lane = threadIdx.x & 31;
-  const int64_t cnt = (int64_t)*A.n_desc;
+// Field-wise broadcast of lane k's description.
+__device__ __forceinline__ DeltaDesc desc_from(const DeltaDesc& m, const int k) {
+  return DeltaDesc{__shfl_sync(kFull, m.oa, k), __shfl_sync(kFull, m.ob, k), __shfl_sync(kFull, m.la, k),
+                   __shfl_sync(kFull, m.lb, k), __shfl_sync(kFull, m.sa, k), __shfl_sync(kFull, m.sb, k)};
+}
+
+// Elements a warp takes per grab of a queue of cnt: up to kGrab, whose descriptions its lanes read
+// together; one where that would leave warps without work.
+__device__ __forceinline__ int grab_size(const int64_t cnt) {
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int grab = (int)max((int64_t)1, min((int64_t)kGrab, cnt / (2 * nw)));
-  const unsigned epoch = *A.item_epoch;
-  for (;;) {
-    unsigned long long g = 0;
-    if (lane == 0) g = atomicAdd(A.e_next, (unsigned long long)grab);
-    g = __shfl_sync(kFull, g, 0);
-    if ((int64_t)g >= cnt) break;
-    const int have = (int)min((int64_t)grab, cnt - (int64_t)g);
+  return (int)max((int64_t)1, min((int64_t)kGrab, cnt / (2 * nw)));
+}
+
+// The next `grab` elements of a queue: the first, or -1 past its end.
+__device__ __forceinline__ int64_t take(unsigned long long* next, const int grab, const int64_t cnt) {
+  unsigned long long g = 0;
+  if ((threadIdx.x & 31) == 0) g = atomicAdd(next, (unsigned long long)grab);
+  g = __shfl_sync(kFull, g, 0);
+  return (int64_t)g < cnt ? (int64_t)g : -1;
+}
+
+// The count of the persistent kernel: the queued items of split intersections, then the other
+// described edges, one warp each. Both queues are complete before the launch (k_hub_place).
+__device__ __forceinline__ void delta_count(const DeltaArgs& A, uint32_t* __restrict__ pv, unsigned long long& tri_acc,
+                                            unsigned long long& bytes_acc) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n_items = (int64_t)min(*A.split_cnt, (unsigned long long)kDeltaItems);
+  const int64_t n_desc = (int64_t)*A.n_desc;
+  int grab = grab_size(n_items);
+  for (int64_t g; (g = take(A.i_next, grab, n_items)) >= 0;) {
+    const int have = (int)min((int64_t)grab, n_items - g);
     DeltaDesc mine = {};
-    if (lane < have) mine = A.desc[g + lane];
+    int32_t i0_l = -1;
+    if (lane < have) {
+      const unsigned long long item = A.split_items[g + lane];
+      if (item != kNoItem) {
+        mine = A.desc[item >> 24];
+        i0_l = (int32_t)(item & 0xffffffu) * A.chunk;
+      }
+    }
     __syncwarp();
     for (int k = 0; k < have; ++k) {
-      DeltaDesc d;
-      d.oa = __shfl_sync(kFull, mine.oa, k);
-      d.ob = __shfl_sync(kFull, mine.ob, k);
-      d.la = __shfl_sync(kFull, mine.la, k);
-      d.lb = __shfl_sync(kFull, mine.lb, k);
-      d.sa = __shfl_sync(kFull, mine.sa, k);
-      d.sb = __shfl_sync(kFull, mine.sb, k);
-      if (lane == 0) bytes_acc += 4ull * ((unsigned long long)d.la + (unsigned long long)d.lb) + 8ull;
-      if (d.la > A.split_min) {
-        const int nch = (d.la + A.chunk - 1) / A.chunk;
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(A.split_cnt, (unsigned long long)nch);
-        at = __shfl_sync(kFull, at, 0);
-        const bool fits = at + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
-        for (int j = lane; j < nch; j += 32)
-          if (at + j < (unsigned long long)kDeltaItems) {
-            A.split_items[at + j] = fits ? ((g + k) << 24) | (unsigned long long)j : kNoItem;
-            st_release(A.item_tag + at + j, epoch);  // the slot is ready
-          }
-        if (fits) continue;
-      }
-      delta_part(A, pv, d, 0, d.la, tri_acc);
+      DeltaDesc d = desc_from(mine, k);
+      const int32_t i0 = __shfl_sync(kFull, i0_l, k);
+      if (i0 < 0) continue;
+      d.la &= ~kSplitFlag;
+      delta_part(A, pv, d, i0, min(d.la, i0 + A.chunk), tri_acc);
     }
   }
-}
-
-// Wait (lane 0 of a warp) until queue slot q holds a published item of this launch: 1 when it
-// does, 0 when no item will come to slot q (every warp has finished the entry pass and q lies
-// beyond the items they queued, or q beyond the queue's capacity), -1 when the wait ran out
-// (spin_ns of device time, at most kSpinMaxIters polls; kErrTimeout is set). A producer publishes
-// each slot before it counts itself done, so once every warp is done a reserved slot is ready.
-__device__ __forceinline__ int wait_item(const DeltaArgs& A, const unsigned long long q, const unsigned epoch,
-                                         const unsigned total) {
-  if (q >= (unsigned long long)kDeltaItems) return 0;
-  unsigned long long t0;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (unsigned it = 0;; ++it) {
-    if (ld_acquire(A.item_tag + q) == epoch) return 1;
-    if (ld_acquire(A.entry_done) >= total && q >= ld_acquire64(A.split_cnt)) return 0;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (it >= kSpinMaxIters || t - t0 > A.spin_ns) {
-      atomicOr(A.err, kErrTimeout);
-      return -1;
-    }
-    __nanosleep(64);
-  }
-}
-
-// The item pass of the persistent kernel: it starts as soon as the warp's own entry pass ends,
-// while other warps may still queue items. Slots are taken in order from the queue head; a slot
-// is read once its tag carries this launch's epoch (items written by other CTAs are read past
-// the non-coherent L1 after the acquire).
-__device__ __forceinline__ void delta_items_stream(const DeltaArgs& A, uint32_t* __restrict__ pv,
-                                                   unsigned long long& tri_acc) {
-  const int lane = threadIdx.x & 31;
-  const unsigned epoch = *A.item_epoch;
-  const unsigned total = (unsigned)(((int64_t)gridDim.x * blockDim.x) >> 5) + A.bar_extra;
-  const unsigned long long cnt = *A.n_desc;
-  for (;;) {
-    unsigned long long q = 0;
-    int state = 0;
-    if (lane == 0) {
-      q = atomicAdd(A.i_next, 1ull);
-      state = wait_item(A, q, epoch, total);
+  grab = grab_size(n_desc);
+  for (int64_t g; (g = take(A.e_next, grab, n_desc)) >= 0;) {
+    const int have = (int)min((int64_t)grab, n_desc - g);
+    DeltaDesc mine = {};
+    if (lane < have) {
+      mine = A.desc[g + lane];
+      bytes_acc += 4ull * ((unsigned long long)(mine.la & ~kSplitFlag) + (unsigned long long)mine.lb) + 8ull;
     }
     __syncwarp();
-    state = __shfl_sync(kFull, state, 0);
-    q = __shfl_sync(kFull, q, 0);
-    if (state != 1) break;
-    const unsigned long long item = __ldcg(A.split_items + q);
-    if (item == kNoItem || (item >> 24) >= cnt) continue;
-    const DeltaDesc d = A.desc[item >> 24];
-    const int32_t i0 = (int32_t)(item & 0xffffffu) * A.chunk;
-    if (i0 < d.la) delta_part(A, pv, d, i0, min(d.la, i0 + A.chunk), tri_acc);
+    for (int k = 0; k < have; ++k) {
+      const DeltaDesc d = desc_from(mine, k);
+      if (d.la >= 0) delta_part(A, pv, d, 0, d.la, tri_acc);
+    }
   }
+}
+
+// All CTAs of a resident grid meet: each waits (spin_ns of device time, at most kSpinMaxIters polls)
+// until every other has arrived. A wait that runs out sets kErrTimeout, and the CTA goes on.
+__device__ __forceinline__ void grid_meet(const DeltaArgs& A) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned total = gridDim.x + A.bar_extra;
+    __threadfence();
+    atomicAdd(A.arrived, 1u);
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (unsigned it = 0; ld_relaxed(A.arrived) < total; ++it) {
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (it >= kSpinMaxIters || t - t0 > A.spin_ns) {
+        atomicOr(A.err, kErrTimeout);
+        break;
+      }
+      __nanosleep(64);
+    }
+    __threadfence();
+  }
+  __syncthreads();
 }
 
 // Two launches: the entry pass, then the item pass (the cuStinger-style count, tc_count_batch).
@@ -1359,30 +1473,54 @@ __global__ void __launch_bounds__(kThreads, 6) k_delta_split(const DeltaArgs A, 
   delta_flush(tri_acc, 0ull, tri_out, nullptr);
 }
 
-// One persistent launch (a resident grid, at most the occupancy limit of CTAs per SM): every warp
-// runs its share of the entry pass, queueing the chunks of split intersections, counts itself
-// done, and then takes queued chunks until none is left: no grid-wide barrier, so warps whose
-// entry work ends early start on the chunks while others still queue them. The batch size is
-// read from device memory, so one captured launch serves every batch of a bin. The launch's
-// epoch (bumped before it) marks the slots published in this launch. A wait that runs out (the
-// grid was not resident, or a test forces it) sets kErrTimeout and the warp leaves the item
-// pass: the batch's count is then incomplete and the host reports TC_ERR_TIMEOUT.
+// What a phase does once its count is done: deletions compact their lists, insertions clear the
+// marks of the new slots and add the batch's triangles to the running delta (NULL = not here).
+struct PhaseEnd {
+  const int4* dlist;               // deletions (phase 0)
+  const unsigned long long* n_del;
+  CompactArgs cmp;
+  const int64_t* slot;             // insertions (phase 1): slots of the 2 * *n_ins new entries
+  const unsigned long long* n_ins;
+  uint8_t* mark;
+  int64_t* delta;
+  const unsigned long long* added;
+  const unsigned long long* removed;
+  BatchStatus* st;
+};
+
+// One persistent launch per phase (a resident grid, at most the occupancy limit of CTAs per SM): the
+// per-edge count, then, once every CTA has met (grid_meet), the phase's end, so that a small
+// batch does not pay a launch for each. The batch's sizes are read from device memory, so one
+// captured launch serves every batch of a bin. A meeting that runs out (the grid was not
+// resident, or a test forces it) sets kErrTimeout: the update still completes and the host reports
+// TC_ERR_TIMEOUT, as the batch's count may be incomplete.
 #ifndef TC_DELTA_MIN_BLOCKS
 #define TC_DELTA_MIN_BLOCKS 6
 #endif
-__global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(const DeltaArgs A, uint32_t* __restrict__ pv,
-                                                          unsigned long long* __restrict__ tri_out) {
+__global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(const DeltaArgs A, const PhaseEnd E,
+                                                                               uint32_t* __restrict__ pv,
+                                                                               unsigned long long* __restrict__ tri_out) {
   unsigned long long tri_acc = 0, bytes_acc = 0;
-  delta_entries(A, pv, tri_acc, bytes_acc);
-  // this warp's items are published: count it done (its lanes' releases before lane 0's add)
-  __threadfence();
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    atomicAdd(A.entry_done, 1u);
-  }
-  delta_items_stream(A, pv, tri_acc);
+  delta_count(A, pv, tri_acc, bytes_acc);
+  bytes_acc = warp_sum(bytes_acc);
   delta_flush(tri_acc, bytes_acc, tri_out, A.bytes_out);
+  grid_meet(A);
+  if (E.dlist) {
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t ends = 2 * (int64_t)*E.n_del;
+    for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < ends; k += nw) {
+      const int4 d = E.dlist[k >> 1];
+      compact_vertex(E.cmp, k & 1 ? d.y : d.x, E.st);
+    }
+  } else {
+    const int64_t n = 2 * (int64_t)*E.n_ins;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t at = E.slot[i];
+      if (at >= 0) E.mark[at] = 0;
+    }
+    if (E.delta && blockIdx.x == 0 && threadIdx.x == 0)
+      *E.delta += (int64_t)__ldcg(E.added) - (int64_t)__ldcg(E.removed);
+  }
 }
 
 // ---- hub-centred delta count ------------------------------------------------------------------
@@ -1448,7 +1586,6 @@ struct HubWs {
   int64_t unit_cap;
   DeltaDesc* desc;   // [cap] the edges not counted at a hub
   unsigned long long* n_desc;
-  unsigned* item_epoch;
   int on;            // hub groups are formed (0: every edge is described)
   unsigned long long* items;  // [item_cap] (hub id << 32 | item index within the hub)
   int64_t item_cap;
@@ -1532,11 +1669,12 @@ __global__ void __launch_bounds__(kThreads) k_hub_alloc(const DeltaArgs A, const
 
 // Place the units of every hub edge in its hub's range and describe every other edge for the per-edge
 // kernel (its lists looked up here once, by a thread per edge, so that a warp of that kernel starts
-// with one load); clears the per-vertex counts and opens the per-edge kernel's launch epoch.
+// with one load), queueing the chunks of long intersections (an edge with a shorter list past
+// A.split_min, two hubs, would be one warp's serial tail; a full queue leaves it whole); clears the
+// per-vertex counts.
 __global__ void __launch_bounds__(kThreads) k_hub_place(const DeltaArgs A, const HubWs H) {
   const int64_t cnt = (int64_t)*A.count_dev;
   const int lane = threadIdx.x & 31;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *H.item_epoch += 1u;
   for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); e0 < cnt;
        e0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t e = e0 + lane;
@@ -1561,7 +1699,19 @@ __global__ void __launch_bounds__(kThreads) k_hub_place(const DeltaArgs A, const
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(H.n_desc, (unsigned long long)__popc(m));
     at = __shfl_sync(kFull, at, 0);
-    if (left) H.desc[at + __popc(m & ((1u << lane) - 1u))] = DeltaDesc{s, h, ls, lh, A.g.start(s), A.g.start(h)};
+    if (left) {
+      const unsigned long long mine = at + __popc(m & ((1u << lane) - 1u));
+      int32_t la = ls;
+      if (ls > A.split_min) {
+        const int nch = (ls + A.chunk - 1) / A.chunk;
+        const unsigned long long q = atomicAdd(A.split_cnt, (unsigned long long)nch);
+        const bool fits = q + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
+        for (int c = 0; c < nch && q + c < (unsigned long long)kDeltaItems; ++c)
+          A.split_items[q + c] = fits ? (mine << 24) | (unsigned long long)c : kNoItem;
+        if (fits) la |= kSplitFlag;
+      }
+      H.desc[mine] = DeltaDesc{s, h, la, lh, A.g.start(s), A.g.start(h)};
+    }
   }
 }
 
@@ -1776,7 +1926,7 @@ __global__ void k_unpack_dir(const uint64_t* __restrict__ keys, const int64_t b,
 // Entries with dup == 0 that are already in the graph become duplicates; the rest are packed
 // as directed insertion keys (sentinel elsewhere).
 __global__ void k_flag_present(const SlackView g, const int32_t* __restrict__ s, const int32_t* __restrict__ d,
-                               int32_t* __restrict__ dup, const int64_t b, uint64_t* __restrict__ dk) {
+                               int32_t* __restrict__ dup, const int64_t b, const int L, uint64_t* __restrict__ dk) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
     uint64_t k = kSentinel;
     if (!dup[i]) {
@@ -1785,7 +1935,7 @@ __global__ void k_flag_present(const SlackView g, const int32_t* __restrict__ s,
       const int32_t lx = g.len(x);
       const int64_t p = lower_bound(g.ind, sx, sx + lx, y);
       if (p < sx + lx && g.ind[p] == y) dup[i] = 1;
-      else k = ((uint64_t)(uint32_t)x << 32) | (uint32_t)y;
+      else k = ((uint64_t)(uint32_t)x << L) | (uint32_t)y;
     }
     dk[i] = k;
   }
@@ -1810,54 +1960,9 @@ __global__ void k_mark_dir_deletions(const SlackView g, const int32_t* __restric
   }
 }
 
-__global__ void k_endpoints(const int4* __restrict__ dlist, const BatchStatus* __restrict__ st, int32_t* __restrict__ vlist) {
-  const int64_t nd = (int64_t)st->n_del;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
-    vlist[2 * i] = dlist[i].x;
-    vlist[2 * i + 1] = dlist[i].y;
-  }
-}
-
-// The compaction epoch and the delta kernel's item epoch live on the device so that a captured
-// launch sequence advances them.
+// The compaction epoch lives on the device so that a captured launch sequence advances it.
 __global__ void k_bump_epoch(unsigned* __restrict__ epoch) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *epoch += 1u;
-}
-
-// Canonical keys of a padded batch: entries [b, cap) (b read on the device) become sentinels,
-// so a launch sequence sized for cap serves every batch of at most cap updates.
-// A device batch into the pipeline's capacity-sized buffers, and its size where the captured
-// graph reads it: one launch in place of three copies and a host-to-device copy of the size.
-__global__ void k_load_batch(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
-                             const uint8_t* __restrict__ isdel, const int64_t b, int32_t* __restrict__ wsrc,
-                             int32_t* __restrict__ wdst, uint8_t* __restrict__ wdel, int64_t* __restrict__ d_b) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
-    wsrc[i] = src[i];
-    wdst[i] = dst[i];
-    wdel[i] = isdel ? isdel[i] : (uint8_t)0;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *d_b = b;
-}
-
-__global__ void k_make_keys_cap(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
-                                const uint8_t* __restrict__ is_del, const int64_t* __restrict__ b_dev,
-                                const int64_t cap, const int32_t n, const int L, uint64_t* __restrict__ keys,
-                                BatchStatus* __restrict__ st) {
-  const uint64_t sent = (1ull << (2 * L + 1)) - 1;
-  const int64_t b = min(*b_dev, cap);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t k = sent;
-    if (i < b) {
-      const int32_t s = src[i], d = dst[i];
-      if (s < 0 || s >= n || d < 0 || d >= n) {
-        atomicOr(&st->err, kErrRange);
-      } else if (s != d) {
-        const uint64_t lo = (uint64_t)min(s, d), hi = (uint64_t)max(s, d);
-        k = (lo << (L + 1)) | (hi << 1) | (uint64_t)(is_del[i] ? 0 : 1);
-      }
-    }
-    keys[i] = k;
-  }
 }
 
 __global__ void k_add_delta(int64_t* __restrict__ delta, const unsigned long long* __restrict__ add,
@@ -1882,14 +1987,11 @@ struct StreamWs {
   uint8_t* isdel = nullptr;
   uint64_t* keys = nullptr;     // [b]
   uint64_t* keys2 = nullptr;    // [b]
-  int32_t* head = nullptr;      // [b]
   int4* dlist = nullptr;        // [b]
   int2* ilist = nullptr;        // [b]
   uint64_t* dk = nullptr;       // [2b]
   uint64_t* dk2 = nullptr;      // [2b]
   int32_t* run_start = nullptr; // [2b]
-  int32_t* long_runs = nullptr; // [2b] starts of the runs whose list is long
-  int32_t* long_cnt = nullptr;  // [2b] their lengths
   LongPlan* long_plan = nullptr;  // [2b]
   CmpPlan* cmp_plan = nullptr;    // [2b] long lists with deletions
   // long-list insertion scratch, sized with the pool (ensure_long_scratch)
@@ -1914,8 +2016,6 @@ struct StreamWs {
   int64_t* scan64 = nullptr;    // [n+1]
   int64_t* tiles = nullptr;
   unsigned long long* split_items = nullptr;  // [kDeltaItems] queued chunks of long intersections
-  unsigned* item_tag = nullptr;    // [kDeltaItems] launch epoch that published each item slot
-  unsigned* item_epoch = nullptr;  // [1] epoch of the current persistent delta launch
   // hub groups of the delta count (k_delta_hub)
   int32_t* hub_cnt = nullptr;     // [n] zero between phases
   long long* hub_sum = nullptr;   // [n] zero between phases
@@ -1933,13 +2033,13 @@ struct StreamWs {
 };
 
 void StreamWs::release() {
-  cudaFree(src); cudaFree(dst); cudaFree(isdel); cudaFree(keys); cudaFree(keys2); cudaFree(head);
-  cudaFree(dlist); cudaFree(ilist); cudaFree(dk); cudaFree(dk2); cudaFree(run_start); cudaFree(long_runs);
-  cudaFree(long_cnt); cudaFree(long_plan); cudaFree(long_scr); cudaFree(long_smark); cudaFree(long_items);
+  cudaFree(src); cudaFree(dst); cudaFree(isdel); cudaFree(keys); cudaFree(keys2);
+  cudaFree(dlist); cudaFree(ilist); cudaFree(dk); cudaFree(dk2); cudaFree(run_start);
+  cudaFree(long_plan); cudaFree(long_scr); cudaFree(long_smark); cudaFree(long_items);
   cudaFree(cmp_plan); cudaFree(long_chunk);
   cudaFree(ins_slot);
   cudaFree(vlist); cudaFree(claim); cudaFree(first_del); cudaFree(d_epoch); cudaFree(cub_tmp); cudaFree(st); cudaFreeHost(st_host); cudaFree(counter);
-  cudaFree(cnt); cudaFree(scan64); cudaFree(tiles); cudaFree(split_items); cudaFree(item_tag); cudaFree(item_epoch);
+  cudaFree(cnt); cudaFree(scan64); cudaFree(tiles); cudaFree(split_items);
   cudaFree(hub_cnt); cudaFree(hub_sum); cudaFree(hub_uni); cudaFree(hub_of); cudaFree(hub_list); cudaFree(hub_off);
   cudaFree(hub_len); cudaFree(hub_fill); cudaFree(hub_chunks); cudaFree(hub_units); cudaFree(desc);
   cudaFree(hub_items);
@@ -2006,40 +2106,34 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
     TC_CUDA_TRY(cudaMemset(w.hub_of, 0, sizeof(int32_t) * n1));
     w.n_cap = g->n + 1;
   }
-  if (!w.st || !w.st_host || !w.counter || !w.split_items || !w.item_tag || !w.item_epoch) {
+  if (!w.st || !w.st_host || !w.counter || !w.split_items) {
     auto free_st = [&w]() {
       cudaFree(w.st); cudaFreeHost(w.st_host); cudaFree(w.counter); cudaFree(w.split_items);
-      cudaFree(w.item_tag); cudaFree(w.item_epoch);
       w.st = nullptr; w.st_host = nullptr; w.counter = nullptr; w.split_items = nullptr;
-      w.item_tag = nullptr; w.item_epoch = nullptr;
     };
     free_st();
     if (::tc::dev_malloc(&w.st, sizeof(BatchStatus)) != cudaSuccess ||
         cudaMallocHost(&w.st_host, sizeof(BatchStatus)) != cudaSuccess ||
         ::tc::dev_malloc(&w.counter, sizeof(unsigned long long)) != cudaSuccess ||
-        ::tc::dev_malloc(&w.split_items, sizeof(unsigned long long) * kDeltaItems) != cudaSuccess ||
-        ::tc::dev_malloc(&w.item_tag, sizeof(unsigned) * kDeltaItems) != cudaSuccess ||
-        ::tc::dev_malloc(&w.item_epoch, sizeof(unsigned)) != cudaSuccess) {
+        ::tc::dev_malloc(&w.split_items, sizeof(unsigned long long) * kDeltaItems) != cudaSuccess) {
       free_st();
       return fail(TC_ERR_OOM, "batch status: allocation failed");
     }
-    TC_CUDA_TRY(cudaMemset(w.item_tag, 0, sizeof(unsigned) * kDeltaItems));
-    TC_CUDA_TRY(cudaMemset(w.item_epoch, 0, sizeof(unsigned)));
     ++w.version;
   }
   if (b <= w.b_cap) return TC_OK;
   const int64_t nb = std::max<int64_t>(b, 1024);
   auto free_batch = [&w]() {
-    cudaFree(w.src); cudaFree(w.dst); cudaFree(w.isdel); cudaFree(w.keys); cudaFree(w.keys2); cudaFree(w.head);
+    cudaFree(w.src); cudaFree(w.dst); cudaFree(w.isdel); cudaFree(w.keys); cudaFree(w.keys2);
     cudaFree(w.dlist); cudaFree(w.ilist); cudaFree(w.dk); cudaFree(w.dk2); cudaFree(w.run_start);
-    cudaFree(w.long_runs); cudaFree(w.ins_slot); cudaFree(w.vlist); cudaFree(w.cub_tmp);
-    cudaFree(w.long_cnt); cudaFree(w.long_plan); cudaFree(w.cmp_plan);
-    w.long_cnt = nullptr; w.long_plan = nullptr; w.cmp_plan = nullptr;
+    cudaFree(w.ins_slot); cudaFree(w.vlist); cudaFree(w.cub_tmp);
+    cudaFree(w.long_plan); cudaFree(w.cmp_plan);
+    w.long_plan = nullptr; w.cmp_plan = nullptr;
     cudaFree(w.hub_list); cudaFree(w.hub_off); cudaFree(w.hub_len); cudaFree(w.hub_fill); cudaFree(w.hub_chunks);
     cudaFree(w.hub_units); cudaFree(w.desc); cudaFree(w.hub_items);
-    w.src = nullptr; w.dst = nullptr; w.isdel = nullptr; w.keys = nullptr; w.keys2 = nullptr; w.head = nullptr;
+    w.src = nullptr; w.dst = nullptr; w.isdel = nullptr; w.keys = nullptr; w.keys2 = nullptr;
     w.dlist = nullptr; w.ilist = nullptr; w.dk = nullptr; w.dk2 = nullptr; w.run_start = nullptr;
-    w.long_runs = nullptr; w.ins_slot = nullptr; w.vlist = nullptr; w.cub_tmp = nullptr;
+    w.ins_slot = nullptr; w.vlist = nullptr; w.cub_tmp = nullptr;
     w.hub_list = nullptr; w.hub_off = nullptr; w.hub_len = nullptr; w.hub_fill = nullptr; w.hub_chunks = nullptr;
     w.hub_units = nullptr; w.desc = nullptr; w.hub_items = nullptr;
     w.b_cap = 0;
@@ -2053,14 +2147,11 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
             ::tc::dev_malloc(&w.isdel, nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.keys, sizeof(uint64_t) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.keys2, sizeof(uint64_t) * nb) == cudaSuccess &&
-            ::tc::dev_malloc(&w.head, sizeof(int32_t) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.dlist, sizeof(int4) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.ilist, sizeof(int2) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.dk, sizeof(uint64_t) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.dk2, sizeof(uint64_t) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.run_start, sizeof(int32_t) * 2 * nb) == cudaSuccess &&
-            ::tc::dev_malloc(&w.long_runs, sizeof(int32_t) * 2 * nb) == cudaSuccess &&
-            ::tc::dev_malloc(&w.long_cnt, sizeof(int32_t) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.long_plan, sizeof(LongPlan) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.cmp_plan, sizeof(CmpPlan) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.ins_slot, sizeof(int64_t) * 2 * nb) == cudaSuccess &&
@@ -2201,31 +2292,74 @@ size_t delta_smem(const DeltaArgs& A) { return A.stage_ok ? kStageSmem : 0; }
 int delta_grid() { return device_info().sms * 8; }
 int long_grid() { return device_info().sms * 8; }
 
-// Deletions from the batch's long lists (k_cmp_plan, k_cmp_stage, k_cmp_prefix, k_cmp_write): the
-// vertices vlist[0 .. nv) (nv = nv_dev * stride when nv_dev is set, else nv_list, at most
-// nv_cap). The scratch must be sized (ensure_long_scratch).
-void long_compact(tc_graph* g, StreamWs& w, const int32_t* vlist, int64_t nv_list, int stride,
-                  const unsigned long long* nv_dev, int64_t nv_cap, cudaStream_t s) {
-  k_cmp_plan<<<grid_for(nv_cap, kThreads), kThreads, 0, s>>>(vlist, nv_list, stride, nv_dev, g->start, g->used, w.claim,
-                                                            w.d_epoch, w.first_del, w.cmp_plan, w.long_items,
-                                                            w.long_item_cap, w.scr_cap, w.st);
+CompactArgs compact_args(tc_graph* g, StreamWs& w) {
+  return CompactArgs{g->start, g->used,      g->pool,       g->mark,         w.claim,  w.d_epoch,
+                     w.first_del, w.cmp_plan, w.long_items, w.long_item_cap, w.scr_cap};
+}
+
+// The long lists that a compaction (compact_vertex) planned. The scratch must be sized
+// (ensure_long_scratch).
+void long_compact(tc_graph* g, StreamWs& w, cudaStream_t s) {
   k_cmp_stage<<<long_grid(), kThreads, 0, s>>>(w.cmp_plan, w.long_items, w.long_item_cap, g->pool, g->mark, w.long_scr,
-                                               w.long_chunk, w.st);
-  k_cmp_prefix<<<grid_for(nv_cap, kThreads), kThreads, 0, s>>>(w.cmp_plan, w.long_chunk, g->used, w.st);
+                                               w.long_chunk, g->used, w.st);
   k_cmp_write<<<long_grid(), kThreads, 0, s>>>(w.cmp_plan, w.long_items, w.long_item_cap, w.long_scr, w.long_chunk,
                                                g->pool, w.st);
 }
 
-// Insertion into the batch's long lists (k_long_plan, k_long_stage, k_long_write); `nd_cap` bounds
-// the long runs (the directed entries' capacity). The scratch must be sized (ensure_pool).
-void long_insert(tc_graph* g, StreamWs& w, int64_t nd_cap, uint8_t* mark, cudaStream_t s) {
-  k_long_plan<<<grid_for(nd_cap, kThreads), kThreads, 0, s>>>(
-      w.dk2, w.long_runs, w.long_cnt, g->start, g->used, g->cap, g->pool, g->pool_cap, w.ins_slot, g->d_pool_top,
-      g->slack_q10, w.long_plan, w.long_items, w.long_item_cap, w.scr_cap, w.st);
-  k_long_stage<<<long_grid(), kThreads, 0, s>>>(w.dk2, g->pool, w.long_plan, w.long_items, w.long_item_cap, w.long_scr,
+// Insertion of the sorted directed keys w.dk2 (nd_cap of them) in at most `runs` runs; the scratch
+// must be sized (ensure_pool).
+void insert_sorted_keys(tc_graph* g, StreamWs& w, int64_t nd_cap, int64_t runs, int L, uint8_t* mark, cudaStream_t s) {
+  const InsertArgs I{w.dk2,      nd_cap,  L,           w.run_start,    g->start,     g->used,      g->cap,         g->pool,
+                     g->pool_cap, mark,    w.ins_slot,  g->d_pool_top,  g->slack_q10, w.long_plan,  w.long_items,
+                     w.long_item_cap, w.scr_cap};
+  k_insert_runs<<<grid_for(runs * 32, kThreads), kThreads, 0, s>>>(I, w.st);
+  k_long_stage<<<long_grid(), kThreads, 0, s>>>(w.dk2, L, g->pool, w.long_plan, w.long_items, w.long_item_cap, w.long_scr,
                                                 w.long_smark, w.ins_slot, w.st);
   k_long_write<<<long_grid(), kThreads, 0, s>>>(w.long_plan, w.long_items, w.long_item_cap, w.long_scr, w.long_smark,
                                                 g->pool, mark, w.st);
+}
+
+// Batches of at most kWarpClassify updates are classified by a warp per key (k_classify_warp).
+constexpr int64_t kWarpClassify = 8192;
+
+// From the sorted keys w.keys2 (cap of them) to the changed-edge lists and the sorted directed keys
+// w.dk2 with their runs.
+cudaError_t classify_and_sort(tc_graph* g, StreamWs& w, int64_t cap, int L, cudaStream_t s) {
+  const SlackView view{g->start, g->used, g->pool};
+  if (cap <= kWarpClassify)
+    k_classify_warp<<<grid_for(cap * 32, kThreads), kThreads, 0, s>>>(view, w.keys2, cap, L, w.dlist, w.ilist, w.dk, w.st);
+  else
+    k_classify<<<grid_for(cap, kThreads), kThreads, 0, s>>>(view, w.keys2, cap, L, w.dlist, w.ilist, w.dk, w.st);
+  if (cap <= kSmallBatch) {
+    k_sort_runs<<<1, kSortThreads, 0, s>>>(w.dk, cap, L, w.dk2, g->used, g->cap, g->slack_q10, w.run_start, w.st);
+    return cudaSuccess;
+  }
+  // the sentinels' low 2L bits are all ones, which no edge has (it would be a self-loop)
+  size_t tb = w.cub_bytes;
+  const cudaError_t e = cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)(2 * cap), 0, 2 * L, s);
+  if (e != cudaSuccess) return e;
+  k_dir_runs<<<grid_for(2 * cap, kThreads), kThreads, 0, s>>>(w.dk2, 2 * cap, L, g->used, g->cap, g->slack_q10,
+                                                              w.run_start, w.st);
+  return cudaSuccess;
+}
+
+// The keys of a device batch of b <= cap updates into w.keys2, sorted, or (cap > kSmallBatch) into
+// w.keys, to be sorted; the status starts at zero.
+cudaError_t load_batch(tc_graph* g, StreamWs& w, const int32_t* src, const int32_t* dst, const uint8_t* is_del, int64_t b,
+                       int64_t cap, int L, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(w.st, 0, sizeof(BatchStatus), s);
+  if (e != cudaSuccess) return e;
+  if (cap <= kSmallBatch)
+    k_load_sorted<<<1, kSortThreads, 0, s>>>(src, dst, is_del, b, cap, g->n, L, w.keys2, w.st);
+  else
+    k_load_keys<<<grid_for(cap, kThreads), kThreads, 0, s>>>(src, dst, is_del, b, cap, g->n, L, w.keys, w.dk, w.st);
+  return cudaGetLastError();
+}
+
+cudaError_t sort_batch(StreamWs& w, int64_t cap, int L, cudaStream_t s) {
+  if (cap <= kSmallBatch) return cudaSuccess;  // k_load_sorted did
+  size_t tb = w.cub_bytes;
+  return cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.keys, w.keys2, (int)cap, 0, 2 * L + 1, s);
 }
 
 // Grid of the persistent delta kernel: ctas_per_sm CTAs per SM (0 = the occupancy limit), never
@@ -2266,10 +2400,13 @@ tc_status hub_grid(int* grid) {
   return TC_OK;
 }
 
+// Phases of at most this many changed edges take none of the hub kernels' four launches.
+constexpr int64_t kHubBatchMin = kSmallBatch;
+
 // Hub groups and their count for one phase of a batch (deletions: phase 0, insertions: 1) on a
 // grid of `grid` hub CTAs, and the descriptions of the edges left to the per-edge kernel that
-// follows (all of them when the hub count is off: hub_min <= 0, or a timing run of one degree
-// cell); `cap` bounds the phase's changed edges. Launches only (it can run inside a stream capture).
+// follows (all of them when the hub count is off: hub_min <= 0, a small batch, or a timing run of
+// one degree cell); `cap` bounds the phase's changed edges. Launches only (it can run inside a stream capture).
 void hub_kernels(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, int grid, uint32_t* pv,
                  unsigned long long* tri_out, cudaStream_t s) {
   HubWs H;
@@ -2286,8 +2423,7 @@ void hub_kernels(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, int grid, ui
   H.unit_cap = kHubUnitsPerUpdate * w.b_cap;
   H.desc = w.desc;
   H.n_desc = &w.st->n_desc[phase];
-  H.item_epoch = w.item_epoch;
-  H.on = A.hub_min > 0 && A.cell_filter == -1;
+  H.on = A.hub_min > 0 && A.cell_filter == -1 && cap > kHubBatchMin;
   H.items = w.hub_items;
   H.item_cap = kHubItemsPerUpdate * w.b_cap;
   H.n_hubs = &w.st->n_hubs[phase];
@@ -2305,36 +2441,47 @@ void hub_kernels(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, int grid, ui
   if (H.on) k_delta_hub<<<grid, kHubThreads, kHubSmem, s>>>(A, H, pv, tri_out);
 }
 
-tc_status launch_hub(DeltaArgs& A, StreamWs& w, int phase, int64_t cap, uint32_t* pv, unsigned long long* tri_out,
-                     cudaStream_t s) {
-  int grid = 0;
-  TC_TRY(hub_grid(&grid));
-  hub_kernels(A, w, phase, cap, grid, pv, tri_out, s);
-  TC_CUDA_TRY(cudaGetLastError());
-  return TC_OK;
-}
-
-// The persistent delta kernel of one phase of a batch (deletions: phase 0, insertions: 1) on
-// the batch workspace's counters, after the hub groups' count.
-tc_status launch_delta_fused(DeltaArgs A, StreamWs& w, int phase, int64_t edges, uint32_t* pv,
-                             unsigned long long* tri_out, cudaStream_t s) {
-  const PipeCand& shape = kPipeCand[default_cand(edges)];
+// The delta of one phase of a batch (deletions: phase 0, insertions: 1) on the batch workspace's
+// counters: hub groups, then the persistent kernel with the phase's end, on grids found outside
+// (launches only: it can run inside a stream capture).
+void delta_phase(tc_graph* g, StreamWs& w, const SchedParams& sp, int phase, int64_t cap, const PipeCand& shape,
+                 int ghub, int gdelta, uint32_t* pv, int64_t* delta, unsigned long long spin_ns, unsigned bar_extra,
+                 cudaStream_t s) {
+  DeltaArgs A = delta_args(g, sp);
+  unsigned long long* const tri = phase ? &w.st->tri_added : &w.st->tri_removed;
+  if (phase) A.ilist = w.ilist;
+  else A.dlist = w.dlist;
+  A.count_dev = phase ? &w.st->n_ins : &w.st->n_del;
+  A.sign = phase ? 1 : -1;
+  A.weight = 2;
   A.chunk = shape.chunk;
   A.split_min = shape.split_min;
+  A.spin_ns = spin_ns;
+  A.bar_extra = bar_extra;
   A.split_items = w.split_items;
   A.split_cnt = &w.st->n_split[phase];
-  A.entry_done = &w.st->entry_done[phase];
-  A.item_tag = w.item_tag;
-  A.item_epoch = w.item_epoch;
+  A.arrived = &w.st->arrived[phase];
   A.err = &w.st->err;
   A.bytes_out = &w.st->delta_bytes;
   A.e_next = &w.st->e_next[phase];
   A.i_next = &w.st->i_next[phase];
-  TC_TRY(launch_hub(A, w, phase, edges, pv, tri_out, s));
-  int grid = 0;
-  TC_TRY(fused_grid(shape.ctas, delta_smem(A), &grid));
-  k_delta_fused<<<grid, kThreads, delta_smem(A), s>>>(A, pv, tri_out);
-  return TC_OK;
+  hub_kernels(A, w, phase, cap, ghub, pv, tri, s);
+  PhaseEnd E;
+  memset(&E, 0, sizeof(E));
+  E.st = w.st;
+  if (phase) {
+    E.slot = w.ins_slot;
+    E.n_ins = &w.st->n_ins;
+    E.mark = g->mark;
+    E.delta = delta;
+    E.added = &w.st->tri_added;
+    E.removed = &w.st->tri_removed;
+  } else {
+    E.dlist = w.dlist;
+    E.n_del = &w.st->n_del;
+    E.cmp = compact_args(g, w);
+  }
+  k_delta_fused<<<gdelta, kThreads, delta_smem(A), s>>>(A, E, pv, tri);
 }
 
 }  // namespace
@@ -2356,7 +2503,6 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
   TC_TRY(ensure_stream_ws(g, b));
   StreamWs& w = *g->sw;
   const SchedParams sp = to_params(sched);
-  TC_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(BatchStatus), s));
   const int32_t* d_src = src;
   const int32_t* d_dst = dst;
   const uint8_t* d_del = is_delete;
@@ -2369,21 +2515,14 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
     d_del = is_delete ? w.isdel : nullptr;
   }
   const int L = bits_for(std::max(g->n, 2));
-  const uint64_t sent = (1ull << (2 * L + 1)) - 1;
-  SlackView view{g->start, g->used, g->pool};
-  const int gb = grid_for(std::max<int64_t>(b, 1), kThreads);
   // 1. canonical keys, sort, unique + classify
   if (b > 0) {
-    k_make_keys<<<gb, kThreads, 0, s>>>(d_src, d_dst, d_del, b, g->n, L, w.keys, w.st);
-    size_t tb = w.cub_bytes;
-    TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.keys, w.keys2, (int)b, 0, 2 * L + 1, s));
-    k_run_heads<<<gb, kThreads, 0, s>>>(w.keys2, b, sent, w.head);
-    TC_CUDA_TRY(cudaMemsetAsync(w.dk, 0xff, sizeof(uint64_t) * 2 * b, s));
-    k_classify<<<gb, kThreads, 0, s>>>(view, w.keys2, b, L, w.head, w.dlist, w.ilist, w.dk, w.st);
-    size_t tb2 = w.cub_bytes;
-    TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb2, w.dk, w.dk2, (int)(2 * b), 0, 64, s));
-    k_dir_runs<<<grid_for(2 * b, kThreads), kThreads, 0, s>>>(w.dk2, 2 * b, g->used, g->cap, g->slack_q10, w.run_start, w.long_runs, w.long_cnt, w.st);
+    TC_CUDA_TRY(load_batch(g, w, d_src, d_dst, d_del, b, b, L, s));
+    TC_CUDA_TRY(sort_batch(w, b, L, s));
+    TC_CUDA_TRY(classify_and_sort(g, w, b, L, s));
     TC_CUDA_TRY(cudaGetLastError());
+  } else {
+    TC_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(BatchStatus), s));
   }
   // 2. one synchronisation: sizes and the pool demand
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
@@ -2405,39 +2544,22 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
     scratch_pv = reinterpret_cast<uint32_t*>(g->pv_scratch);
     pv_use = scratch_pv;
   }
-  view = SlackView{g->start, g->used, g->pool};
+  int ghub = 0, gdelta = 0;
+  TC_TRY(hub_grid(&ghub));
+  TC_TRY(fused_grid(0, delta_smem(delta_args(g, sp)), &gdelta));
   // 3. deletions: mark, count on the pre-deletion graph, compact
   if (h.n_del > 0) {
-    const int gd = grid_for((int64_t)h.n_del, kThreads);
-    k_mark_deletions<<<gd, kThreads, 0, s>>>(w.dlist, w.st, g->start, g->mark, w.first_del);
-    DeltaArgs A = delta_args(g, sp);
-    A.dlist = w.dlist;
-    A.count_dev = &w.st->n_del;
-    A.sign = -1;
-    A.weight = 2;
-    TC_TRY(launch_delta_fused(A, w, 0, (int64_t)h.n_del, pv_use, &w.st->tri_removed, s));
-    k_endpoints<<<gd, kThreads, 0, s>>>(w.dlist, w.st, w.vlist);
-    k_bump_epoch<<<1, 32, 0, s>>>(w.d_epoch);
-    k_compact_marked<<<grid_for(2 * (int64_t)h.n_del * 32, kThreads), kThreads, 0, s>>>(
-        w.vlist, 2 * (int64_t)h.n_del, 1, nullptr, g->start, g->used, g->pool, g->mark, w.claim, w.d_epoch,
-        w.first_del, w.st);
-    long_compact(g, w, w.vlist, 2 * (int64_t)h.n_del, 1, nullptr, 2 * (int64_t)h.n_del, s);
+    const int64_t nd = (int64_t)h.n_del;
+    k_mark_deletions<<<grid_for(nd, kThreads), kThreads, 0, s>>>(w.dlist, w.st, g->start, g->mark, w.first_del, w.d_epoch);
+    delta_phase(g, w, sp, 0, nd, kPipeCand[default_cand(nd)], ghub, gdelta, pv_use, nullptr, kSpinNs, 0, s);
+    long_compact(g, w, s);
     TC_CUDA_TRY(cudaGetLastError());
   }
   // 4. insertions: merge into the lists, count on the post-insertion graph, clear marks
   if (h.n_ins > 0) {
-    k_insert_runs<<<grid_for((int64_t)h.n_runs * 32, kThreads), kThreads, 0, s>>>(
-        w.dk2, 2 * b, w.run_start, g->start, g->used, g->cap, g->pool, g->pool_cap, g->mark, w.ins_slot,
-        g->d_pool_top, g->slack_q10, w.st);
-    long_insert(g, w, 2 * b, g->mark, s);
-    DeltaArgs A = delta_args(g, sp);
-    A.ilist = w.ilist;
-    A.count_dev = &w.st->n_ins;
-    A.sign = 1;
-    A.weight = 2;
-    TC_TRY(launch_delta_fused(A, w, 1, (int64_t)h.n_ins, pv_use, &w.st->tri_added, s));
-    k_clear_slots<<<grid_for(2 * (int64_t)h.n_ins, kThreads), kThreads, 0, s>>>(w.ins_slot, 2 * (int64_t)h.n_ins,
-                                                                                  nullptr, g->mark);
+    const int64_t ni = (int64_t)h.n_ins;
+    insert_sorted_keys(g, w, 2 * b, (int64_t)h.n_runs, L, g->mark, s);
+    delta_phase(g, w, sp, 1, ni, kPipeCand[default_cand(ni)], ghub, gdelta, pv_use, nullptr, kSpinNs, 0, s);
     TC_CUDA_TRY(cudaGetLastError());
   }
   g->m += 2 * ((int64_t)h.n_ins - (int64_t)h.n_del);
@@ -2523,10 +2645,11 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   SlackView view{g->start, g->used, g->pool};
   // entries come sorted by (src, dst): the packed keys of the new ones stay sorted, sentinel
   // elsewhere; sort once more to push the sentinels to the end.
-  k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, w.dk);
+  const int L = bits_for(std::max(g->n, 2));
+  k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, L, w.dk);
   size_t tb = w.cub_bytes;
-  TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, 64, s));
-  k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, g->used, g->cap, g->slack_q10, w.run_start, w.long_runs, w.long_cnt, w.st);
+  TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, 2 * L, s));
+  k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.run_start, w.st);
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaMemcpyAsync(&w.st_host->pool_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2534,10 +2657,7 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   g->pool_top = (int64_t)h.pool_top;
   TC_TRY(ensure_pool(g, (int64_t)h.demand, s));
   if (h.n_runs > 0) {
-    k_insert_runs<<<grid_for((int64_t)h.n_runs * 32, kThreads), kThreads, 0, s>>>(
-        w.dk2, b, w.run_start, g->start, g->used, g->cap, g->pool, g->pool_cap, nullptr, w.ins_slot, g->d_pool_top,
-        g->slack_q10, w.st);
-    long_insert(g, w, b, nullptr, s);
+    insert_sorted_keys(g, w, b, (int64_t)h.n_runs, L, nullptr, s);
     TC_CUDA_TRY(cudaGetLastError());
   }
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
@@ -2564,10 +2684,8 @@ tc_status tc_delete_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   k_mark_dir_deletions<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, g->mark, w.first_del,
                                                                    w.vlist, w.counter);
   k_bump_epoch<<<1, 32, 0, s>>>(w.d_epoch);
-  k_compact_marked<<<grid_for(b * 32, kThreads), kThreads, 0, s>>>(w.vlist, b, 1, w.counter, g->start, g->used,
-                                                                   g->pool, g->mark, w.claim, w.d_epoch, w.first_del,
-                                                                   w.st);
-  long_compact(g, w, w.vlist, b, 1, w.counter, b, s);
+  k_compact<<<grid_for(b * 32, kThreads), kThreads, 0, s>>>(compact_args(g, w), w.vlist, w.counter, w.st);
+  long_compact(g, w, s);
   TC_CUDA_TRY(cudaGetLastError());
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2669,7 +2787,6 @@ struct tc_pipeline {
   unsigned long long spin_ns = tc::kSpinNs;          // bound of the delta kernel's barrier wait
   unsigned bar_extra = 0;                            // (test hook: arrivals that never come)
   cudaStream_t cs = nullptr;     // capture stream
-  int64_t* d_b = nullptr;
   tc::BatchStatus* h_st = nullptr;          // pinned: status of the last batch
   unsigned long long* h_top = nullptr;      // pinned: pool bump pointer after it
   uint32_t* pv_scratch = nullptr;
@@ -2782,79 +2899,27 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
   const PipeCand& pc = kPipeCand[cand];
   cudaStream_t s = p->cs;
   const int L = bits_for(std::max(g->n, 2));
-  const uint64_t sent = (1ull << (2 * L + 1)) - 1;
-  const SlackView view{g->start, g->used, g->pool};
-  const int gb = grid_for(cap, kThreads);
-  const int g2 = grid_for(2 * cap, kThreads);
-  const int gw = grid_for(2 * cap * 32, kThreads);
   int gdelta = 0, ghub = 0;
-  const size_t dsm = delta_smem(delta_args(g, p->sp));
-  TC_TRY(fused_grid(pc.ctas, dsm, &gdelta));
+  TC_TRY(fused_grid(pc.ctas, delta_smem(delta_args(g, p->sp)), &gdelta));
   TC_TRY(hub_grid(&ghub));
   cudaGraph_t graph = nullptr;
   TC_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
   do {
-    cudaMemsetAsync(w.st, 0, sizeof(BatchStatus), s);
-    k_make_keys_cap<<<gb, kThreads, 0, s>>>(w.src, w.dst, w.isdel, p->d_b, cap, g->n, L, w.keys, w.st);
-    size_t tb = w.cub_bytes;
-    if ((e = cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.keys, w.keys2, (int)cap, 0, 2 * L + 1, s)) != cudaSuccess)
-      break;
-    k_run_heads<<<gb, kThreads, 0, s>>>(w.keys2, cap, sent, w.head);
-    cudaMemsetAsync(w.dk, 0xff, sizeof(uint64_t) * 2 * cap, s);
-    k_classify<<<gb, kThreads, 0, s>>>(view, w.keys2, cap, L, w.head, w.dlist, w.ilist, w.dk, w.st);
-    size_t tb2 = w.cub_bytes;
-    if ((e = cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb2, w.dk, w.dk2, (int)(2 * cap), 0, 64, s)) != cudaSuccess)
-      break;
-    k_dir_runs<<<g2, kThreads, 0, s>>>(w.dk2, 2 * cap, g->used, g->cap, g->slack_q10, w.run_start, w.long_runs, w.long_cnt, w.st);
+    if ((e = sort_batch(w, cap, L, s)) != cudaSuccess) break;
+    if ((e = classify_and_sort(g, w, cap, L, s)) != cudaSuccess) break;
     // deletions: mark, count on the pre-deletion graph, compact
-    k_mark_deletions<<<gb, kThreads, 0, s>>>(w.dlist, w.st, g->start, g->mark, w.first_del);
-    DeltaArgs A = delta_args(g, p->sp);
-    A.dlist = w.dlist;
-    A.count_dev = &w.st->n_del;
-    A.sign = -1;
-    A.weight = 2;
-    A.chunk = pc.chunk;
-    A.split_min = pc.split_min;
-    A.spin_ns = p->spin_ns;
-    A.bar_extra = p->bar_extra;
-    A.split_items = w.split_items;
-    A.split_cnt = &w.st->n_split[0];
-    A.entry_done = &w.st->entry_done[0];
-    A.item_tag = w.item_tag;
-    A.item_epoch = w.item_epoch;
-    A.err = &w.st->err;
-    A.bytes_out = &w.st->delta_bytes;
-    A.e_next = &w.st->e_next[0];
-    A.i_next = &w.st->i_next[0];
+    k_mark_deletions<<<grid_for(cap, kThreads), kThreads, 0, s>>>(w.dlist, w.st, g->start, g->mark, w.first_del,
+                                                                  w.d_epoch);
     if (p->profile) cudaEventRecordWithFlags(p->pev[0], s, cudaEventRecordExternal);
-    hub_kernels(A, w, 0, cap, ghub, pv, &w.st->tri_removed, s);
-    k_delta_fused<<<gdelta, kThreads, dsm, s>>>(A, pv, &w.st->tri_removed);
+    delta_phase(g, w, p->sp, 0, cap, pc, ghub, gdelta, pv, nullptr, p->spin_ns, p->bar_extra, s);
     if (p->profile) cudaEventRecordWithFlags(p->pev[1], s, cudaEventRecordExternal);
-    k_endpoints<<<gb, kThreads, 0, s>>>(w.dlist, w.st, w.vlist);
-    k_bump_epoch<<<1, 32, 0, s>>>(w.d_epoch);
-    k_compact_marked<<<gw, kThreads, 0, s>>>(w.vlist, 0, 2, &w.st->n_del, g->start, g->used, g->pool, g->mark,
-                                             w.claim, w.d_epoch, w.first_del, w.st);
-    long_compact(g, w, w.vlist, 0, 2, &w.st->n_del, 2 * cap, s);
+    long_compact(g, w, s);
     // insertions: merge, count on the post-insertion graph, clear the marks
-    k_insert_runs<<<gw, kThreads, 0, s>>>(w.dk2, 2 * cap, w.run_start, g->start, g->used, g->cap, g->pool,
-                                          g->pool_cap, g->mark, w.ins_slot, g->d_pool_top, g->slack_q10, w.st);
-    long_insert(g, w, 2 * cap, g->mark, s);
-    DeltaArgs B = A;
-    B.dlist = nullptr;
-    B.ilist = w.ilist;
-    B.count_dev = &w.st->n_ins;
-    B.sign = 1;
-    B.split_cnt = &w.st->n_split[1];
-    B.entry_done = &w.st->entry_done[1];
-    B.e_next = &w.st->e_next[1];
-    B.i_next = &w.st->i_next[1];
+    insert_sorted_keys(g, w, 2 * cap, 2 * cap, L, g->mark, s);
     if (p->profile) cudaEventRecordWithFlags(p->pev[2], s, cudaEventRecordExternal);
-    hub_kernels(B, w, 1, cap, ghub, pv, &w.st->tri_added, s);
-    k_delta_fused<<<gdelta, kThreads, dsm, s>>>(B, pv, &w.st->tri_added);
+    delta_phase(g, w, p->sp, 1, cap, pc, ghub, gdelta, pv, delta, p->spin_ns, p->bar_extra, s);
     if (p->profile) cudaEventRecordWithFlags(p->pev[3], s, cudaEventRecordExternal);
-    k_clear_slots<<<g2, kThreads, 0, s>>>(w.ins_slot, 0, &w.st->n_ins, g->mark);
-    k_add_delta<<<1, 32, 0, s>>>(delta, &w.st->tri_added, &w.st->tri_removed);
     cudaMemcpyAsync(p->h_st, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(p->h_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     e = cudaGetLastError();
@@ -2941,7 +3006,6 @@ tc_status tc_pipeline_create(tc_graph* g, int64_t max_batch, const tc_sched* sch
   do {
     if ((rc = ensure_stream_ws(g, p->b_max)) != TC_OK) break;
     if (cudaStreamCreateWithFlags(&p->cs, cudaStreamNonBlocking) != cudaSuccess ||
-        ::tc::dev_malloc(&p->d_b, sizeof(int64_t)) != cudaSuccess ||
         cudaMallocHost(&p->h_st, sizeof(BatchStatus)) != cudaSuccess ||
         cudaMallocHost(&p->h_top, sizeof(unsigned long long)) != cudaSuccess ||
         ::tc::dev_malloc(&p->pv_scratch, sizeof(uint32_t) * ((size_t)g->n + 1)) != cudaSuccess ||
@@ -2970,7 +3034,6 @@ tc_status tc_pipeline_destroy(tc_pipeline* p) {
   if (p->pending) cudaEventSynchronize(p->done);
   drop_graphs(p);
   if (p->cs) cudaStreamDestroy(p->cs);
-  cudaFree(p->d_b);
   cudaFreeHost(p->h_st);
   cudaFreeHost(p->h_top);
   cudaFree(p->pv_scratch);
@@ -3021,10 +3084,8 @@ tc_status tc_pipeline_apply(tc_pipeline* p, const int32_t* d_src, const int32_t*
     cand = arm < kPipeCands ? arm : 0;
   }
   if (!p->exec[bin][cand]) TC_TRY(pipe_capture(p, bin, cand, pv, delta));
-  // the batch into the capacity-sized buffers the graph reads, and its size
-  k_load_batch<<<grid_for(b, kThreads), kThreads, 0, s>>>(d_src, d_dst, d_is_delete, b, w.src, w.dst, w.isdel,
-                                                         p->d_b);
-  TC_CUDA_TRY(cudaGetLastError());
+  // the batch's keys, padded to the bin's capacity, where the graph reads them
+  TC_CUDA_TRY(load_batch(g, w, d_src, d_dst, d_is_delete, b, p->bin_cap[bin], bits_for(std::max(g->n, 2)), s));
   p->timing = arm >= 0;
   if (p->timing) TC_CUDA_TRY(cudaEventRecord(p->t0, s));
   TC_CUDA_TRY(cudaGraphLaunch(p->exec[bin][cand], s));
