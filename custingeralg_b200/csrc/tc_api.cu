@@ -348,6 +348,7 @@ tc_status tc_workspace_release(void) {
   std::lock_guard<std::mutex> lk(g.mu);
   TC_CUDA_TRY(cudaDeviceSynchronize());  // no count may still use it
   g.ws[dev].release();
+  release_sort_ws(dev);
   return TC_OK;
 }
 

@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 
 #include "tc_graph.cuh"
 
@@ -31,9 +32,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr uint64_t kSentinel = ~0ull;
 constexpr int kLongList = 2048;  // lists longer than this are rewritten by a whole CTA
-// Tile shape of the cuStinger-style delta count (tc_count_batch):
-constexpr int kDeltaSplit = 2048;   // intersections whose shorter list is longer are split ...
-constexpr int kDeltaChunk = 1024;   // ... into items of this many entries of the shorter list
 constexpr int64_t kDeltaItems = 1 << 20;  // capacity of the split-item queue
 constexpr unsigned long long kNoItem = ~0ull;
 constexpr int kGrab = 4;  // most changed edges a warp takes per grab from the delta kernel's queue
@@ -537,8 +535,9 @@ __global__ void __launch_bounds__(kThreads) k_insert_runs(const InsertArgs I, Ba
     const int32_t m31 = __shfl_sync(kFull, mine, 31);
     // Old entries: final position i + #(new < A[i]); backwards in steps of 128 entries, each read whole
     // before its first write, so that, in place, no unread entry is overwritten (targets never
-    // precede sources). The new entries below an old one are counted from the lanes for runs of at
-    // most 32 (the usual case), else by a search of the keys.
+    // precede sources). The new entries below an old one are counted from the lanes: one by one for
+    // runs of at most 8 (the usual case), by a search over the lanes up to 32; else by a search of
+    // the keys.
     const int32_t low = (keep_below / 128) * 128;
     for (int32_t base = a > 0 ? ((a - 1) / 128) * 128 : -1; base >= low; base -= 128) {
       int32_t val[4];
@@ -548,10 +547,19 @@ __global__ void __launch_bounds__(kThreads) k_insert_runs(const InsertArgs I, Ba
         val[q] = i < a && i >= keep_below ? A[i] : -1;
       }
       __syncwarp();
+      int32_t few[4] = {0, 0, 0, 0};
+      if (c <= 8) {
+        for (int j = 0; j < c; ++j) {
+          const int32_t x = __shfl_sync(kFull, mine, j);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) few[q] += x < val[q];
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        int32_t below = 0;
-        if (c <= 32) {
+        int32_t below = few[q];
+        if (c <= 8) {
+        } else if (c <= 32) {
 #pragma unroll
           for (int h = 16; h > 0; h >>= 1)
             if (__shfl_sync(kFull, mine, below + h - 1) < val[q]) below += h;
@@ -1019,17 +1027,22 @@ __device__ __forceinline__ int cell_of(int a, int b) {
   return ca * 16 + cb;
 }
 
+// Does the batch hold the non-duplicate entry (x, y)?
+__device__ __forceinline__ bool batch_has(const BatchLists& bl, const int32_t x, const int32_t y) {
+  const int32_t hi = bl.off[x + 1];
+  int32_t l = bl.off[x], h = hi;
+  while (l < h) {
+    const int32_t mid = (l + h) >> 1;
+    if (bl.dst[mid] < y) l = mid + 1;
+    else h = mid;
+  }
+  return l < hi && bl.dst[l] == y && bl.dup[l] == 0;
+}
+
 template <int PRED>
 __device__ __forceinline__ bool changed(const DeltaArgs& A, int32_t owner, int64_t slot_abs, int32_t w) {
   if (PRED == kPredMark) return A.mark[slot_abs] != 0;
-  const int32_t lo = A.bl.off[owner], hi = A.bl.off[owner + 1];
-  int32_t l = lo, h = hi;
-  while (l < h) {
-    const int32_t mid = (l + h) >> 1;
-    if (A.bl.dst[mid] < w) l = mid + 1;
-    else h = mid;
-  }
-  return l < hi && A.bl.dst[l] == w && A.bl.dup[l] == 0;
+  return batch_has(A.bl, owner, w);
 }
 
 // Entry e of the changed-edge list: its endpoints and whether it adds to the total (the
@@ -1108,7 +1121,7 @@ __device__ __forceinline__ DeltaPair delta_pair(const DeltaArgs& A, int32_t x, i
 // per-vertex update here, the endpoints get theirs from the caller.
 template <int PRED>
 __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaPair& P, int32_t i_begin,
-                                                int32_t i_end, uint32_t* __restrict__ pv) {
+                                                int32_t i_end, const uint32_t inc, uint32_t* __restrict__ pv) {
   const int lane = threadIdx.x & 31;
   const int32_t* L = A.g.ind;
   uint32_t c = 0;
@@ -1117,7 +1130,7 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
     const bool keep = (!ca || P.key < ekey(P.oa, w)) && (!cb || P.key < ekey(P.ob, w));
     if (keep) {
       ++c;
-      atomicAdd(&pv[w], A.weight * (uint32_t)A.sign);
+      atomicAdd(&pv[w], inc);
     }
   };
   auto on_match = [&](int64_t ia, int64_t ib, int32_t w) { match(changed<PRED>(A, P.oa, P.sa + ia, w), ib, w); };
@@ -1263,8 +1276,13 @@ __device__ __forceinline__ int edge_shard(int32_t x, int32_t y, int nshards) {
   return (int)((z ^ (z >> 31)) % (uint64_t)nshards);
 }
 
+// Flags of its split items: the edge counts for both directions; its triangles enter the total.
+constexpr unsigned long long kItemTwice = 1ull << 62, kItemTotal = 1ull << 61;
+
 // The cuStinger-style count (tc_count_batch): the triangle delta of the batch's edges, one warp per
-// edge (warp-strided; with shards, only this rank's edges). An edge whose shorter list is longer
+// edge (warp-strided; with shards, only this rank's edges). Both directions of an edge keep the same
+// triangles, so where the batch holds both (as a symmetric batch does) the one from the smaller
+// id counts for both: its increments are doubled and the other one is skipped. An edge whose shorter list is longer
 // than A.split_min (two hubs) would be one warp's serial tail of the whole launch: it is queued
 // instead as items of A.chunk entries of its shorter list, which the second launch spreads over
 // all warps (a full queue leaves the edge to this warp). Lane 0 of each warp accumulates the kept
@@ -1277,20 +1295,27 @@ __device__ __forceinline__ void batch_entries(const DeltaArgs& A, uint32_t* __re
     int32_t x, y;
     bool count_total;
     if (!delta_entry<kPredBatch>(A, e, x, y, count_total)) continue;
+    const bool both = batch_has(A.bl, y, x);
+    if (both && x > y) continue;  // counted from (y, x)
+    uint32_t times = both ? 2 : 1;
     if (A.nshards > 1 && edge_shard(x, y, A.nshards) != A.shard) continue;
     const int32_t lx = A.g.len(x), ly = A.g.len(y);
     if (lx < 2 || ly < 2) continue;
     const int64_t sx = A.g.start(x), sy = A.g.start(y);
     if (A.only_present) {
-      // the edge must exist for its triangles to be destroyed
+      // the edge must exist for its triangles to be destroyed: each direction is looked up in its list
       bool pres = false;
-      if (lane == 0) {
-        const int64_t p = lower_bound(A.g.ind, sx, sx + lx, y);
-        pres = p < sx + lx && A.g.ind[p] == y;
+      if (lane == 0 || (lane == 1 && both)) {
+        const int64_t p = lane == 0 ? lower_bound(A.g.ind, sx, sx + lx, y) : lower_bound(A.g.ind, sy, sy + ly, x);
+        pres = lane == 0 ? p < sx + lx && A.g.ind[p] == y : p < sy + ly && A.g.ind[p] == x;
       }
       __syncwarp();
-      if (!__shfl_sync(kFull, pres, 0)) continue;
+      const unsigned m = __ballot_sync(kFull, pres);
+      if (m == 0) continue;
+      times = __popc(m);
+      count_total = count_total && (m & 1u);
     }
+    const uint32_t inc = A.weight * (uint32_t)A.sign * times;
     const DeltaPair P = delta_pair<kPredBatch>(A, x, y, lx, ly, sx, sy);
     if (A.cell_filter == -2 || (A.cell_filter >= 0 && P.cell != A.cell_filter)) continue;
     if (lane == 0 && count_total) bytes_acc += 4ull * (unsigned long long)(lx + ly) + 8ull;
@@ -1302,13 +1327,15 @@ __device__ __forceinline__ void batch_entries(const DeltaArgs& A, uint32_t* __re
       const bool fits = at + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
       for (int j = lane; j < nch; j += 32)
         if (at + j < (unsigned long long)kDeltaItems)
-          A.split_items[at + j] = fits ? ((unsigned long long)e << 24) | (unsigned long long)j : kNoItem;
+          A.split_items[at + j] = fits ? ((unsigned long long)e << 24) | (unsigned long long)j |
+                                             (times == 2 ? kItemTwice : 0) | (count_total ? kItemTotal : 0)
+                                       : kNoItem;
       if (fits) continue;
     }
-    const uint32_t c = delta_range<kPredBatch>(A, P, 0, P.la, pv);
+    const uint32_t c = delta_range<kPredBatch>(A, P, 0, P.la, inc, pv);
     if (lane == 0 && c) {
-      atomicAdd(&pv[x], c * A.weight * (uint32_t)A.sign);
-      atomicAdd(&pv[y], c * A.weight * (uint32_t)A.sign);
+      atomicAdd(&pv[x], c * inc);
+      atomicAdd(&pv[y], c * inc);
       if (count_total) tri_acc += c;
     }
   }
@@ -1323,18 +1350,20 @@ __device__ __forceinline__ void batch_items(const DeltaArgs& A, uint32_t* __rest
   for (int64_t q = gw; q < n_items; q += nw) {
     const unsigned long long item = A.split_items[q];
     if (item == kNoItem) continue;
-    const int64_t e = (int64_t)(item >> 24);
+    const int64_t e = (int64_t)((item & ~(kItemTwice | kItemTotal)) >> 24);
     int32_t x, y;
     bool count_total;
     if (!delta_entry<kPredBatch>(A, e, x, y, count_total)) continue;
+    count_total = (item & kItemTotal) != 0;
     const DeltaPair P =
         delta_pair<kPredBatch>(A, x, y, A.g.len(x), A.g.len(y), A.g.start(x), A.g.start(y));
     const int32_t i0 = (int32_t)(item & 0xffffffu) * A.chunk;
     if (i0 >= P.la) continue;
-    const uint32_t c = delta_range<kPredBatch>(A, P, i0, min(P.la, i0 + A.chunk), pv);
+    const uint32_t inc = A.weight * (uint32_t)A.sign * (item & kItemTwice ? 2u : 1u);
+    const uint32_t c = delta_range<kPredBatch>(A, P, i0, min(P.la, i0 + A.chunk), inc, pv);
     if (lane == 0 && c) {
-      atomicAdd(&pv[x], c * A.weight * (uint32_t)A.sign);
-      atomicAdd(&pv[y], c * A.weight * (uint32_t)A.sign);
+      atomicAdd(&pv[x], c * inc);
+      atomicAdd(&pv[y], c * inc);
       if (count_total) tri_acc += c;
     }
   }
@@ -1358,10 +1387,11 @@ __device__ __forceinline__ DeltaPair described_pair(const DeltaArgs& A, const De
 // Entries [i0, i1) of a described edge's shorter list, run by the warp.
 __device__ __forceinline__ void delta_part(const DeltaArgs& A, uint32_t* __restrict__ pv, const DeltaDesc& d,
                                            const int32_t i0, const int32_t i1, unsigned long long& tri_acc) {
-  const uint32_t c = delta_range<kPredMark>(A, described_pair(A, d), i0, i1, pv);
+  const uint32_t inc = A.weight * (uint32_t)A.sign;
+  const uint32_t c = delta_range<kPredMark>(A, described_pair(A, d), i0, i1, inc, pv);
   if ((threadIdx.x & 31) == 0 && c) {
-    atomicAdd(&pv[d.oa], c * A.weight * (uint32_t)A.sign);
-    atomicAdd(&pv[d.ob], c * A.weight * (uint32_t)A.sign);
+    atomicAdd(&pv[d.oa], c * inc);
+    atomicAdd(&pv[d.ob], c * inc);
     tri_acc += c;
   }
 }
@@ -1565,9 +1595,11 @@ constexpr int kHubPass = 3 << (kHubSlotBits - 2);  // entries of N(h) per pass (
 constexpr int32_t kHubMarkBit = INT32_MIN;    // bit 31 of a stored key: the edge (h, key) is changed
 constexpr int64_t kHubSearchCost = 64;        // an item's estimate of one range search, in probes
 #ifndef TC_HUB_ITEM_LOG2
-#define TC_HUB_ITEM_LOG2 17
+#define TC_HUB_ITEM_LOG2 19
 #endif
-constexpr int64_t kHubItemMin = 1ll << TC_HUB_ITEM_LOG2;  // probes of work per item at least ...
+// probes of work per item at least (a build and three block barriers each; 2 x 10^6 updates on R-MAT
+// 22: 2^17 10.90 ms a pass, 2^18 10.67, 2^19 10.57, 2^20 10.63) ...
+constexpr int64_t kHubItemMin = 1ll << TC_HUB_ITEM_LOG2;
 constexpr int64_t kHubBuildShare = 16;        // ... and at least this many times its table build
 constexpr int64_t kHubItemsPerUpdate = 4;     // item queue capacity per batch update
 constexpr int64_t kHubUnitsPerUpdate = kHubUnit >= 1024 ? 4 : 4 * 1024 / kHubUnit;  // unit slots per update
@@ -2257,8 +2289,6 @@ DeltaArgs delta_args(tc_graph* g, const SchedParams& sp) {
   A.search_ratio_x16 = sp.search_ratio_x16;
   A.use_table = sp.use_table;
   A.cell_filter = sp.cell_filter;
-  A.split_min = kDeltaSplit;
-  A.chunk = kDeltaChunk;
   A.shard = sp.shard;
   A.nshards = sp.nshards;
   A.spin_ns = kSpinNs;
@@ -2484,7 +2514,96 @@ void delta_phase(tc_graph* g, StreamWs& w, const SchedParams& sp, int phase, int
   k_delta_fused<<<gdelta, kThreads, delta_smem(A), s>>>(A, E, pv, tri);
 }
 
+// Working memory of tc_batch_sort. Each device keeps one, used by one call at a time (the call waits
+// for its stream before it returns it); a call that finds it taken, or needs more than kSortWsKeep
+// bytes, works on memory of its own. Allocating and freeing seven arrays per call took longer than
+// sorting the batch (100,000 entries of a graph of 2^20 vertices: 1-10 ms against 0.2 ms).
+constexpr size_t kSortWsKeep = (size_t)256 << 20;
+
+struct SortWs {
+  int64_t n_cap = -1, b_cap = -1;
+  uint64_t *k1 = nullptr, *k2 = nullptr;  // [b]
+  void* tmp = nullptr;
+  size_t tmp_bytes = 0;
+  int32_t* cnt = nullptr;                 // [n + 1]
+  int64_t *off64 = nullptr, *tiles = nullptr;
+  unsigned* err = nullptr;
+
+  void release() {
+    cudaFree(k1); cudaFree(k2); cudaFree(tmp); cudaFree(cnt); cudaFree(off64); cudaFree(tiles); cudaFree(err);
+    *this = SortWs();
+  }
+  size_t bytes() const {
+    return 16 * (size_t)std::max<int64_t>(b_cap, 0) + tmp_bytes + 12 * (size_t)std::max<int64_t>(n_cap, 0);
+  }
+  // n vertices, b entries; after a failure nothing is held.
+  tc_status ensure(int64_t n, int64_t b) {
+    if (n <= n_cap && b <= b_cap) return TC_OK;
+    const int64_t nn = std::max(n, n_cap), nb = std::max(b, b_cap);
+    release();
+    size_t tb = 0;
+    const size_t bb = (size_t)std::max<int64_t>(nb, 1);
+    const bool ok = ::tc::dev_malloc(&k1, sizeof(uint64_t) * bb) == cudaSuccess &&
+                    ::tc::dev_malloc(&k2, sizeof(uint64_t) * bb) == cudaSuccess &&
+                    ::tc::dev_malloc(&cnt, sizeof(int32_t) * ((size_t)nn + 1)) == cudaSuccess &&
+                    ::tc::dev_malloc(&off64, sizeof(int64_t) * ((size_t)nn + 2)) == cudaSuccess &&
+                    ::tc::dev_malloc(&tiles, sizeof(int64_t) * (size_t)(scan_tiles(nn) + 1)) == cudaSuccess &&
+                    ::tc::dev_malloc(&err, sizeof(unsigned)) == cudaSuccess &&
+                    cub::DeviceRadixSort::SortKeys(nullptr, tb, k1, k2, (int)bb, 0, 64) == cudaSuccess &&
+                    ::tc::dev_malloc(&tmp, std::max<size_t>(tb, 1)) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      release();
+      return fail(TC_ERR_OOM, "batch sort: allocation failed");
+    }
+    tmp_bytes = tb;
+    n_cap = nn;
+    b_cap = nb;
+    return TC_OK;
+  }
+};
+
+struct SortWsPool {
+  std::mutex mu[64];
+  SortWs ws[64];
+};
+SortWsPool& sort_ws_pool() {
+  static SortWsPool* p = new SortWsPool();  // intentionally leaked: outlives CUDA teardown
+  return *p;
+}
+
+// One call's use of a workspace: the device's, or its own. Unless done() says that the call's work on
+// it has ended, leaving waits for the device first.
+class SortWsLease {
+ public:
+  SortWsLease() {
+    if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) dev_ = -1;
+    if (dev_ >= 0 && !sort_ws_pool().mu[dev_].try_lock()) dev_ = -1;
+  }
+  ~SortWsLease() {
+    if (!done_) cudaDeviceSynchronize();
+    SortWs& w = ws();
+    if (dev_ < 0 || w.bytes() > kSortWsKeep) w.release();
+    if (dev_ >= 0) sort_ws_pool().mu[dev_].unlock();
+  }
+  SortWsLease(const SortWsLease&) = delete;
+  SortWsLease& operator=(const SortWsLease&) = delete;
+  SortWs& ws() { return dev_ >= 0 ? sort_ws_pool().ws[dev_] : own_; }
+  void done() { done_ = true; }
+
+ private:
+  int dev_ = -1;
+  bool done_ = false;
+  SortWs own_;
+};
+
 }  // namespace
+
+void release_sort_ws(int dev) {
+  std::lock_guard<std::mutex> lk(sort_ws_pool().mu[dev]);
+  sort_ws_pool().ws[dev].release();
+}
+
 }  // namespace tc
 
 using namespace tc;
@@ -2589,48 +2708,26 @@ tc_status tc_batch_sort(int32_t nv, int32_t* d_src, int32_t* d_dst, int64_t b, i
     return fail(TC_ERR_INVALID_ARG, "invalid batch arguments");
   if (b > (int64_t)INT32_MAX / 2) return fail(TC_ERR_CAPACITY, "batch too large");
   cudaStream_t s = (cudaStream_t)stream;
-  uint64_t *k1 = nullptr, *k2 = nullptr;
-  void* tmp = nullptr;
-  size_t tb = 0;
-  int32_t* cnt = nullptr;
-  int64_t *off64 = nullptr, *tiles = nullptr;
-  unsigned* err = nullptr;
-  tc_status rc = TC_OK;
+  SortWsLease lease;
+  SortWs& w = lease.ws();
+  TC_TRY(w.ensure(nv, b));
   unsigned herr = 0;
-  do {
-    if (::tc::dev_malloc(&k1, sizeof(uint64_t) * std::max<int64_t>(b, 1)) != cudaSuccess ||
-        ::tc::dev_malloc(&k2, sizeof(uint64_t) * std::max<int64_t>(b, 1)) != cudaSuccess ||
-        ::tc::dev_malloc(&cnt, sizeof(int32_t) * ((size_t)nv + 1)) != cudaSuccess ||
-        ::tc::dev_malloc(&off64, sizeof(int64_t) * ((size_t)nv + 2)) != cudaSuccess ||
-        ::tc::dev_malloc(&tiles, sizeof(int64_t) * (size_t)(scan_tiles(nv) + 1)) != cudaSuccess ||
-        ::tc::dev_malloc(&err, sizeof(unsigned)) != cudaSuccess) {
-      rc = fail(TC_ERR_OOM, "batch sort: allocation failed");
-      break;
-    }
-    cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nv + 1), s);
-    cudaMemsetAsync(err, 0, sizeof(unsigned), s);
-    if (b > 0) {
-      k_pack_dir<<<grid_for(b, kThreads), kThreads, 0, s>>>(d_src, d_dst, b, k1);
-      cub::DeviceRadixSort::SortKeys(nullptr, tb, k1, k2, (int)b, 0, 64, s);
-      if (::tc::dev_malloc(&tmp, std::max<size_t>(tb, 1)) != cudaSuccess) {
-        rc = fail(TC_ERR_OOM, "batch sort: allocation failed");
-        break;
-      }
-      cub::DeviceRadixSort::SortKeys(tmp, tb, k1, k2, (int)b, 0, 64, s);
-      k_unpack_dir<<<grid_for(b, kThreads), kThreads, 0, s>>>(k2, b, nv, d_src, d_dst, d_dup, cnt, err);
-    }
-    rc = scan_counts(cnt, nv, off64, tiles, s);
-    if (rc != TC_OK) break;
-    k_to_int32<<<grid_for((int64_t)nv + 1, kThreads), kThreads, 0, s>>>(off64, nv, d_offsets);
-    cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) {
-      rc = fail(TC_ERR_CUDA, "batch sort: %s", cudaGetErrorString(cudaGetLastError()));
-      break;
-    }
-    if (herr) rc = fail(TC_ERR_INVALID_ARG, "batch has vertex ids outside [0, %d)", nv);
-  } while (0);
-  cudaFree(k1); cudaFree(k2); cudaFree(tmp); cudaFree(cnt); cudaFree(off64); cudaFree(tiles); cudaFree(err);
-  return rc;
+  TC_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(int32_t) * ((size_t)nv + 1), s));
+  TC_CUDA_TRY(cudaMemsetAsync(w.err, 0, sizeof(unsigned), s));
+  if (b > 0) {
+    k_pack_dir<<<grid_for(b, kThreads), kThreads, 0, s>>>(d_src, d_dst, b, w.k1);
+    size_t tb = w.tmp_bytes;
+    TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.tmp, tb, w.k1, w.k2, (int)b, 0, 64, s));
+    k_unpack_dir<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.k2, b, nv, d_src, d_dst, d_dup, w.cnt, w.err);
+  }
+  TC_TRY(scan_counts(w.cnt, nv, w.off64, w.tiles, s));
+  k_to_int32<<<grid_for((int64_t)nv + 1, kThreads), kThreads, 0, s>>>(w.off64, nv, d_offsets);
+  TC_CUDA_TRY(cudaGetLastError());
+  TC_CUDA_TRY(cudaMemcpyAsync(&herr, w.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  TC_CUDA_TRY(cudaStreamSynchronize(s));  // the working memory is free again
+  lease.done();
+  if (herr) return fail(TC_ERR_INVALID_ARG, "batch has vertex ids outside [0, %d)", nv);
+  return TC_OK;
 }
 
 tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_dst, int64_t b, int32_t* d_dup,
@@ -2711,6 +2808,9 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
     A.sign = sign;
     A.weight = 1;
     A.only_present = sign < 0;
+    const PipeCand& shape = kPipeCand[default_cand(b / 2)];
+    A.chunk = shape.chunk;
+    A.split_min = shape.split_min;
     A.split_items = w.split_items;
     A.split_cnt = &w.st->n_split[0];
     TC_CUDA_TRY(cudaMemsetAsync(A.split_cnt, 0, sizeof(unsigned long long), s));
