@@ -317,37 +317,47 @@ __device__ __forceinline__ int32_t dir_dst(const uint64_t k, const int L) {
 
 // Heads of source-vertex runs in the sorted directed entries ((src << L) | dst), and the pool slots
 // the lists that must move could take (computed on the pre-deletion lengths, an upper bound).
-// A run whose list will be long (used + new > kLongList) is stored as -1 - start.
+// A run is stored as (start, length), one whose list will be long (used + new > kLongList) as
+// (-1 - start, length).
 __device__ __forceinline__ void dir_run(const uint64_t* __restrict__ dk, const int64_t i, const int64_t nd_cap, const int L,
                                         const int32_t* __restrict__ used, const int32_t* __restrict__ cap,
-                                        const int32_t slack_q10, int32_t* __restrict__ run_start,
+                                        const int32_t slack_q10, int2* __restrict__ runs,
                                         BatchStatus* __restrict__ st) {
   const uint64_t k = dk[i];
   if (k == kSentinel) return;
   const uint32_t v = (uint32_t)(k >> L);
   if (i > 0 && (uint32_t)(dk[i - 1] >> L) == v) return;
-  int64_t j = i;
-  while (j + 1 < nd_cap && dk[j + 1] != kSentinel && (uint32_t)(dk[j + 1] >> L) == v) ++j;
-  const int32_t c = (int32_t)(j - i + 1);
+  // the run's end: doubling steps, then a binary search (a hub's run can hold 10^4 entries; a
+  // sentinel's source is 2^32 - 1)
+  int64_t end = i + 1, step = 1;
+  while (end + step <= nd_cap && (uint32_t)(dk[end + step - 1] >> L) == v) {
+    end += step;
+    step *= 2;
+  }
+  for (int64_t hi = min(nd_cap, end + step - 1); end < hi;) {
+    const int64_t mid = (end + hi) >> 1;
+    if ((uint32_t)(dk[mid] >> L) == v) end = mid + 1;
+    else hi = mid;
+  }
+  const int32_t c = (int32_t)(end - i);
   const unsigned long long r = atomicAdd(&st->n_runs, 1ull);
   const int32_t need = used[v] + c;
-  run_start[r] = need > kLongList ? -1 - (int32_t)i : (int32_t)i;
+  runs[r] = make_int2(need > kLongList ? -1 - (int32_t)i : (int32_t)i, c);
   if (need > cap[v]) atomicAdd(&st->demand, (unsigned long long)slack_capacity(need, max(slack_q10, 256)));
 }
 
 __global__ void k_dir_runs(const uint64_t* __restrict__ dk, const int64_t nd_cap, const int L,
                            const int32_t* __restrict__ used, const int32_t* __restrict__ cap, const int32_t slack_q10,
-                           int32_t* __restrict__ run_start, BatchStatus* __restrict__ st) {
+                           int2* __restrict__ runs, BatchStatus* __restrict__ st) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd_cap; i += (int64_t)gridDim.x * blockDim.x)
-    dir_run(dk, i, nd_cap, L, used, cap, slack_q10, run_start, st);
+    dir_run(dk, i, nd_cap, L, used, cap, slack_q10, runs, st);
 }
 
 // A small batch's directed keys sorted by one CTA (padded with sentinels to 2 * cap), and their runs.
 __global__ void __launch_bounds__(kSortThreads) k_sort_runs(const uint64_t* __restrict__ dk, const int64_t cap, const int L,
                                                             uint64_t* __restrict__ sorted, const int32_t* __restrict__ used,
                                                             const int32_t* __restrict__ vcap, const int32_t slack_q10,
-                                                            int32_t* __restrict__ run_start,
-                                                            BatchStatus* __restrict__ st) {
+                                                            int2* __restrict__ runs, BatchStatus* __restrict__ st) {
   __shared__ uint64_t k[2 * kSmallBatch];
   const int64_t n = 2 * (int64_t)st->n_ins;
   const int P = pow2_at_least(n);
@@ -356,7 +366,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_runs(const uint64_t* __re
   cta_sort(k, P);
   for (int i = threadIdx.x; i < 2 * cap; i += kSortThreads) sorted[i] = i < P ? k[i] : kSentinel;
   for (int i = threadIdx.x; i < n; i += kSortThreads)
-    dir_run(k, i, n, L, used, vcap, slack_q10, run_start, st);
+    dir_run(k, i, n, L, used, vcap, slack_q10, runs, st);
 }
 
 // The long-list insertion's plan of one run (see k_long_stage).
@@ -374,10 +384,9 @@ struct LongPlan {
 constexpr int kLongChunk = 4096;  // entries per work item of the long-list kernels
 
 struct InsertArgs {
-  const uint64_t* dk;        // sorted directed keys, nd_cap of them
-  int64_t nd_cap;
+  const uint64_t* dk;        // sorted directed keys
   int L;
-  const int32_t* run_start;
+  const int2* runs;
   int64_t* start;
   int32_t* used;
   int32_t* cap;
@@ -448,26 +457,12 @@ __global__ void __launch_bounds__(kThreads) k_insert_runs(const InsertArgs I, Ba
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t nruns = (int64_t)st->n_runs;
   for (int64_t r = gw; r < nruns; r += nw) {
-    const int32_t at_run = I.run_start[r];
-    const bool is_long = at_run < 0;
-    const int64_t i0 = is_long ? -1 - at_run : at_run;
+    const int2 run = I.runs[r];
+    const bool is_long = run.x < 0;
+    const int64_t i0 = is_long ? -1 - run.x : run.x;
+    const int32_t c = run.y;
+    const int64_t i1 = i0 + c;
     const int32_t v = dir_src(I.dk[i0], I.L);
-    int64_t i1 = i0;  // run end (exclusive), found cooperatively
-    {
-      int64_t k = i0 + lane;
-      while (true) {
-        const bool same = k < I.nd_cap && I.dk[k] != kSentinel && dir_src(I.dk[k], I.L) == v;
-        __syncwarp();
-        const unsigned m = __ballot_sync(kFull, same);
-        if (m != kFull) {
-          i1 = k - lane + __ffs(~m) - 1;
-          break;
-        }
-        k += 32;
-      }
-      i1 = __shfl_sync(kFull, i1, 0);
-    }
-    const int32_t c = (int32_t)(i1 - i0);
     const int32_t a = I.used[v];
     const int64_t s_old = I.start[v];
     int64_t s_new = s_old;
@@ -858,6 +853,7 @@ __global__ void __launch_bounds__(kThreads) k_cmp_stage(
     const int32_t* __restrict__ pool, uint8_t* __restrict__ mark, int32_t* __restrict__ scr,
     int2* __restrict__ chunk, int32_t* __restrict__ used, BatchStatus* __restrict__ st) {
   __shared__ int32_t sh_wsum[kThreads / 32];
+  __shared__ int32_t sh_kept[kLongChunk];  // the chunk's kept entries, for coalesced writes
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t n_items = min((int64_t)st->cmp_items, item_cap);
   for (int64_t q = blockIdx.x; q < n_items; q += gridDim.x) {
@@ -924,7 +920,9 @@ __global__ void __launch_bounds__(kThreads) k_cmp_stage(
     int32_t at = before + incl - kept;
 #pragma unroll
     for (int t = 0; t < kCmpPer; ++t)
-      if (keepm >> t & 1u) scr[P.soff + r0 + at++] = val[t];
+      if (keepm >> t & 1u) sh_kept[at++] = val[t];
+    __syncthreads();
+    for (int32_t t = threadIdx.x; t < total; t += kThreads) scr[P.soff + r0 + t] = sh_kept[t];
     if (threadIdx.x == 0) {
       __stcg(&chunk[P.ib + (j - P.j0)], make_int2(0, total));
       __threadfence();
@@ -1866,6 +1864,7 @@ __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const 
         const uint8_t* mrk = A.mark + ss + cur + lane;
         uint32_t c = 0;
         // N(s)[cur, end), 128 entries per step: four loads per lane, and the entries' marks beside them
+        // (eight loads: 1 % slower; marks read after a hit: 7 %)
         for (int32_t left = end - cur - lane; left > -lane; left -= 128, lst += 128, mrk += 128) {
           int32_t w[4];
           uint32_t m[4];
@@ -1880,14 +1879,16 @@ __global__ void __launch_bounds__(kHubThreads, kHubCtasPerSm) k_delta_hub(const 
             const int32_t q1 = hub_lds(t.slot1(x)), q2 = hub_lds(t.slot2(x));
             const bool f = (q1 & INT32_MAX) == w[r], g = (q2 & INT32_MAX) == w[r];
             bool keep = f | g;
-            const bool ch = (f ? q1 : q2) < 0;  // (h, w) is changed
-            if (keep && (ch || m[r])) {         // or (s, w) is: the triangle is the smallest changed edge's
-              const uint64_t key_hs = ekey(h, s);
-              keep = (!ch || key_hs < ekey(h, w[r])) && (!m[r] || key_hs < ekey(s, w[r]));
-            }
             if (keep) {
-              ++c;
-              atomicAdd(&pv[w[r]], inc);
+              const bool ch = (f ? q1 : q2) < 0;  // (h, w) is changed
+              if (ch || m[r]) {  // or (s, w) is: the triangle is the smallest changed edge's
+                const uint64_t key_hs = ekey(h, s);
+                keep = (!ch || key_hs < ekey(h, w[r])) && (!m[r] || key_hs < ekey(s, w[r]));
+              }
+              if (keep) {
+                ++c;
+                atomicAdd(&pv[w[r]], inc);
+              }
             }
           }
           __syncwarp();
@@ -2023,7 +2024,7 @@ struct StreamWs {
   int2* ilist = nullptr;        // [b]
   uint64_t* dk = nullptr;       // [2b]
   uint64_t* dk2 = nullptr;      // [2b]
-  int32_t* run_start = nullptr; // [2b]
+  int2* runs = nullptr;         // [2b]
   LongPlan* long_plan = nullptr;  // [2b]
   CmpPlan* cmp_plan = nullptr;    // [2b] long lists with deletions
   // long-list insertion scratch, sized with the pool (ensure_long_scratch)
@@ -2066,7 +2067,7 @@ struct StreamWs {
 
 void StreamWs::release() {
   cudaFree(src); cudaFree(dst); cudaFree(isdel); cudaFree(keys); cudaFree(keys2);
-  cudaFree(dlist); cudaFree(ilist); cudaFree(dk); cudaFree(dk2); cudaFree(run_start);
+  cudaFree(dlist); cudaFree(ilist); cudaFree(dk); cudaFree(dk2); cudaFree(runs);
   cudaFree(long_plan); cudaFree(long_scr); cudaFree(long_smark); cudaFree(long_items);
   cudaFree(cmp_plan); cudaFree(long_chunk);
   cudaFree(ins_slot);
@@ -2157,14 +2158,14 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
   const int64_t nb = std::max<int64_t>(b, 1024);
   auto free_batch = [&w]() {
     cudaFree(w.src); cudaFree(w.dst); cudaFree(w.isdel); cudaFree(w.keys); cudaFree(w.keys2);
-    cudaFree(w.dlist); cudaFree(w.ilist); cudaFree(w.dk); cudaFree(w.dk2); cudaFree(w.run_start);
+    cudaFree(w.dlist); cudaFree(w.ilist); cudaFree(w.dk); cudaFree(w.dk2); cudaFree(w.runs);
     cudaFree(w.ins_slot); cudaFree(w.vlist); cudaFree(w.cub_tmp);
     cudaFree(w.long_plan); cudaFree(w.cmp_plan);
     w.long_plan = nullptr; w.cmp_plan = nullptr;
     cudaFree(w.hub_list); cudaFree(w.hub_off); cudaFree(w.hub_len); cudaFree(w.hub_fill); cudaFree(w.hub_chunks);
     cudaFree(w.hub_units); cudaFree(w.desc); cudaFree(w.hub_items);
     w.src = nullptr; w.dst = nullptr; w.isdel = nullptr; w.keys = nullptr; w.keys2 = nullptr;
-    w.dlist = nullptr; w.ilist = nullptr; w.dk = nullptr; w.dk2 = nullptr; w.run_start = nullptr;
+    w.dlist = nullptr; w.ilist = nullptr; w.dk = nullptr; w.dk2 = nullptr; w.runs = nullptr;
     w.ins_slot = nullptr; w.vlist = nullptr; w.cub_tmp = nullptr;
     w.hub_list = nullptr; w.hub_off = nullptr; w.hub_len = nullptr; w.hub_fill = nullptr; w.hub_chunks = nullptr;
     w.hub_units = nullptr; w.desc = nullptr; w.hub_items = nullptr;
@@ -2183,7 +2184,7 @@ tc_status ensure_stream_ws(tc_graph* g, int64_t b) {
             ::tc::dev_malloc(&w.ilist, sizeof(int2) * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.dk, sizeof(uint64_t) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.dk2, sizeof(uint64_t) * 2 * nb) == cudaSuccess &&
-            ::tc::dev_malloc(&w.run_start, sizeof(int32_t) * 2 * nb) == cudaSuccess &&
+            ::tc::dev_malloc(&w.runs, sizeof(int2) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.long_plan, sizeof(LongPlan) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.cmp_plan, sizeof(CmpPlan) * 2 * nb) == cudaSuccess &&
             ::tc::dev_malloc(&w.ins_slot, sizeof(int64_t) * 2 * nb) == cudaSuccess &&
@@ -2336,10 +2337,10 @@ void long_compact(tc_graph* g, StreamWs& w, cudaStream_t s) {
                                                g->pool, w.st);
 }
 
-// Insertion of the sorted directed keys w.dk2 (nd_cap of them) in at most `runs` runs; the scratch
+// Insertion of the sorted directed keys w.dk2, in at most `runs` runs; the scratch
 // must be sized (ensure_pool).
-void insert_sorted_keys(tc_graph* g, StreamWs& w, int64_t nd_cap, int64_t runs, int L, uint8_t* mark, cudaStream_t s) {
-  const InsertArgs I{w.dk2,      nd_cap,  L,           w.run_start,    g->start,     g->used,      g->cap,         g->pool,
+void insert_sorted_keys(tc_graph* g, StreamWs& w, int64_t runs, int L, uint8_t* mark, cudaStream_t s) {
+  const InsertArgs I{w.dk2,      L,           w.runs,    g->start,     g->used,      g->cap,         g->pool,
                      g->pool_cap, mark,    w.ins_slot,  g->d_pool_top,  g->slack_q10, w.long_plan,  w.long_items,
                      w.long_item_cap, w.scr_cap};
   k_insert_runs<<<grid_for(runs * 32, kThreads), kThreads, 0, s>>>(I, w.st);
@@ -2361,7 +2362,7 @@ cudaError_t classify_and_sort(tc_graph* g, StreamWs& w, int64_t cap, int L, cuda
   else
     k_classify<<<grid_for(cap, kThreads), kThreads, 0, s>>>(view, w.keys2, cap, L, w.dlist, w.ilist, w.dk, w.st);
   if (cap <= kSmallBatch) {
-    k_sort_runs<<<1, kSortThreads, 0, s>>>(w.dk, cap, L, w.dk2, g->used, g->cap, g->slack_q10, w.run_start, w.st);
+    k_sort_runs<<<1, kSortThreads, 0, s>>>(w.dk, cap, L, w.dk2, g->used, g->cap, g->slack_q10, w.runs, w.st);
     return cudaSuccess;
   }
   // the sentinels' low 2L bits are all ones, which no edge has (it would be a self-loop)
@@ -2369,7 +2370,7 @@ cudaError_t classify_and_sort(tc_graph* g, StreamWs& w, int64_t cap, int L, cuda
   const cudaError_t e = cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)(2 * cap), 0, 2 * L, s);
   if (e != cudaSuccess) return e;
   k_dir_runs<<<grid_for(2 * cap, kThreads), kThreads, 0, s>>>(w.dk2, 2 * cap, L, g->used, g->cap, g->slack_q10,
-                                                              w.run_start, w.st);
+                                                              w.runs, w.st);
   return cudaSuccess;
 }
 
@@ -2677,7 +2678,7 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
   // 4. insertions: merge into the lists, count on the post-insertion graph, clear marks
   if (h.n_ins > 0) {
     const int64_t ni = (int64_t)h.n_ins;
-    insert_sorted_keys(g, w, 2 * b, (int64_t)h.n_runs, L, g->mark, s);
+    insert_sorted_keys(g, w, (int64_t)h.n_runs, L, g->mark, s);
     delta_phase(g, w, sp, 1, ni, kPipeCand[default_cand(ni)], ghub, gdelta, pv_use, nullptr, kSpinNs, 0, s);
     TC_CUDA_TRY(cudaGetLastError());
   }
@@ -2746,7 +2747,7 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, L, w.dk);
   size_t tb = w.cub_bytes;
   TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, 2 * L, s));
-  k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.run_start, w.st);
+  k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.runs, w.st);
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaMemcpyAsync(&w.st_host->pool_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2754,7 +2755,7 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   g->pool_top = (int64_t)h.pool_top;
   TC_TRY(ensure_pool(g, (int64_t)h.demand, s));
   if (h.n_runs > 0) {
-    insert_sorted_keys(g, w, b, (int64_t)h.n_runs, L, nullptr, s);
+    insert_sorted_keys(g, w, (int64_t)h.n_runs, L, nullptr, s);
     TC_CUDA_TRY(cudaGetLastError());
   }
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
@@ -3016,7 +3017,7 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
     if (p->profile) cudaEventRecordWithFlags(p->pev[1], s, cudaEventRecordExternal);
     long_compact(g, w, s);
     // insertions: merge, count on the post-insertion graph, clear the marks
-    insert_sorted_keys(g, w, 2 * cap, 2 * cap, L, g->mark, s);
+    insert_sorted_keys(g, w, 2 * cap, L, g->mark, s);
     if (p->profile) cudaEventRecordWithFlags(p->pev[2], s, cudaEventRecordExternal);
     delta_phase(g, w, p->sp, 1, cap, pc, ghub, gdelta, pv, delta, p->spin_ns, p->bar_extra, s);
     if (p->profile) cudaEventRecordWithFlags(p->pev[3], s, cudaEventRecordExternal);
