@@ -178,10 +178,24 @@ __global__ void __launch_bounds__(kThreads) k_load_keys(const int32_t* __restric
 constexpr int64_t kSmallBatch = 2048;
 constexpr int kSortThreads = 1024;
 
-// Ascending bitonic sort of P (a power of two) keys in shared memory by the CTA.
+// Ascending bitonic sort of P >= 32 (a power of two) keys in shared memory by the CTA. Exchanges at a
+// distance below 32 stay in registers (shuffles), so P = 1024 takes 21 block barriers, not 55.
 __device__ __forceinline__ void cta_sort(uint64_t* __restrict__ k, const int P) {
-  for (int size = 2; size <= P; size <<= 1) {
-    for (int h = size >> 1; h > 0; h >>= 1) {
+  auto exchange = [](const uint64_t x, const int i, const int h, const int size) {
+    const uint64_t y = __shfl_xor_sync(kFull, x, h);
+    return (((i & h) == 0) == ((i & size) == 0)) == (x < y) ? x : y;  // equal keys: either
+  };
+  for (int i = threadIdx.x; i < P; i += kSortThreads) {  // P a multiple of 32: whole warps
+    uint64_t x = k[i];
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+      for (int h = size >> 1; h > 0; h >>= 1) x = exchange(x, i, h, size);
+    k[i] = x;
+  }
+  __syncthreads();
+  for (int size = 64; size <= P; size <<= 1) {
+    for (int h = size >> 1; h >= 32; h >>= 1) {
       for (int p = threadIdx.x; p < P / 2; p += kSortThreads) {
         const int i = ((p & ~(h - 1)) << 1) | (p & (h - 1)), j = i | h;
         const uint64_t x = k[i], y = k[j];
@@ -192,6 +206,13 @@ __device__ __forceinline__ void cta_sort(uint64_t* __restrict__ k, const int P) 
       }
       __syncthreads();
     }
+    for (int i = threadIdx.x; i < P; i += kSortThreads) {
+      uint64_t x = k[i];
+#pragma unroll
+      for (int h = 16; h > 0; h >>= 1) x = exchange(x, i, h, size);
+      k[i] = x;
+    }
+    __syncthreads();
   }
 }
 
@@ -828,6 +849,7 @@ __global__ void __launch_bounds__(kThreads) k_long_write(
     if (item == kNoLongItem) continue;
     const LongPlan P = plan[item >> 32];
     const int32_t k0 = (int32_t)(uint32_t)item * kLongChunk, k1 = min(P.len, k0 + kLongChunk);
+#pragma unroll 4
     for (int32_t k = k0 + (int32_t)threadIdx.x; k < k1; k += kThreads) {
       const int64_t dest = P.s_new + P.first + k;
       pool[dest] = scr[P.soff + k];
@@ -953,6 +975,7 @@ __global__ void __launch_bounds__(kThreads) k_cmp_write(
     const CmpPlan P = plan[item >> 32];
     const int32_t j = (int32_t)(uint32_t)item - P.j0;
     const int2 oc = chunk[P.ib + j];
+#pragma unroll 4
     for (int32_t t = threadIdx.x; t < oc.y; t += kThreads) pool[P.s + oc.x + t] = scr[P.soff + j * kLongChunk + t];
   }
 }
@@ -1407,13 +1430,29 @@ __device__ __forceinline__ int grab_size(const int64_t cnt) {
   return (int)max((int64_t)1, min((int64_t)kGrab, cnt / (2 * nw)));
 }
 
-// The next `grab` elements of a queue: the first, or -1 past its end.
-__device__ __forceinline__ int64_t take(unsigned long long* next, const int grab, const int64_t cnt) {
-  unsigned long long g = 0;
-  if ((threadIdx.x & 31) == 0) g = atomicAdd(next, (unsigned long long)grab);
-  g = __shfl_sync(kFull, g, 0);
-  return (int64_t)g < cnt ? (int64_t)g : -1;
-}
+// A queue of cnt elements taken `grab` at a time by the grid's warps: each warp's first piece by its
+// index, the rest from a shared counter (zero at launch). 7104 warps asking one counter for work
+// take longer than a small batch's count.
+struct Queue {
+  unsigned long long* next;
+  int64_t cnt, at, warps;
+  int grab;
+  __device__ __forceinline__ Queue(unsigned long long* n, const int64_t c) : next(n), cnt(c) {
+    warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    grab = grab_size(c);
+    at = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * grab;
+  }
+  // Advance to the next piece; `at` is past the end when there is none.
+  __device__ __forceinline__ void advance() {
+    if (cnt <= warps * grab) {
+      at = cnt;
+      return;
+    }
+    unsigned long long g = 0;
+    if ((threadIdx.x & 31) == 0) g = atomicAdd(next, (unsigned long long)grab);
+    at = warps * grab + (int64_t)__shfl_sync(kFull, g, 0);
+  }
+};
 
 // The count of the persistent kernel: the queued items of split intersections, then the other
 // described edges, one warp each. Both queues are complete before the launch (k_hub_place).
@@ -1422,9 +1461,9 @@ __device__ __forceinline__ void delta_count(const DeltaArgs& A, uint32_t* __rest
   const int lane = threadIdx.x & 31;
   const int64_t n_items = (int64_t)min(*A.split_cnt, (unsigned long long)kDeltaItems);
   const int64_t n_desc = (int64_t)*A.n_desc;
-  int grab = grab_size(n_items);
-  for (int64_t g; (g = take(A.i_next, grab, n_items)) >= 0;) {
-    const int have = (int)min((int64_t)grab, n_items - g);
+  for (Queue q(A.i_next, n_items); q.at < n_items; q.advance()) {
+    const int64_t g = q.at;
+    const int have = (int)min((int64_t)q.grab, n_items - g);
     DeltaDesc mine = {};
     int32_t i0_l = -1;
     if (lane < have) {
@@ -1443,9 +1482,9 @@ __device__ __forceinline__ void delta_count(const DeltaArgs& A, uint32_t* __rest
       delta_part(A, pv, d, i0, min(d.la, i0 + A.chunk), tri_acc);
     }
   }
-  grab = grab_size(n_desc);
-  for (int64_t g; (g = take(A.e_next, grab, n_desc)) >= 0;) {
-    const int have = (int)min((int64_t)grab, n_desc - g);
+  for (Queue q(A.e_next, n_desc); q.at < n_desc; q.advance()) {
+    const int64_t g = q.at;
+    const int have = (int)min((int64_t)q.grab, n_desc - g);
     DeltaDesc mine = {};
     if (lane < have) {
       mine = A.desc[g + lane];
@@ -1729,18 +1768,26 @@ __global__ void __launch_bounds__(kThreads) k_hub_place(const DeltaArgs A, const
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(H.n_desc, (unsigned long long)__popc(m));
     at = __shfl_sync(kFull, at, 0);
+    const unsigned long long mine = at + __popc(m & ((1u << lane) - 1u));
+    int nch = 0;  // items of a split edge
+    unsigned long long q = 0;
     if (left) {
-      const unsigned long long mine = at + __popc(m & ((1u << lane) - 1u));
       int32_t la = ls;
       if (ls > A.split_min) {
-        const int nch = (ls + A.chunk - 1) / A.chunk;
-        const unsigned long long q = atomicAdd(A.split_cnt, (unsigned long long)nch);
-        const bool fits = q + (unsigned long long)nch <= (unsigned long long)kDeltaItems;
-        for (int c = 0; c < nch && q + c < (unsigned long long)kDeltaItems; ++c)
-          A.split_items[q + c] = fits ? (mine << 24) | (unsigned long long)c : kNoItem;
-        if (fits) la |= kSplitFlag;
+        nch = (ls + A.chunk - 1) / A.chunk;
+        q = atomicAdd(A.split_cnt, (unsigned long long)nch);
+        if (q + (unsigned long long)nch <= (unsigned long long)kDeltaItems) la |= kSplitFlag;
       }
       H.desc[mine] = DeltaDesc{s, h, la, lh, A.g.start(s), A.g.start(h)};
+    }
+    __syncwarp();
+    for (unsigned split = __ballot_sync(kFull, nch > 0); split; split &= split - 1) {
+      const int k = __ffs(split) - 1;
+      const int cnt_k = __shfl_sync(kFull, nch, k);
+      const unsigned long long q_k = __shfl_sync(kFull, q, k), d_k = __shfl_sync(kFull, mine, k);
+      const bool fits = q_k + (unsigned long long)cnt_k <= (unsigned long long)kDeltaItems;
+      for (int c = lane; c < cnt_k && q_k + c < (unsigned long long)kDeltaItems; c += 32)
+        A.split_items[q_k + c] = fits ? (d_k << 24) | (unsigned long long)c : kNoItem;
     }
   }
 }
