@@ -166,7 +166,7 @@ struct Workspace {
   int64_t n_cap = 0;       // vertices
   int64_t e_cap = 0;       // oriented edge slots
   int32_t* dplus = nullptr;      // [n]
-  int64_t* offp = nullptr;       // [n+1]
+  int64_t* offp = nullptr;       // [n+1] start of N+(u) and, from bit 40 up, its length
   int32_t* indp = nullptr;       // [e_cap] N+(u) at indp[start(u) ...] (the input's own index space)
   int32_t* degv = nullptr;       // [n] deg(u)
   unsigned long long* large = nullptr;   // [item_cap] count work items (centre << 32 | first neighbour)

@@ -369,7 +369,39 @@ __host__ __device__ constexpr int pack_lanes() {
 // range just miss the hash set); longer ones are first cut to the range by two binary searches.
 constexpr int kRangeSearchMin = 32;
 
-// One warp takes the neighbours o = nbr[0 .. gcount) of centre c (out-degree a) and
+// offp[u] holds where N+(u) starts and, in its upper bits, how long it is (dplus[u], cut at
+// kHeadMax), so that a neighbour's list is looked up with one 8-byte load. The warp tiers wait on
+// chains of dependent loads (58 % of their cycles on BA n = 2^22: neighbour, out-degree, start where
+// the edge is the centre's, list); with one load for both, the first neighbours read beside the
+// entries and the centres' heads read by the chunk: BA 6.72 -> 6.05 ms, Erdos-Renyi n = 10^6 1.353 ->
+// 1.256, R-MAT 24 125.1 -> 121.4, R-MAT 20 3.95 -> 3.88. Not kept: the next centre's or group's
+// loads a step ahead (BA + 3 %, registers), neighbours' heads before the set is built (BA + 1 %).
+constexpr int kHeadShift = 40;
+constexpr int kHeadMax = (1 << 23) - 1;
+__device__ __forceinline__ int64_t head_of(const int64_t start, const int32_t a) {
+  return start | ((int64_t)min(a, kHeadMax) << kHeadShift);
+}
+__device__ __forceinline__ int64_t head_start(const int64_t head) { return head & (((int64_t)1 << kHeadShift) - 1); }
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// A lane's neighbour o (-1: none), its out-degree and its oriented list (b = 0 where there is none).
+struct Group {
+  int32_t o;
+  int b;
+  const int32_t* lst;
+};
+__device__ __forceinline__ Group fetch_group(const int32_t n, int32_t o, const int32_t* __restrict__ dplus,
+                                             const int64_t* __restrict__ offp, const int32_t* __restrict__ indp) {
+  const bool valid = o >= 0 && o < n;  // ids out of range were flagged by the orientation
+  if (!valid) o = 0;
+  const int64_t head = __ldg(offp + o);
+  int b = (int)(head >> kHeadShift);
+  if (b == kHeadMax) b = __ldg(dplus + o);
+  return {o, valid ? b : 0, indp + head_start(head)};
+}
+
+// One warp takes a group of up to 32 neighbours o of centre c (out-degree a), one per lane, and
 // intersects every edge {c, o} whose centre is c: N+(o), the shorter list (b <= a entries), goes
 // through the hash set of the staged chunk of N+(c). Per edge the scheduler picks how (table cell,
 // else the thresholds b <= lane_max, b <= packed_max):
@@ -384,22 +416,17 @@ constexpr int kRangeSearchMin = 32;
 // (CountSmem::ranged, vlo, vhi), so it holds no register across the group loop; the CTA tier
 // compiles the cut in, the warp tiers leave it out.
 template <int PV, int kCnt>
-__device__ __forceinline__ void process_group(const int32_t n, const int32_t c, const int a,
-                                              const int32_t* __restrict__ nbr, const int gcount,
+__device__ __forceinline__ void process_group(Group f, const int32_t c, const int a,
                                               const Set<kCnt>& t, const CountSmem& sm, const int lane,
-                                              const int32_t* __restrict__ dplus,
-                                              const int64_t* __restrict__ offp, const int32_t* __restrict__ indp,
                                               uint32_t* __restrict__ out, const SchedParams& sp, uint32_t& tri,
                                               uint32_t& c_acc) {
   constexpr bool kMayRange = kCnt == kHashMax * 4;  // the CTA tier
-  int32_t o = lane < gcount ? __ldg(nbr + lane) : -1;
-  const bool valid = o >= 0 && o < n;  // ids out of range were flagged by the orientation
-  if (!valid) o = 0;
-  const int b = valid ? __ldg(dplus + o) : 0;
-  const bool mine = valid && b > 0 && centre_of(c, a, o, b) &&
+  const int32_t o = f.o;
+  const int b = f.b;
+  const int32_t* lst = f.lst;
+  const bool mine = b > 0 && centre_of(c, a, o, b) &&
                     (sp.cell_filter == -1 ||
                      (sp.cell_filter >= 0 && log2_cell(a) * 16 + log2_cell(b) == sp.cell_filter));
-  const int32_t* lst = indp + (mine ? __ldg(offp + o) : 0);
   int strat = !mine ? -1
               : sp.use_table ? sp.table[log2_cell(a)][log2_cell(b)]
                              : (b <= sp.lane_max ? 1 : b <= sp.packed_max ? 2 : 0);
@@ -425,6 +452,11 @@ __device__ __forceinline__ void process_group(const int32_t n, const int32_t c, 
     }
     __syncwarp();
   }
+  // The lists are on their way from DRAM while the first ones are walked (first and last line: a
+  // packed list is seldom longer than two). BA n = 2^22 6.05 -> 5.69 ms, Erdos-Renyi n = 10^6 1.257
+  // -> 1.222, R-MAT 24 121.5 -> 121.0; R-MAT 20, whose lists are in L2, 3.883 -> 3.895.
+  if (strat >= 0) prefetch_l2(lst);
+  if (strat == 2) prefetch_l2(lst + len - 1);
   const unsigned packed = __ballot_sync(kFull, strat == 2);
   if (packed) {
     // the packed lists' fields, moved to the first lanes: lane r holds the r-th such list
@@ -512,19 +544,30 @@ __device__ __forceinline__ void warp_centre(const int32_t n, const int32_t c, co
   const WarpSet t{table, bits};
   uint32_t c_acc = 0;
   int clen = a;  // entries staged at a time: all of them, fewer only after a failed build
+  // The first neighbours and entries are in flight together, while the set is cleared.
+  int32_t nbr = lane < k1 - k0 ? __ldg(ind + start + k0 + lane) : -1;
+  const int32_t first = lane < a ? __ldg(indp + start + lane) : kNoKey;
   for (int cb = 0; cb < a; cb += clen) {
     clen = min(clen, a - cb);
     while (true) {
       clear_set(t, lane, kWarp);
       __syncwarp();
       bool ok = true;
-      for (int j = lane; j < clen; j += kWarp) ok &= insert(t, __ldg(indp + start + cb + j));
+      int j = lane;
+      if (cb == 0 && j < clen) {
+        ok = insert(t, first);
+        j += kWarp;
+      }
+      for (; j < clen; j += kWarp) ok &= insert(t, __ldg(indp + start + cb + j));
       __syncwarp();
       if (__all_sync(kFull, ok)) break;
       clen = (clen + 1) / 2;
     }
-    for (int g = k0; g < k1; g += kWarp)
-      process_group<PV>(n, c, a, ind + start + g, min(kWarp, k1 - g), t, sm, lane, dplus, offp, indp, out, sp, tri, c_acc);
+    for (int g = k0; g < k1; g += kWarp) {
+      if (g > k0 || cb > 0) nbr = lane < k1 - g ? __ldg(ind + start + g + lane) : -1;
+      const Group f = fetch_group(n, nbr, dplus, offp, indp);
+      process_group<PV>(f, c, a, t, sm, lane, out, sp, tri, c_acc);
+    }
     if (PV != TC_PV_NONE) {
       flush_set<PV>(t, lane, kWarp, out);
       __syncwarp();
@@ -581,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_count(const int32_t n,
     const int32_t c = (int32_t)(item >> 32);
     const int32_t k0 = (int32_t)(uint32_t)item;
     const int32_t a = dplus[c];
-    const int64_t start = offp[c];
+    const int64_t start = head_start(offp[c]);
     const int32_t k1 = min(degv[c], k0 + sp.cta_range);
     uint32_t c_acc = 0;
     // N+(c) in passes of at most kChunk entries, split evenly; a pass holds the entries of N+(c) in
@@ -623,8 +666,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_count(const int32_t n,
         g = __shfl_sync(kFull, g, 0);
         if (g >= ngroups) break;
         const int gk = k0 + g * kWarp;
-        process_group<PV>(n, c, a, ind + start + gk, min(kWarp, k1 - gk), L, sm, lane, dplus, offp, indp, out, sp, tri,
-                                c_acc);
+        const Group f = fetch_group(n, lane < k1 - gk ? __ldg(ind + start + gk + lane) : -1, dplus, offp, indp);
+        process_group<PV>(f, c, a, L, sm, lane, out, sp, tri, c_acc);
       }
       __syncwarp();
       __syncthreads();
@@ -656,7 +699,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_count(const int32_t n,
     const int32_t c = (int32_t)(item >> 32);
     const int32_t k0 = (int32_t)(uint32_t)item;
     const int a = __ldg(dplus + c);
-    const int64_t start = __ldg(offp + c);
+    const int64_t start = head_start(__ldg(offp + c));
     const int k1 = min(__ldg(degv + c), k0 + sp.warp_range);
     warp_centre<PV>(n, c, a, start, k0, k1, W, sm, lane, ind, dplus, offp, indp, out, sp, tri);
   }
@@ -676,17 +719,23 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_count(const int32_t n,
     for (int32_t ub = (int32_t)c0; ub < cend; ub += kWarp) {
       const int32_t uu = ub + lane;
       const bool in = uu < cend;
-      const int aa = in ? __ldg(dplus + uu) : 0;
+      const int64_t head = in ? __ldg(offp + uu) : 0;
+      const int aa = (int)(head >> kHeadShift);  // a centre of this tier has a <= warp_max < kHeadMax
       const int dd = in ? __ldg(degv + uu) : 0;
       unsigned elig = __ballot_sync(
           kFull, aa >= 1 && aa <= sp.warp_max && dd <= sp.warp_range && (!sharded || (uu >= s_lo && uu < s_hi)));
+      if (aa >= 1) {  // the rows of the chunk's later centres
+        prefetch_l2(ind + head_start(head));
+        prefetch_l2(indp + head_start(head));
+      }
       while (elig) {
         const int sl = __ffs(elig) - 1;
         elig &= elig - 1;
         const int32_t c = ub + sl;
         const int a = __shfl_sync(kFull, aa, sl);
         const int d = __shfl_sync(kFull, dd, sl);
-        warp_centre<PV>(n, c, a, __ldg(offp + c), 0, d, W, sm, lane, ind, dplus, offp, indp, out, sp, tri);
+        const int64_t start = head_start(__shfl_sync(kFull, head, sl));
+        warp_centre<PV>(n, c, a, start, 0, d, W, sm, lane, ind, dplus, offp, indp, out, sp, tri);
       }
     }
   }
@@ -763,7 +812,7 @@ __device__ __forceinline__ void finish_vertex(const int32_t u, const int32_t d, 
   const int lane = threadIdx.x & (kWarp - 1);
   if (lane == 0) {
     dplus[u] = a;
-    offp[u] = s;
+    offp[u] = head_of(s, a);
     degv[u] = d;
     if (d >= 2) acc.ei += (unsigned long long)a;
     // sum over u -> v of d+(u) + d+(v) = sum over v of d+(v) deg(v)
@@ -807,7 +856,7 @@ __global__ void __launch_bounds__(256) k_find_hubs(const View g, const int32_t n
 }
 
 // Single-pass orientation into the input's own index space: N+(u) is written at
-// indp[start(u) ...], so no offsets scan is needed (offp[u] = start(u)). A persistent grid of
+// indp[start(u) ...], so no offsets scan is needed (offp[u] = start(u) and the length). A persistent grid of
 // warps first takes hub chunks from one queue, then tiles of vertex ids from another. A hub
 // chunk is written at its own position in the hub's list; the warp that finishes a hub's last
 // chunk (a counter per hub) moves the pieces together and completes the vertex.
@@ -970,7 +1019,7 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
     // Finish the tile's vertices, one per lane (the bookkeeping of finish_vertex).
     if (own_l) {
       dplus[u_l] = a_l;
-      offp[u_l] = cap_bad ? 0 : s_l;
+      offp[u_l] = head_of(cap_bad ? 0 : s_l, a_l);
       degv[u_l] = cap_bad ? 0 : d_l;
       const int32_t dd = cap_bad ? 0 : d_l;
       if (dd >= 2) acc.ei += (unsigned long long)a_l;
@@ -1475,7 +1524,7 @@ __global__ void __launch_bounds__(256) k_cell_stats(const int32_t n, const int32
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t uu = gw; uu < n; uu += nw) {
     const int32_t du = dplus[uu];
-    const int64_t s = offp[uu];
+    const int64_t s = head_start(offp[uu]);
     for (int32_t k = lane; k < du; k += 32) {
       // the cell the count files the edge under: (centre's out-degree, the other endpoint's)
       const int32_t dv = dplus[indp[s + k]];
