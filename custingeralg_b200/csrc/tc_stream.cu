@@ -1197,55 +1197,69 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
       }
     }
   } else if (P.strat == kStratSearch) {
-    // The first five search levels come from 32 evenly spaced samples of the longer list, one
-    // per lane (a single coalesced load): a lane counts the samples below its key with
-    // shuffles, then searches memory only inside that bucket.
-    // Each lane searches two entries at once (two independent chains of loads in flight).
-    const int64_t step = ((int64_t)P.lb + 31) / 32;
-    const int32_t smp = (int64_t)lane * step < P.lb ? L[sb + (int64_t)lane * step] : INT32_MAX;
-    const int32_t s31 = __shfl_sync(kFull, smp, 31);
+    // The first seven search levels come from 128 evenly spaced samples of the longer list, four
+    // per lane in ascending order (one round of loads): a lane counts the samples below its key
+    // with shuffles, then searches memory only inside that bucket, two entries at once (two
+    // independent chains of loads in flight). Bound by the rounds of those chains and, in the
+    // fused kernel, by registers: with 32 samples, 64-bit positions and 6 CTAs an SM (40
+    // registers, 140 bytes spilled) 10^6 updates on R-MAT 22 took 9.89 ms a pass, with 32-bit positions
+    // 9.57, with 128 samples as well 9.45 (256: 9.74), and 1000 updates 1.56, 1.54, 1.50 (5 CTAs: 1.47).
+    constexpr int kS = 4;  // samples per lane
+    const int32_t* const B = L + sb;
+    const int32_t step = (int32_t)(((unsigned)P.lb + 32 * kS - 1) / (32 * kS));
+    int32_t smp[kS];
+#pragma unroll
+    for (int r = 0; r < kS; ++r) {
+      const unsigned at = (unsigned)(lane * kS + r) * (unsigned)step;
+      smp[r] = at < (unsigned)P.lb ? B[at] : INT32_MAX;
+    }
+    const int32_t s31 = __shfl_sync(kFull, smp[0], 31);
     // [lo, hi): the part of the longer list between the samples around w
-    auto bucket = [&](const int32_t w, int64_t& lo, int64_t& hi) {
-      int pos = 0;  // samples below w (they ascend with the lane)
+    auto bucket = [&](const int32_t w, const bool in, int32_t& lo, int32_t& hi) {
+      int pos = 0;  // lanes whose first sample is below w (they ascend with the lane)
 #pragma unroll
       for (int st = 16; st > 0; st >>= 1)
-        if (__shfl_sync(kFull, smp, pos + st - 1) < w) pos += st;
+        if (__shfl_sync(kFull, smp[0], pos + st - 1) < w) pos += st;
       if (pos == 31 && s31 < w) pos = 32;
-      lo = sb + (pos > 0 ? (int64_t)(pos - 1) * step + 1 : 0);
-      hi = sb + (pos < 32 ? min((int64_t)pos * step, (int64_t)P.lb) : (int64_t)P.lb);
-    };
-    for (int32_t base = i_begin; base < i_end; base += 64) {
-      const int32_t i = base + lane, i2 = i + 32;
-      const bool in = i < i_end, in2 = i2 < i_end;
-      const int32_t w = in ? L[P.sa + i] : INT32_MAX;
-      const int32_t w2 = in2 ? L[P.sa + i2] : INT32_MAX;
-      // the shorter list's marks are read beside its entries, not after a match
-      const bool ca = PRED == kPredMark && in && A.mark[P.sa + i] != 0;
-      const bool ca2 = PRED == kPredMark && in2 && A.mark[P.sa + i2] != 0;
-      int64_t lo, hi, lo2, hi2;
-      bucket(w, lo, hi);
-      bucket(w2, lo2, hi2);
+      int cnt = (pos - 1) * kS + 1;  // samples below w (below 1: none)
+#pragma unroll
+      for (int r = 1; r < kS; ++r) cnt += __shfl_sync(kFull, smp[r], pos - 1) < w;
+      if (pos == 0) cnt = 0;
+      hi = (int32_t)min((unsigned)cnt * (unsigned)step, (unsigned)P.lb);
+      lo = cnt > 0 ? min((cnt - 1) * step + 1, hi) : 0;
       if (!in) lo = hi;
-      if (!in2) lo2 = hi2;
+    };
+    const int32_t* const Q = L + P.sa;
+    const uint8_t* const MQ = A.mark + P.sa;
+    for (int32_t i = i_begin + lane; i < i_end + lane; i += 64) {
+      const bool in = i < i_end, in2 = i + 32 < i_end;
+      const int32_t w = in ? Q[i] : INT32_MAX;
+      const int32_t w2 = in2 ? Q[i + 32] : INT32_MAX;
+      // the shorter list's marks are read beside its entries, not after a match
+      const bool ca = PRED == kPredMark && in && MQ[i] != 0;
+      const bool ca2 = PRED == kPredMark && in2 && MQ[i + 32] != 0;
+      int32_t lo, hi, lo2, hi2;
+      bucket(w, in, lo, hi);
+      bucket(w2, in2, lo2, hi2);
       while (lo < hi || lo2 < hi2) {  // two lower bounds, one step of each per round
         if (lo < hi) {
-          const int64_t mid = lo + ((hi - lo) >> 1);
-          if (__ldg(L + mid) < w) lo = mid + 1;
+          const int32_t mid = (int32_t)(((unsigned)lo + (unsigned)hi) >> 1);
+          if (__ldg(B + mid) < w) lo = mid + 1;
           else hi = mid;
         }
         if (lo2 < hi2) {
-          const int64_t mid = lo2 + ((hi2 - lo2) >> 1);
-          if (__ldg(L + mid) < w2) lo2 = mid + 1;
+          const int32_t mid = (int32_t)(((unsigned)lo2 + (unsigned)hi2) >> 1);
+          if (__ldg(B + mid) < w2) lo2 = mid + 1;
           else hi2 = mid;
         }
       }
-      const bool m = in && lo < eb && L[lo] == w, m2 = in2 && lo2 < eb && L[lo2] == w2;
+      const bool m = in && lo < P.lb && B[lo] == w, m2 = in2 && lo2 < P.lb && B[lo2] == w2;
       if (PRED == kPredMark) {
-        if (m) match(ca, lo - sb, w);
-        if (m2) match(ca2, lo2 - sb, w2);
+        if (m) match(ca, lo, w);
+        if (m2) match(ca2, lo2, w2);
       } else {
-        if (m) on_match(i, lo - sb, w);
-        if (m2) on_match(i2, lo2 - sb, w2);
+        if (m) on_match(i, lo, w);
+        if (m2) on_match(i + 32, lo2, w2);
       }
     }
   } else {
@@ -1561,12 +1575,10 @@ struct PhaseEnd {
 // captured launch serves every batch of a bin. A meeting that runs out (the grid was not
 // resident, or a test forces it) sets kErrTimeout: the update still completes and the host reports
 // TC_ERR_TIMEOUT, as the batch's count may be incomplete.
-#ifndef TC_DELTA_MIN_BLOCKS
-#define TC_DELTA_MIN_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kThreads, TC_DELTA_MIN_BLOCKS) k_delta_fused(const DeltaArgs A, const PhaseEnd E,
-                                                                               uint32_t* __restrict__ pv,
-                                                                               unsigned long long* __restrict__ tri_out) {
+constexpr int kDeltaCtasPerSm = 5;  // 48 registers; 1000 updates on R-MAT 22: 6 CTAs + 2 %; 10^6: 4 CTAs + 1.3 %
+__global__ void __launch_bounds__(kThreads, kDeltaCtasPerSm) k_delta_fused(const DeltaArgs A, const PhaseEnd E,
+                                                                           uint32_t* __restrict__ pv,
+                                                                           unsigned long long* __restrict__ tri_out) {
   unsigned long long tri_acc = 0, bytes_acc = 0;
   delta_count(A, pv, tri_acc, bytes_acc);
   bytes_acc = warp_sum(bytes_acc);
