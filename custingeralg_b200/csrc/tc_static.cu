@@ -11,7 +11,7 @@
 //     id, at indp[start(u) ...], so no offsets scan is needed. Every triangle {x < y < z in
 //     that order} is found exactly once: at x, on edge x->y, as the common element z of N+(x)
 //     and N+(y). Warps take hub chunks of up to 2048 entries from one queue (the warp that
-//     finishes a hub's last chunk moves the pieces together), then tiles of 32 vertex ids from
+//     finishes a hub's last chunk moves the pieces together), then tiles of up to 32 vertex ids from
 //     another, walking a tile's concatenated lists (at most 32 x 256 entries), so neither a
 //     degree-64k hub nor a run of low-id vertices of degree 2000 (R-MAT) is one warp's serial
 //     tail. The same pass
@@ -19,7 +19,7 @@
 //     checksum for symmetry) and fills the work queues of the count.
 //  2. Counting. Every edge {c, o} is intersected once, at its centre c: the endpoint with the
 //     larger out-degree (ties to the smaller id). The centre's N+(c) is a shared-memory hash set
-//     of 4-slot buckets; the other list N+(o), the shorter one, goes through it, so the probe
+//     with two possible slots per key; the other list N+(o), the shorter one, goes through it, so the probe
 //     work is the sum over edges of min(d+u, d+v). k_count is a persistent grid; a centre walks
 //     its original neighbour list N(c) in groups of 32 and takes the neighbours it is centre
 //     for. Tiers by a = d+(c):

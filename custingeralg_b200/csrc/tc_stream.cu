@@ -6,17 +6,18 @@
 // cct_upd.cu:231-410), whose inclusion-exclusion nets +2 per vertex of every new triangle on a
 // symmetric batch (K1 counts a triangle with k new edges k times, K2 and K3 correct the
 // overcount). Here a triangle is attributed once, to the smallest of its changed edges in the
-// (min id, max id) order: k_delta intersects N(x) and N(y) for each changed edge {x, y} and keeps
+// (min id, max id) order: N(x) and N(y) are intersected for each changed edge {x, y}, which keeps
 // a common neighbour w unless (x, w) or (y, w) is a changed edge with a smaller key. Whether an
 // edge is changed comes either from a per-slot mark array parallel to the adjacency pool
 // (tc_apply_batch) or from a lookup in the sorted batch (the cuStinger-style path).
 //
-// Per changed edge the warp intersects the two full lists with a strategy chosen by their
-// lengths: binary search of the shorter list's entries into the longer ("search", for skewed
-// pairs), a partitioned merge in which each lane owns a contiguous slice of the shorter list and
-// merges it against the longer one from a binary-searched start ("merge", for balanced pairs), or,
-// where the strategy table asks for it, the longer list staged into shared memory piece by piece
-// with cp.async and searched there ("stage").
+// With marks, an edge whose longer list belongs to a hub of the batch is counted there
+// (k_delta_hub); the others by a warp each (k_delta_fused), which searches the shorter list's entries
+// in the longer one ("search") or, where the strategy table asks for it, stages the longer list into
+// shared memory piece by piece with cp.async and searches it there ("stage"). The cuStinger-style path
+// (k_delta, k_delta_split) chooses by the lengths or the table between search and, for balanced
+// pairs, a partitioned merge in which each lane owns a contiguous slice of the shorter list and
+// merges it against the longer one from a binary-searched start ("merge").
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -2897,8 +2898,8 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
 // one CUDA graph per batch-size bin instead: every launch is sized for the bin's capacity and
 // reads the batch's real counts from device memory (grid-stride loops over device counts, the
 // batch padded with sentinel keys), so a batch is one small launch that loads it and its size
-// into the bin's buffers (k_load_batch) and one graph launch, with no host synchronisation
-// inside. The delta count of each phase (deletions, insertions) is one
+// into the bin's buffers (sorted as well where one CTA can) and one graph launch, with no host
+// synchronisation inside. The delta count of each phase (deletions, insertions) is one
 // persistent kernel (k_delta_fused). The pool headroom the relocations of one batch can take is
 // bounded ahead (every touched list moving: (m + 2b)(1 + slack) slots) and reserved before the
 // launch, so the device bump allocator cannot run out. The graphs capture the graph's pool and

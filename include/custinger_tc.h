@@ -250,8 +250,8 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
  * up to max_batch, until the autotuner merges bins); each bin's graph is captured on first use
  * with launches sized for the bin and reads the batch's counts on the device. The triangle
  * delta of each phase of a batch (deletions, insertions) is one persistent kernel over a
- * resident grid: each warp runs its share of the per-edge pass, then takes the queued chunks of
- * long intersections as other warps publish them (each wait for a chunk is bounded). Pool
+ * resident grid: its warps take chunks of long intersections and whole edges from two queues filled
+ * before it starts, then its CTAs meet once (a bounded wait) and end the phase. Pool
  * headroom for the worst case of a batch (every list it touches relocating) is reserved before
  * each launch.
  *
@@ -265,7 +265,7 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
  * tc_pipeline_prepare: reserve pool headroom for max_batch and capture every bin's graph for these
  *                     outputs now (optional; otherwise both happen on first use).
  * tc_pipeline_sync:   wait for the last batch and report it (errors of that batch surface here;
- *                     TC_ERR_TIMEOUT when a delta kernel's wait for queued work ran out).
+ *                     TC_ERR_TIMEOUT when the meeting of a delta kernel's CTAs ran out).
  * tc_pipeline_autotune: explore over the next `batches` batches: each runs under one arm of its
  *                     natural bin, a candidate tile shape of the delta kernel (CTAs per SM: the
  *                     occupancy limit; split threshold / split-item size 2048/1024, 1024/512,
@@ -280,9 +280,9 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
  *                     (drops the graphs when it changes; call before tc_pipeline_prepare) and
  *                     count their algorithmic bytes, sum over changed edges {x,y} of
  *                     4 (deg x + deg y) + 8; tc_pipeline_stats returns the totals since.
- * tc_pipeline_set_wait_bound: the bound of the delta kernels' wait for queued work (default 2 s)
- *                     and a number of warps it waits for beyond the grid (0 normally; a test gives
- *                     1 to make the waits run out and checks that the batch reports
+ * tc_pipeline_set_wait_bound: the bound of the wait in which the delta kernels' CTAs meet (default
+ *                     2 s) and a number of CTAs it waits for beyond the grid (0 normally; a test
+ *                     gives 1 to make the wait run out and checks that the batch reports
  *                     TC_ERR_TIMEOUT with the device still usable). Drops the captured graphs. */
 typedef struct tc_pipeline tc_pipeline;
 typedef struct tc_pipeline_plan {
