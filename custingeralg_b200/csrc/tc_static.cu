@@ -401,6 +401,20 @@ __device__ __forceinline__ Group fetch_group(const int32_t n, int32_t o, const i
   return {o, valid ? b : 0, indp + head_start(head)};
 }
 
+// Position of the n-th (from 0) set bit of m.
+__device__ __forceinline__ int nth_bit(const unsigned m, int n) {
+  int at = 0;
+#pragma unroll
+  for (int step = kWarp / 2; step > 0; step >>= 1) {
+    const int below = __popc((m >> at) & ((1u << step) - 1u));
+    if (n >= below) {
+      n -= below;
+      at += step;
+    }
+  }
+  return at;
+}
+
 // One warp takes a group of up to 32 neighbours o of centre c (out-degree a), one per lane, and
 // intersects every edge {c, o} whose centre is c: N+(o), the shorter list (b <= a entries), goes
 // through the hash set of the staged chunk of N+(c). Per edge the scheduler picks how (table cell,
@@ -461,18 +475,7 @@ __device__ __forceinline__ void process_group(Group f, const int32_t c, const in
   if (packed) {
     // the packed lists' fields, moved to the first lanes: lane r holds the r-th such list
     const int count = __popc(packed);
-    int from = 0;  // position of the lane-th set bit of packed
-    {
-      int r = lane;
-#pragma unroll
-      for (int step = kWarp / 2; step > 0; step >>= 1) {
-        const int below = __popc((packed >> from) & ((1u << step) - 1u));
-        if (r >= below) {
-          r -= below;
-          from += step;
-        }
-      }
-    }
+    const int from = nth_bit(packed, lane);
     constexpr int kPackLanes = pack_lanes<PV>();
     const int32_t po_l = __shfl_sync(kFull, o, from);
     const int plen_l = __shfl_sync(kFull, len, from);
@@ -860,8 +863,9 @@ __global__ void __launch_bounds__(256) k_find_hubs(const View g, const int32_t n
 // warps first takes hub chunks from one queue, then tiles of vertex ids from another. A hub
 // chunk is written at its own position in the hub's list; the warp that finishes a hub's last
 // chunk (a counter per hub) moves the pieces together and completes the vertex.
+constexpr int kOrientCtasPerSm = 5;  // 48 registers (6 CTAs spill: Erdos-Renyi n = 10^6 count + 1.4 %)
 template <class View, bool kWrite>
-__global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, int32_t* __restrict__ dplus,
+__global__ void __launch_bounds__(256, kOrientCtasPerSm) k_orient(const View g, const int32_t n, int32_t* __restrict__ dplus,
                                                 int64_t* __restrict__ offp, int32_t* __restrict__ degv,
                                                 int32_t* __restrict__ indp, const int64_t e_cap,
                                                 const int32_t* __restrict__ hub_u,
@@ -934,12 +938,16 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
   }
 
   // Vertex tiles (hubs skipped: done above). The warp walks the concatenated lists of a tile's
-  // vertices (at most 32), 32 entries per step: short lists leave no lane idle, and a step is one round of
-  // coalesced loads instead of one dependent round per vertex. Lane i keeps vertex t0 + i; the
-  // owner of entry k is the last vertex whose list starts at or before k (a binary search over
-  // the lanes' exclusive prefix of the lengths). An out-neighbour's rank in N+(u) is its vertex's
-  // count from earlier steps (per-warp shared counter) plus the predecessors in its segment.
-  constexpr int kTile = 32;
+  // vertices (at most 32), 32 entries per step and two steps in flight: short lists leave no lane idle,
+  // and a step is one round of coalesced loads instead of one dependent round per vertex. Lane i
+  // keeps the i-th list that has entries. The lists that start in a step are one bit each of a word
+  // or-ed over the lanes, so an entry's owner is a population count. An out-neighbour's rank in
+  // N+(u) is the count carried from earlier steps (of the list that goes on into this one) plus the
+  // predecessors in its segment. Bound by issue (68 % on BA n = 2^22) and by the round trip to
+  // each neighbour's length. With a binary search over the lanes for the owner, one step in flight and
+  // the ranks' counters in shared memory the whole count took: R-MAT 16 215 us (now 206), Erdos-Renyi n =
+  // 10^6 1.230 ms (1.217), BA n = 2^22 5.76 ms (5.71), R-MAT 20 3.906 ms (3.895).
+  constexpr int kTile = 32, kUnr = 2;
   __shared__ int32_t s_out[256 / kWarp][kTile];
   int32_t* const my_out = s_out[threadIdx.x / kWarp];
   const unsigned lt = lanemask_lt();
@@ -969,50 +977,71 @@ __global__ void __launch_bounds__(256) k_orient(const View g, const int32_t n, i
     const int32_t excl_l = incl - len_l;
     const int32_t total = __shfl_sync(kFull, incl, kWarp - 1);
     my_out[lane] = 0;
-    __syncwarp();
+    // The lists that have entries, moved to the first lanes: where entry k = 0 of the tile would be if
+    // it were this list's, and the list's degree, lane and first k in one word.
+    const unsigned full = __ballot_sync(kFull, len_l > 0);
+    const int from = nth_bit(full, lane);
+    const int64_t c_at = __shfl_sync(kFull, s_l - excl_l, from);
+    static_assert(kHubMin <= 256 && kTile <= 32, "fields of c_word");
+    const uint32_t word_l = (uint32_t)excl_l << 14 | (uint32_t)lane << 9 | (uint32_t)(len_l & 511);
+    const uint32_t c_word = __shfl_sync(kFull, word_l, from);
+    const int32_t c_first = lane < __popc(full) ? (int32_t)(c_word >> 14) : INT32_MAX;
+    int started = 0;  // lists that started before the step
+    int carry = 0;    // out-neighbours so far of the list that goes on into the step
     int32_t last = INT32_MIN;
-    for (int32_t k0 = 0; k0 < total; k0 += kWarp) {
-      const int32_t k = k0 + lane;
-      const bool in = k < total;
-      int i = 0;  // owner lane: the largest i with excl_i <= k (its list is non-empty)
+    __syncwarp();
+    for (int32_t k0 = 0; k0 < total; k0 += kUnr * kWarp) {
+      unsigned heads[kUnr];
+      uint32_t word[kUnr];
+      int64_t at[kUnr];
+      int32_t vs[kUnr], lens[kUnr];
 #pragma unroll
-      for (int step = kWarp / 2; step > 0; step >>= 1) {
-        const int32_t e = __shfl_sync(kFull, excl_l, i + step);  // i + step <= 31
-        if (e <= k) i += step;
+      for (int j = 0; j < kUnr; ++j) {
+        const int32_t k = k0 + j * kWarp;
+        const unsigned rel = (unsigned)(c_first - k);
+        heads[j] = __reduce_or_sync(kFull, rel < kWarp ? 1u << rel : 0u);
+        const int i = started + __popc(heads[j] & (lt | (1u << lane))) - 1;
+        started += __popc(heads[j]);
+        at[j] = __shfl_sync(kFull, c_at, i);
+        word[j] = __shfl_sync(kFull, c_word, i);
+        vs[j] = k + lane < total ? g.ind[at[j] + (k + lane)] : INT32_MAX;
       }
-      const int32_t d = __shfl_sync(kFull, d_l, i);
-      const int64_t s = __shfl_sync(kFull, s_l, i);
-      const int32_t pos = k - __shfl_sync(kFull, excl_l, i);
-      const int32_t u = (int32_t)t0 + i;
-      const int32_t v = in ? g.ind[s + pos] : INT32_MAX;
-      int32_t prev = __shfl_up_sync(kFull, v, 1);
-      if (lane == 0) prev = last;
-      last = __shfl_sync(kFull, v, kWarp - 1);
-      bool pred = false;
-      if (in) {
-        if (v < 0 || v >= n) {
-          bad |= kBadRange;
-        } else {
-          if (pos > 0 && prev >= v) bad |= kBadOrder;
-          if (v == u) bad |= kBadSelfLoop;
-          pred = precedes(d, u, g.len(v), v);
-          const uint64_t h = (u < v) ? sym_hash((uint32_t)u, (uint32_t)v) : sym_hash((uint32_t)v, (uint32_t)u);
-          chk += (u < v) ? h : (0ull - h);
+#pragma unroll
+      for (int j = 0; j < kUnr; ++j) lens[j] = (uint32_t)vs[j] < (uint32_t)n ? g.len(vs[j]) : 0;
+#pragma unroll
+      for (int j = 0; j < kUnr; ++j) {
+        const bool in = k0 + j * kWarp + lane < total;
+        const bool starts = (heads[j] >> lane) & 1u;
+        const int slot = (word[j] >> 9) & 31;
+        const int32_t u = (int32_t)t0 + slot;
+        const int32_t v = vs[j];
+        int32_t prev = __shfl_up_sync(kFull, v, 1);
+        if (lane == 0) prev = last;
+        last = __shfl_sync(kFull, v, kWarp - 1);
+        bool pred = false;
+        if (in) {
+          if (v < 0 || v >= n) {
+            bad |= kBadRange;
+          } else {
+            if (!starts && prev >= v) bad |= kBadOrder;
+            if (v == u) bad |= kBadSelfLoop;
+            pred = precedes((int32_t)(word[j] & 511), u, lens[j], v);
+            const uint64_t h = (u < v) ? sym_hash((uint32_t)u, (uint32_t)v) : sym_hash((uint32_t)v, (uint32_t)u);
+            chk += (u < v) ? h : (0ull - h);
+          }
         }
+        const unsigned msk = __ballot_sync(kFull, pred);
+        const unsigned mine = heads[j] & (lt | (1u << lane));  // the lists that start up to this lane
+        const int prior = mine ? 0 : carry;
+        const unsigned seg = mine ? ~0u << (31 - __clz(mine)) : ~0u;  // from this list's first lane on
+        if (kWrite && pred) indp[at[j] + (int32_t)((word[j] >> 14) + prior + __popc(msk & lt & seg))] = v;
+        if (in && (starts || lane == 0)) {
+          const unsigned above = heads[j] & ~(lt | (1u << lane));
+          my_out[slot] = prior + __popc(msk & ~lt & (above ? (above & (0u - above)) - 1u : ~0u));
+        }
+        carry = heads[j] ? __popc(msk >> (31 - __clz(heads[j]))) : carry + __popc(msk);
+        __syncwarp();
       }
-      const unsigned msk = __ballot_sync(kFull, pred);
-      const bool head = in && (pos == 0 || lane == 0);  // first entry of its vertex in this step
-      const unsigned heads = __ballot_sync(kFull, head);
-      const int seg0 = 31 - __clz(heads & (lt | (1u << lane)));
-      const int prior = in ? my_out[i] : 0;
-      __syncwarp();
-      if (kWrite && pred) indp[s + prior + __popc(msk & lt & ~((1u << seg0) - 1u))] = v;
-      if (head) {
-        const unsigned above = heads & ~(lt | (1u << lane));
-        const unsigned below_next = above ? ((1u << (__ffs(above) - 1)) - 1u) : ~0u;
-        my_out[i] = prior + __popc(msk & below_next & ~((1u << lane) - 1u));
-      }
-      __syncwarp();
     }
     const int32_t a_l = own_l ? my_out[lane] : 0;
     __syncwarp();
