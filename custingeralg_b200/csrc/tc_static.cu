@@ -105,7 +105,8 @@ __device__ unsigned long long* tc_dbg_kern = nullptr;
 // sits beside its slot: cnt[s] counts the triangles found through the key keys[s], so a hit adds
 // to the slot it found with no indirection. A build that finds no place for an entry in kKicks
 // moves fails (at these loads that takes ids chosen against the hash), and the caller stages half
-// as many entries; two entries always fit.
+// as many entries; two entries always fit. A list that repeats an id is refused (kBadOrder), but only
+// once the count is done, so repeats must not fail builds: an entry that meets its like is dropped.
 //
 // The kernel is bound by the instructions around each lookup and by the shared-memory pipe. On R-MAT
 // 20 (1.97 G lookups, 2 t(v) per vertex): 16-byte buckets of four slots, 62 warp instructions per
@@ -209,8 +210,9 @@ template <class S>
 __device__ __forceinline__ bool insert(const S& t, int32_t key) {
   uint32_t at = t.slot1(hash_of(key));
   for (int it = 0; it < kKicks; ++it) {
-    key = exchange(at, key);
-    if (key == kFreeSlot) return true;
+    const int32_t old = exchange(at, key);
+    if (old == kFreeSlot || old == key) return true;
+    key = old;
     const uint32_t h = hash_of(key), s1 = t.slot1(h);
     at = at == s1 ? t.slot2(h) : s1;
   }

@@ -1833,12 +1833,15 @@ __device__ __forceinline__ int32_t hub_lds(const uint32_t at) {
 }
 
 // Insert a key (concurrently with others): into its first slot, the key found there into its other
-// one, and so on; false when a key is left over.
+// one, and so on; false when a key is left over. A key that meets its like is dropped, so the repeats
+// of a list that was never checked do not fail the build.
 __device__ __forceinline__ bool hub_insert(const HubSet& t, int32_t key) {
   uint32_t at = t.slot1(hub_hash(key & INT32_MAX));
   for (int it = 0; it < kHubKicks; ++it) {
-    asm volatile("atom.shared.exch.b32 %0, [%1], %0;" : "+r"(key) : "r"(at) : "memory");
-    if (key == kHubFree) return true;
+    int32_t old;
+    asm volatile("atom.shared.exch.b32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(key) : "memory");
+    if (old == kHubFree || old == key) return true;
+    key = old;
     const uint32_t x = hub_hash(key & INT32_MAX), s1 = t.slot1(x);
     at = at == s1 ? t.slot2(x) : s1;
   }
