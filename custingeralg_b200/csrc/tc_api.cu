@@ -292,7 +292,7 @@ void tc_sched_default(tc_sched* s) {
   s->lane_max_deg = 8;       // static: one lane walks each list of at most 8 entries
   s->packed_max_deg = 32;    // static: longer lists up to 32 entries walked packed
   s->blocks_per_sm = 0;
-  s->chunk = 64;
+  s->chunk = 0;              // static: vertices claimed at a time by the graph's size
   s->use_table = 0;
   s->shard = 0;
   s->nshards = 1;

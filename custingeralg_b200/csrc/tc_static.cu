@@ -1437,7 +1437,7 @@ SchedParams to_params(const tc_sched* s) {
   p.warp_max = std::min(kWarpTierMax, std::max(2, s->warp_max_deg));
   p.search_ratio_x16 = std::max(0, s->search_ratio_x16);
   p.use_table = s->use_table ? 1 : 0;
-  p.chunk = std::max(32, (s->chunk + 31) / 32 * 32);
+  p.chunk = s->chunk > 0 ? (std::min(s->chunk, 1 << 30) + 31) / 32 * 32 : 0;
   p.blocks_per_sm = std::max(0, s->blocks_per_sm);
   p.nshards = std::max(1, s->nshards);
   p.shard = std::min(std::max(0, s->shard), p.nshards - 1);
@@ -1461,10 +1461,10 @@ void set_work_sizes(SchedParams& sp, int64_t n, int64_t m, int64_t item_cap) {
   sp.cta_range = small ? 512 : 4096;
   sp.warp_range = small && item_cap >= Workspace::items_for(n, m, 64) ? 64 : 256;
   sp.hub_chunk = small ? kHubChunkMin : kHubChunk;
-  // Vertices claimed at a time: at least two claims per warp, at most 16 (64: R-MAT 20 + 2 %,
-  // Erdos-Renyi n = 2^20 + 6 %; 1: 16384 vertices + 2 %, 90601 + 25 %).
+  // Vertices claimed at a time, where the caller gives no number: at least two claims per warp, at most
+  // 16 (64: R-MAT 20 + 2 %, Erdos-Renyi n = 2^20 + 6 %; 1: 16384 vertices + 2 %, 90601 + 25 %).
   const int64_t warps = (int64_t)device_info().sms * kCtasPerSm * kWarps;
-  sp.chunk = (int32_t)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sp.chunk, 16, n / (2 * warps)}));
+  if (sp.chunk == 0) sp.chunk = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, n / (2 * warps)));
   // Orientation tiles: 32 vertices, or on a graph of fewer tiles than warps as many as hold about 128
   // entries (four steps).
   sp.tile = kWarp;

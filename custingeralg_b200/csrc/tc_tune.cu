@@ -43,7 +43,7 @@ std::vector<tc_sched> candidates() {
   const int warp_max[] = {32, 64, 128};
   // (lane_max, packed_max): lists up to lane_max walked by a lane, up to packed_max packed
   const int list_rule[][2] = {{8, 0}, {0, 64}, {4, 32}, {8, 32}, {16, 128}};
-  const int chunk[] = {32, 128};
+  const int chunk[] = {0, 32};
   const int bps[] = {0, 6};
   for (int w : warp_max)
     for (const auto& r : list_rule)

@@ -66,8 +66,9 @@ typedef struct tc_sched {
                                into the longer one when 16 d_long > ratio * d_short (log2 d_long + 1),
                                else merges */
   int32_t blocks_per_sm;  /* persistent grid = SMs x blocks_per_sm (0 = occupancy limit) */
-  int32_t chunk;          /* most vertices a warp claims per work-queue grab (graphs with few
-                             vertices per warp, and all at 16, use fewer) */
+  int32_t chunk;          /* static count: vertices a warp claims per work-queue grab, rounded up to a
+                             multiple of 32; 0 = by the graph's size (at most 16, at least two grabs
+                             a warp) */
   int32_t use_table;      /* 1 = the per-degree-cell strategy table below overrides the rules */
   uint8_t table[16][16];  /* strategy per cell [log2 d_a][log2 d_b]. Static count (a = the centre's
                              out-degree, b = the other endpoint's): 0 = the warp streams N+(b)
