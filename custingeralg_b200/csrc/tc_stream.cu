@@ -1024,9 +1024,9 @@ struct DeltaArgs {
   int nshards;
   unsigned long long* bytes_out;  // algorithmic bytes of the intersections run (NULL = not kept)
   // persistent kernel (k_delta_fused): its CTAs meet once, between the count and the update that
-  // needs the count done. arrived counts them (zero at launch). A wait that runs out reports
-  // kErrTimeout in err; bar_extra is added to the CTAs waited for (0; a test sets 1 to make the wait
-  // run out); spin_ns bounds the wait.
+  // needs the count done. arrived counts them (zero at launch; kMeetLeft). A wait that runs out
+  // reports kErrTimeout in err; bar_extra is added to the CTAs waited for (0; a test sets 1 to make the
+  // wait run out); spin_ns bounds the wait.
   unsigned* arrived;
   unsigned* err;
   unsigned bar_extra;
@@ -1513,27 +1513,47 @@ __device__ __forceinline__ void delta_count(const DeltaArgs& A, uint32_t* __rest
   }
 }
 
+// Which part of a phase's end a CTA does once the CTAs of its grid have met.
+enum : int { kShareOwn, kShareNone, kShareAll };
+constexpr unsigned kMeetLeft = 1u << 31;  // of the arrivals: a CTA left before the last one arrived
+
 // All CTAs of a resident grid meet: each waits (spin_ns of device time, at most kSpinMaxIters polls)
-// until every other has arrived. A wait that runs out sets kErrTimeout, and the CTA goes on.
-__device__ __forceinline__ void grid_meet(const DeltaArgs& A) {
+// until every other has arrived. The phase's end rewrites what the count reads, so no CTA starts on
+// it while another still counts: a CTA whose wait runs out (kErrTimeout) before the last arrival
+// leaves its share undone, and the last CTA to arrive then does all of it. kMeetLeft is set only
+// below that last arrival, in the word that counts them, so all CTAs see the same outcome.
+__device__ __forceinline__ int grid_meet(const DeltaArgs& A) {
+  __shared__ int s_share;
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned total = gridDim.x + A.bar_extra;
+    const unsigned wanted = gridDim.x + A.bar_extra;
     __threadfence();
-    atomicAdd(A.arrived, 1u);
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    for (unsigned it = 0; ld_relaxed(A.arrived) < total; ++it) {
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (it >= kSpinMaxIters || t - t0 > A.spin_ns) {
-        atomicOr(A.err, kErrTimeout);
-        break;
+    unsigned seen = atomicAdd(A.arrived, 1u) + 1u;
+    if (!(seen & kMeetLeft)) {
+      unsigned long long t0, t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+      for (unsigned it = 0; (seen & ~kMeetLeft) < wanted; ++it, seen = ld_relaxed(A.arrived)) {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (it >= kSpinMaxIters || t - t0 > A.spin_ns) {
+          atomicOr(A.err, kErrTimeout);
+          while ((seen & ~kMeetLeft) < gridDim.x) {
+            const unsigned was = atomicCAS(A.arrived, seen, seen | kMeetLeft);
+            if (was == seen) break;
+            seen = was;
+          }
+          break;
+        }
+        __nanosleep(64);
       }
-      __nanosleep(64);
+      // here either every CTA of the grid has arrived or this one has left
+      s_share = (seen & ~kMeetLeft) < gridDim.x || (seen & kMeetLeft) ? kShareNone : kShareOwn;
+    } else {
+      s_share = (seen & ~kMeetLeft) == gridDim.x ? kShareAll : kShareNone;
     }
     __threadfence();
   }
   __syncthreads();
+  return s_share;
 }
 
 // Two launches: the entry pass, then the item pass (the cuStinger-style count, tc_count_batch).
@@ -1579,8 +1599,8 @@ struct PhaseEnd {
 // per-edge count, then, once every CTA has met (grid_meet), the phase's end, so that a small
 // batch does not pay a launch for each. The batch's sizes are read from device memory, so one
 // captured launch serves every batch of a bin. A meeting that runs out (the grid was not
-// resident, or a test forces it) sets kErrTimeout: the update still completes and the host reports
-// TC_ERR_TIMEOUT, as the batch's count may be incomplete.
+// resident, or a test forces it) sets kErrTimeout, which the host reports as TC_ERR_TIMEOUT; the
+// batch's count and update still complete.
 constexpr int kDeltaCtasPerSm = 5;  // 48 registers; 1000 updates on R-MAT 22: 6 CTAs + 2 %; 10^6: 4 CTAs + 1.3 %
 __global__ void __launch_bounds__(kThreads, kDeltaCtasPerSm) k_delta_fused(const DeltaArgs A, const PhaseEnd E,
                                                                            uint32_t* __restrict__ pv,
@@ -1589,22 +1609,23 @@ __global__ void __launch_bounds__(kThreads, kDeltaCtasPerSm) k_delta_fused(const
   delta_count(A, pv, tri_acc, bytes_acc);
   bytes_acc = warp_sum(bytes_acc);
   delta_flush(tri_acc, bytes_acc, tri_out, A.bytes_out);
-  grid_meet(A);
+  const int share = grid_meet(A);
+  if (share == kShareNone) return;
+  const int64_t thread = share == kShareAll ? threadIdx.x : (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t threads = share == kShareAll ? blockDim.x : (int64_t)gridDim.x * blockDim.x;
   if (E.dlist) {
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ends = 2 * (int64_t)*E.n_del;
-    for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < ends; k += nw) {
+    for (int64_t k = thread >> 5; k < ends; k += threads >> 5) {
       const int4 d = E.dlist[k >> 1];
       compact_vertex(E.cmp, k & 1 ? d.y : d.x, E.st);
     }
   } else {
     const int64_t n = 2 * (int64_t)*E.n_ins;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = thread; i < n; i += threads) {
       const int64_t at = E.slot[i];
       if (at >= 0) E.mark[at] = 0;
     }
-    if (E.delta && blockIdx.x == 0 && threadIdx.x == 0)
-      *E.delta += (int64_t)__ldcg(E.added) - (int64_t)__ldcg(E.removed);
+    if (E.delta && thread == 0) *E.delta += (int64_t)__ldcg(E.added) - (int64_t)__ldcg(E.removed);
   }
 }
 
@@ -2468,7 +2489,7 @@ cudaError_t sort_batch(StreamWs& w, int64_t cap, int L, cudaStream_t s) {
 }
 
 // Grid of the persistent delta kernel: ctas_per_sm CTAs per SM (0 = the occupancy limit), never
-// more than can be resident at once (its item pass waits for every warp's entry pass).
+// more than can be resident at once (its CTAs meet before the phase's end).
 tc_status fused_grid(int ctas_per_sm, size_t smem, int* grid) {
   constexpr int kMaxDev = 64;
   static int occ[kMaxDev][2] = {};  // without, with the staging buffers
@@ -2765,7 +2786,8 @@ tc_status tc_apply_batch(tc_graph* g, const int32_t* src, const int32_t* dst, co
     TC_CUDA_TRY(cudaStreamSynchronize(s));
     const BatchStatus& f = *w.st_host;
     if (f.err & (kErrPool | kErrScratch)) return fail(TC_ERR_CAPACITY, "adjacency pool or insertion scratch exhausted");
-    if (f.err & kErrTimeout) return fail(TC_ERR_TIMEOUT, "the delta kernel gave up waiting for queued work");
+    if (f.err & kErrTimeout)
+      return fail(TC_ERR_TIMEOUT, "a delta kernel's CTAs did not meet in time (the batch is applied and counted)");
     info->updates = b;
     info->inserted = (int64_t)f.n_ins;
     info->deleted = (int64_t)f.n_del;
@@ -3039,7 +3061,7 @@ tc_status pipe_settle(tc_pipeline* p) {
   }
   if (f.err & kErrTimeout) {
     p->last.status = TC_ERR_TIMEOUT;
-    return fail(TC_ERR_TIMEOUT, "the delta kernel gave up waiting for queued work; the batch's count is incomplete");
+    return fail(TC_ERR_TIMEOUT, "a delta kernel's CTAs did not meet in time (the batch is applied and counted)");
   }
   return TC_OK;
 }
