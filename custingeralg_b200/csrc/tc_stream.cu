@@ -1095,7 +1095,7 @@ __device__ __forceinline__ bool delta_entry(const DeltaArgs& A, int64_t e, int32
 enum : int { kStratSearch = 0, kStratMerge = 1, kStratStage = 2 };
 constexpr int kStageEntries = 1024;  // entries of the longer list a warp stages per piece
 // Dynamic shared memory of a delta kernel launch that may stage (one buffer per warp); a launch
-// without it runs the staged cells as merges.
+// without it searches the staged cells (with marks) or merges them.
 constexpr size_t kStageSmem = sizeof(int32_t) * kStageEntries * (kThreads / 32);
 
 // The two lists of edge {x, y} as the intersection takes them: A the shorter, B the longer.
@@ -1140,7 +1140,9 @@ __device__ __forceinline__ DeltaPair delta_pair(const DeltaArgs& A, int32_t x, i
 
 // The warp intersects entries [i_begin, i_end) of the shorter list with the longer one and
 // returns (in every lane) the triangles kept there; each kept common neighbour w gets its
-// per-vertex update here, the endpoints get theirs from the caller.
+// per-vertex update here, the endpoints get theirs from the caller. With marks the lists are read by
+// plain loads: the launch rewrites them later (k_delta_fused), and the read-only path is only for what
+// no thread writes during the launch.
 template <int PRED>
 __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaPair& P, int32_t i_begin,
                                                 int32_t i_end, const uint32_t inc, uint32_t* __restrict__ pv) {
@@ -1245,12 +1247,12 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
       while (lo < hi || lo2 < hi2) {  // two lower bounds, one step of each per round
         if (lo < hi) {
           const int32_t mid = (int32_t)(((unsigned)lo + (unsigned)hi) >> 1);
-          if (__ldg(B + mid) < w) lo = mid + 1;
+          if (B[mid] < w) lo = mid + 1;
           else hi = mid;
         }
         if (lo2 < hi2) {
           const int32_t mid = (int32_t)(((unsigned)lo2 + (unsigned)hi2) >> 1);
-          if (__ldg(B + mid) < w2) lo2 = mid + 1;
+          if (B[mid] < w2) lo2 = mid + 1;
           else hi2 = mid;
         }
       }
@@ -1263,7 +1265,7 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
         if (m2) on_match(i + 32, lo2, w2);
       }
     }
-  } else {
+  } else if (PRED == kPredBatch) {
     const int32_t len = i_end - i_begin;
     const int32_t per = (len + 31) / 32;
     const int32_t i0 = i_begin + min(len, lane * per), i1 = min(i_end, i0 + per);
