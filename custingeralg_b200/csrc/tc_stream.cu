@@ -2844,7 +2844,10 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   const int L = bits_for(std::max(g->n, 2));
   k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, L, w.dk);
   size_t tb = w.cub_bytes;
-  TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, 2 * L, s));
+  // The caller says what is a duplicate, so a self-loop can come, and that of the last of 2^L ids has the
+  // sentinels' low 2L bits: one bit more keeps it in its vertex's run.
+  const int bits = 2 * L + (g->n == (int64_t)1 << L ? 1 : 0);
+  TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, bits, s));
   k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.runs, w.st);
   TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
   TC_CUDA_TRY(cudaMemcpyAsync(&w.st_host->pool_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
