@@ -59,8 +59,8 @@ def _run(cmd, verbose):
 def build_tc(force=False, verbose=False, extra=()):
     os.makedirs(BUILD, exist_ok=True)
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "**", "*.h*"),
-                                                                          recursive=True))
+    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) +
+                     glob.glob(os.path.join(INCLUDE, "**", "*.h*"), recursive=True))
     objs = []
     jobs = []
     for src in sources:

@@ -25,6 +25,7 @@
 #include <mutex>
 
 #include "tc_graph.cuh"
+#include "tc_pipe_tune.h"
 
 namespace tc {
 
@@ -2397,7 +2398,6 @@ struct PipeCand {
   int chunk;      // split-item size: entries of the shorter list
   int split_min;  // intersections whose shorter list is longer than this are split
 };
-constexpr int kPipeCands = 5;
 constexpr PipeCand kPipeCand[kPipeCands] = {
     {0, 1024, 2048}, {0, 512, 1024}, {0, 256, 512}, {0, 128, 256}, {0, 64, 128}};
 
@@ -2950,18 +2950,17 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
 // Autotuner (tc_pipeline_autotune): the bins start as a fine ladder of capacities (2^10, 2^11,
 // ... up to max_batch). Over the next k batches each batch runs under one "arm" of its natural
 // bin (the smallest that holds it): one of the candidate tile shapes of the delta kernel (CTAs
-// per SM, split threshold and split-item size) in that bin's graph, or the default shape in the
-// next bin's graph. Each arm's time per update is measured with events. At the end every bin
-// keeps its fastest shape, and a bin whose batches ran no more than 3 % slower in the next bin's
-// graph is merged into it: its threshold is dropped and its batches use that graph (fewer
-// graphs where padding costs nothing, the fine ladder where it does).
+// per SM, split threshold and split-item size) in that bin's graph, or the fastest of them so far in
+// the next bin's graph. Each arm's time per update is measured with events, the load of the batch
+// included. At the end every bin keeps its fastest shape, and a bin whose batches ran no more than
+// 3 % slower in the next bin's graph than with that shape in their own is merged into it: its
+// threshold is dropped and its batches use that graph (fewer graphs where padding costs nothing, the
+// fine ladder where it does).
 
 namespace tc {
 namespace {
 constexpr int kPipeBins = 16;
 constexpr int64_t kPipeMinBin = 1 << 10;
-constexpr int kPipeArms = kPipeCands + 1;  // + the default shape in the next bin's graph
-constexpr double kMergeSlack = 1.03;
 }  // namespace
 }  // namespace tc
 
@@ -2974,9 +2973,7 @@ struct tc_pipeline {
   int cand[tc::kPipeBins] = {};                      // chosen tile-shape candidate per bin
   int serve[tc::kPipeBins] = {};                     // bin whose graph runs this bin's batches
   cudaGraphExec_t exec[tc::kPipeBins][tc::kPipeCands] = {};
-  // autotuning: per natural bin and arm, accumulated ms per update and samples
-  double tune_ms_per_update[tc::kPipeBins][tc::kPipeArms] = {};
-  int tune_n[tc::kPipeBins][tc::kPipeArms] = {};
+  tc::BinTimes tune[tc::kPipeBins];                  // autotuning: per natural bin
   int tune_left = 0;                                 // batches still spent exploring
   // what the captured graphs hold
   const void* key_pool = nullptr;
@@ -3038,9 +3035,7 @@ tc_status pipe_settle(tc_pipeline* p) {
   if (p->timing) {
     float ms = 0.f;
     TC_CUDA_TRY(cudaEventElapsedTime(&ms, p->t0, p->t1));
-    const int bi = p->pending_nat, a = p->pending_arm;
-    p->tune_ms_per_update[bi][a] += (double)ms / (double)std::max<int64_t>(p->pending_b, 1);
-    p->tune_n[bi][a] += 1;
+    p->tune[p->pending_nat].add(p->pending_arm, (double)ms / (double)std::max<int64_t>(p->pending_b, 1));
     p->timing = false;
   }
   if (p->profile && p->prof_delta_ms >= 0.0) {
@@ -3140,29 +3135,9 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
 // End of the exploration: the fastest shape per bin, then the merges (top bin down, so a chain
 // of merged bins resolves to the graph that serves the highest of them).
 void pipe_finish_tuning(tc_pipeline* p) {
-  for (int i = 0; i < p->nbins; ++i) {
-    int best = p->cand[i];
-    double best_v = 0.0;
-    for (int j = 0; j < kPipeCands; ++j) {
-      if (p->tune_n[i][j] < 1) continue;
-      const double v = p->tune_ms_per_update[i][j] / p->tune_n[i][j];
-      if (best_v == 0.0 || v < best_v) {
-        best_v = v;
-        best = j;
-      }
-    }
-    p->cand[i] = best;
-  }
+  for (int i = 0; i < p->nbins; ++i) p->cand[i] = p->tune[i].best(p->cand[i]);
   p->serve[p->nbins - 1] = p->nbins - 1;
-  for (int i = p->nbins - 2; i >= 0; --i) {
-    p->serve[i] = i;
-    const int own = 0, up = kPipeCands;
-    if (p->tune_n[i][own] > 0 && p->tune_n[i][up] > 0) {
-      const double v_own = p->tune_ms_per_update[i][own] / p->tune_n[i][own];
-      const double v_up = p->tune_ms_per_update[i][up] / p->tune_n[i][up];
-      if (v_up <= kMergeSlack * v_own) p->serve[i] = p->serve[i + 1];
-    }
-  }
+  for (int i = p->nbins - 2; i >= 0; --i) p->serve[i] = p->tune[i].merges() ? p->serve[i + 1] : i;
 }
 
 int pipe_natural_bin(const tc_pipeline* p, int64_t b) {
@@ -3278,20 +3253,18 @@ tc_status tc_pipeline_apply(tc_pipeline* p, const int32_t* d_src, const int32_t*
   int arm = -1;
   if (p->tune_left > 0) {
     // explore: the arm of this natural bin with the fewest samples
-    arm = 0;
-    const int narms = nat + 1 < p->nbins ? kPipeArms : kPipeCands;
-    for (int j = 1; j < narms; ++j)
-      if (p->tune_n[nat][j] < p->tune_n[nat][arm]) arm = j;
+    arm = p->tune[nat].next(nat + 1 < p->nbins ? kPipeArms : kPipeCands);
     bin = arm < kPipeCands ? nat : nat + 1;
-    cand = arm < kPipeCands ? arm : 0;
+    cand = arm < kPipeCands ? arm : p->tune[nat].best(p->cand[nat]);
   }
   if (!p->exec[bin][cand]) TC_TRY(pipe_capture(p, bin, cand, pv, delta));
+  p->timing = false;
+  if (arm >= 0) TC_CUDA_TRY(cudaEventRecord(p->t0, s));
   // the batch's keys, padded to the bin's capacity, where the graph reads them
   TC_CUDA_TRY(load_batch(g, w, d_src, d_dst, d_is_delete, b, p->bin_cap[bin], bits_for(std::max(g->n, 2)), s));
-  p->timing = arm >= 0;
-  if (p->timing) TC_CUDA_TRY(cudaEventRecord(p->t0, s));
   TC_CUDA_TRY(cudaGraphLaunch(p->exec[bin][cand], s));
-  if (p->timing) TC_CUDA_TRY(cudaEventRecord(p->t1, s));
+  if (arm >= 0) TC_CUDA_TRY(cudaEventRecord(p->t1, s));
+  p->timing = arm >= 0;
   TC_CUDA_TRY(cudaEventRecord(p->done, s));
   p->pending = true;
   p->pending_bin = bin;
@@ -3335,9 +3308,10 @@ tc_status tc_pipeline_sync(tc_pipeline* p, tc_batch_info* last) {
 tc_status tc_pipeline_autotune(tc_pipeline* p, int32_t batches) {
   if (!p || batches < 0) return fail(TC_ERR_INVALID_ARG, "invalid autotune arguments");
   TC_TRY(pipe_settle(p));
-  memset(p->tune_ms_per_update, 0, sizeof(p->tune_ms_per_update));
-  memset(p->tune_n, 0, sizeof(p->tune_n));
-  for (int i = 0; i < kPipeBins; ++i) p->serve[i] = i;
+  for (int i = 0; i < kPipeBins; ++i) {
+    p->tune[i] = BinTimes();
+    p->serve[i] = i;
+  }
   p->tune_left = batches;
   return TC_OK;
 }
