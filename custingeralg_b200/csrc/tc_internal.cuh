@@ -1,6 +1,7 @@
 // Internal declarations shared by the library's translation units.
 #pragma once
 
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
@@ -28,7 +29,9 @@ constexpr int kHubChunkMin = 512;   // (on small graphs, where a chunk's chain o
 constexpr int kHubMin = 256;        // orientation: lists longer than this are oriented as hubs
 static_assert(kHubMin <= kHubChunk, "a hub has at least one chunk");
 constexpr int kWarpTierMax = 128;   // largest out-degree a single warp counts on its own
-constexpr int kItemRangeMin = 64;   // fewest neighbours of a count work item (queue sizing)
+constexpr int kItemRange = 256;     // fewest neighbours of a count work item (queue sizing)
+constexpr int kItemRangeMin = 64;   // (on small graphs)
+constexpr int64_t kSmallEdges = (int64_t)1 << 23;  // fewer directed edges: a small graph (set_work_sizes)
 
 // ---- error reporting -------------------------------------------------------------------
 
@@ -190,11 +193,17 @@ struct Workspace {
   tc_status ensure(int64_t n, int64_t m_directed, int64_t extent = -1);
   tc_status ensure_shards(int64_t n);
   void release();
-  // Hub arrays needed for a graph of m directed edges.
+  // Hub arrays needed for a graph of m directed edges, cut as set_work_sizes cuts it. Sized for every graph
+  // of fewer edges too, so a graph that loses edges is still counted without an allocation.
   static int64_t hubs_for(int64_t m) { return m / kHubMin + 1; }
-  static constexpr int64_t chunks_for(int64_t m) { return m / kHubMin + m / kHubChunkMin + 2; }
+  static constexpr int64_t chunks_for(int64_t m) {
+    return m / kHubMin + std::max(m / kHubChunk, std::min(m, kSmallEdges) / kHubChunkMin) + 2;
+  }
   // Count work items of one queue: at most one per vertex plus one per `range` neighbours.
-  static constexpr int64_t items_for(int64_t n, int64_t m, int64_t range = kItemRangeMin) { return n + m / range + 1; }
+  static constexpr int64_t items_for(int64_t n, int64_t m, int64_t range) { return n + m / range + 1; }
+  static constexpr int64_t items_for(int64_t n, int64_t m) {
+    return std::max(items_for(n, m, kItemRange), items_for(n, std::min(m, kSmallEdges), kItemRangeMin));
+  }
 };
 
 // Device properties cached per device.

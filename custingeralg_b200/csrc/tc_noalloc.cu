@@ -38,7 +38,7 @@ constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kOffStatus = 0;
 constexpr size_t kOffOffp = align256(kOffStatus + sizeof(DevStatus));
 constexpr size_t kOffDplus = align256(kOffOffp + sizeof(int64_t) * (kMaxNv + 1));
-constexpr int64_t kMaxItems = Workspace::items_for(kMaxNv, kMaxEdges, 256);
+constexpr int64_t kMaxItems = Workspace::items_for(kMaxNv, kMaxEdges, kItemRange);
 constexpr size_t kOffDegv = align256(kOffDplus + sizeof(int32_t) * (kMaxNv + 1));
 constexpr size_t kOffLarge = align256(kOffDegv + sizeof(int32_t) * (kMaxNv + 1));
 constexpr size_t kOffMedium = align256(kOffLarge + sizeof(unsigned long long) * kMaxItems);

@@ -1457,9 +1457,9 @@ SchedParams to_params(const tc_sched* s) {
 // of 8 vertices instead of 32 and hub chunks of 512 entries -> 222 us. On R-MAT 20 the same small items
 // cost 1 % and tiles of 8 nothing, on Barabasi-Albert n = 2^22 3 % and 2 %.
 void set_work_sizes(SchedParams& sp, int64_t n, int64_t m, int64_t item_cap) {
-  const bool small = m < (int64_t)1 << 23;
+  const bool small = m < kSmallEdges;
   sp.cta_range = small ? 512 : 4096;
-  sp.warp_range = small && item_cap >= Workspace::items_for(n, m, 64) ? 64 : 256;
+  sp.warp_range = small && item_cap >= Workspace::items_for(n, m, kItemRangeMin) ? kItemRangeMin : kItemRange;
   sp.hub_chunk = small ? kHubChunkMin : kHubChunk;
   // Vertices claimed at a time, where the caller gives no number: at least two claims per warp, at most
   // 16 (64: R-MAT 20 + 2 %, Erdos-Renyi n = 2^20 + 6 %; 1: 16384 vertices + 2 %, 90601 + 25 %).
