@@ -29,12 +29,22 @@ std::atomic<long long> g_alloc_cap{0};  // 0 = no cap
 }  // namespace
 
 cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
-  const long long cap = g_alloc_cap.load(std::memory_order_relaxed);
-  if (cap > 0 && (long long)bytes > cap) {
-    *p = nullptr;
-    return cudaErrorMemoryAllocation;
+  auto attempt = [&] {
+    const long long cap = g_alloc_cap.load(std::memory_order_relaxed);
+    if (cap > 0 && (long long)bytes > cap) {
+      *p = nullptr;
+      return cudaErrorMemoryAllocation;
+    }
+    return cudaMalloc(p, bytes);
+  };
+  cudaError_t e = attempt();
+  int dev = -1;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 &&
+      release_sort_ws(dev, false)) {
+    cudaGetLastError();
+    e = attempt();
   }
-  return cudaMalloc(p, bytes);
+  return e;
 }
 
 void prof_mark(int point, cudaStream_t stream) {
@@ -348,7 +358,7 @@ tc_status tc_workspace_release(void) {
   std::lock_guard<std::mutex> lk(g.mu);
   TC_CUDA_TRY(cudaDeviceSynchronize());  // no count may still use it
   g.ws[dev].release();
-  release_sort_ws(dev);
+  release_sort_ws(dev, true);
   return TC_OK;
 }
 

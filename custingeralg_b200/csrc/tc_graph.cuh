@@ -6,7 +6,6 @@
 namespace tc {
 struct StreamWs;
 void release_stream_ws(StreamWs* w);
-void release_sort_ws(int dev);  // tc_batch_sort's working memory on a device
 }  // namespace tc
 
 // Slack-managed adjacency: vertex v owns pool[start[v] .. start[v] + cap[v]); its first used[v]

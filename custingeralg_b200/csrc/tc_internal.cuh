@@ -51,12 +51,17 @@ tc_status fail(tc_status s, const char* fmt, ...);
 // Every device allocation of the library goes through dev_malloc. A test hook
 // (tc_debug_alloc_cap) makes allocations above a size fail the way cudaMalloc fails when device
 // memory runs out (cudaErrorMemoryAllocation, nothing allocated), so the out-of-memory paths can
-// be tested without exhausting a GPU.
+// be tested without exhausting a GPU. An allocation that fails is tried once more after the
+// working memory that tc_batch_sort keeps on the device, when no call uses it, has been freed.
 cudaError_t dev_malloc_bytes(void** p, size_t bytes);
 template <typename T>
 inline cudaError_t dev_malloc(T** p, size_t bytes) {
   return dev_malloc_bytes(reinterpret_cast<void**>(p), bytes);
 }
+
+// Free tc_batch_sort's working memory on a device (once the call that uses it has ended, or not at
+// all); was any freed?
+bool release_sort_ws(int dev, bool wait);
 
 #define TC_TRY(expr)                  \
   do {                                \

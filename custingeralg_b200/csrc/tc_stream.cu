@@ -21,6 +21,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
 
@@ -2634,11 +2635,17 @@ struct SortWs {
   size_t bytes() const {
     return 16 * (size_t)std::max<int64_t>(b_cap, 0) + tmp_bytes + 12 * (size_t)std::max<int64_t>(n_cap, 0);
   }
-  // n vertices, b entries; after a failure nothing is held.
+  // n vertices, b entries, and what is held already where both fit; after a failure nothing is held.
   tc_status ensure(int64_t n, int64_t b) {
     if (n <= n_cap && b <= b_cap) return TC_OK;
     const int64_t nn = std::max(n, n_cap), nb = std::max(b, b_cap);
     release();
+    if (allocate(nn, nb) || ((nn > n || nb > b) && allocate(n, b))) return TC_OK;
+    return fail(TC_ERR_OOM, "batch sort: allocation failed");
+  }
+
+ private:
+  bool allocate(int64_t nn, int64_t nb) {
     size_t tb = 0;
     const size_t bb = (size_t)std::max<int64_t>(nb, 1);
     const bool ok = ::tc::dev_malloc(&k1, sizeof(uint64_t) * bb) == cudaSuccess &&
@@ -2652,18 +2659,35 @@ struct SortWs {
     if (!ok) {
       cudaGetLastError();
       release();
-      return fail(TC_ERR_OOM, "batch sort: allocation failed");
+      return false;
     }
     tmp_bytes = tb;
     n_cap = nn;
     b_cap = nb;
-    return TC_OK;
+    return true;
   }
 };
 
+// The kept workspaces and who uses them (not a lock held through the call: the call's own allocations
+// may ask for what is kept here).
 struct SortWsPool {
-  std::mutex mu[64];
+  std::mutex mu;
+  std::condition_variable given_back;
+  bool taken[64] = {};
   SortWs ws[64];
+  bool take(int dev, bool wait) {
+    std::unique_lock<std::mutex> lk(mu);
+    if (wait) given_back.wait(lk, [&] { return !taken[dev]; });
+    if (taken[dev]) return false;
+    return taken[dev] = true;
+  }
+  void give_back(int dev) {
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      taken[dev] = false;
+    }
+    given_back.notify_all();
+  }
 };
 SortWsPool& sort_ws_pool() {
   static SortWsPool* p = new SortWsPool();  // intentionally leaked: outlives CUDA teardown
@@ -2676,13 +2700,13 @@ class SortWsLease {
  public:
   SortWsLease() {
     if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) dev_ = -1;
-    if (dev_ >= 0 && !sort_ws_pool().mu[dev_].try_lock()) dev_ = -1;
+    if (dev_ >= 0 && !sort_ws_pool().take(dev_, false)) dev_ = -1;
   }
   ~SortWsLease() {
     if (!done_) cudaDeviceSynchronize();
     SortWs& w = ws();
     if (dev_ < 0 || w.bytes() > kSortWsKeep) w.release();
-    if (dev_ >= 0) sort_ws_pool().mu[dev_].unlock();
+    if (dev_ >= 0) sort_ws_pool().give_back(dev_);
   }
   SortWsLease(const SortWsLease&) = delete;
   SortWsLease& operator=(const SortWsLease&) = delete;
@@ -2697,9 +2721,13 @@ class SortWsLease {
 
 }  // namespace
 
-void release_sort_ws(int dev) {
-  std::lock_guard<std::mutex> lk(sort_ws_pool().mu[dev]);
-  sort_ws_pool().ws[dev].release();
+bool release_sort_ws(int dev, bool wait) {
+  SortWsPool& p = sort_ws_pool();
+  if (!p.take(dev, wait)) return false;
+  const bool held = p.ws[dev].bytes() > 0;
+  p.ws[dev].release();
+  p.give_back(dev);
+  return held;
 }
 
 }  // namespace tc

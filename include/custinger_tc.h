@@ -193,7 +193,7 @@ tc_status tc_debug_alloc_cap(int64_t bytes);
 tc_status tc_workspace_status(void* stream, tc_count_info* info);
 /* Free the working memory the stateless counts (tc_count_csr32/64) and tc_batch_sort (at most
  * 256 MB) keep on the current device (it is allocated again by the next such call). Waits for the
- * device first. */
+ * device first. What tc_batch_sort keeps is also freed when an allocation of the library fails. */
 tc_status tc_workspace_release(void);
 
 /* ---- streaming updates ------------------------------------------------------------------ */
