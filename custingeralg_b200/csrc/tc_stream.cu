@@ -1605,7 +1605,11 @@ struct PhaseEnd {
 // captured launch serves every batch of a bin. A meeting that runs out (the grid was not
 // resident, or a test forces it) sets kErrTimeout, which the host reports as TC_ERR_TIMEOUT; the
 // batch's count and update still complete.
-constexpr int kDeltaCtasPerSm = 5;  // 48 registers; 1000 updates on R-MAT 22: 6 CTAs + 2 %; 10^6: 4 CTAs + 1.3 %
+#ifndef TC_DELTA_MIN_BLOCKS
+#define TC_DELTA_MIN_BLOCKS 5
+#endif
+constexpr int kDeltaCtasPerSm = TC_DELTA_MIN_BLOCKS;  // 48 registers; 1000 updates on R-MAT 22: 6 CTAs
+                                                      // + 2 %; 10^6: 4 CTAs + 1.3 %
 __global__ void __launch_bounds__(kThreads, kDeltaCtasPerSm) k_delta_fused(const DeltaArgs A, const PhaseEnd E,
                                                                            uint32_t* __restrict__ pv,
                                                                            unsigned long long* __restrict__ tri_out) {
