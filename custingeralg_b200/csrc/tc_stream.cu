@@ -2984,10 +2984,10 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
 // bin (the smallest that holds it): one of the candidate tile shapes of the delta kernel (CTAs
 // per SM, split threshold and split-item size) in that bin's graph, or the fastest of them so far in
 // the next bin's graph. Each arm's time per update is measured with events, the load of the batch
-// included. At the end every bin keeps its fastest shape, and a bin whose batches ran no more than
-// 3 % slower in the next bin's graph than with that shape in their own is merged into it: its
-// threshold is dropped and its batches use that graph (fewer graphs where padding costs nothing, the
-// fine ladder where it does).
+// included. At the end every bin keeps its fastest shape, and a bin to whose batches the padding adds no
+// more than 3 % (merge_bins) is merged into the next one: its threshold is dropped and its batches use
+// the graph that serves that bin (fewer graphs where padding costs nothing, the fine ladder where it
+// does).
 
 namespace tc {
 namespace {
@@ -3067,7 +3067,7 @@ tc_status pipe_settle(tc_pipeline* p) {
   if (p->timing) {
     float ms = 0.f;
     TC_CUDA_TRY(cudaEventElapsedTime(&ms, p->t0, p->t1));
-    p->tune[p->pending_nat].add(p->pending_arm, (double)ms / (double)std::max<int64_t>(p->pending_b, 1));
+    p->tune[p->pending_nat].add(p->pending_arm, ms, p->pending_b);
     p->timing = false;
   }
   if (p->profile && p->prof_delta_ms >= 0.0) {
@@ -3168,8 +3168,7 @@ tc_status pipe_capture(tc_pipeline* p, int bin, int cand, uint32_t* pv, int64_t*
 // of merged bins resolves to the graph that serves the highest of them).
 void pipe_finish_tuning(tc_pipeline* p) {
   for (int i = 0; i < p->nbins; ++i) p->cand[i] = p->tune[i].best(p->cand[i]);
-  p->serve[p->nbins - 1] = p->nbins - 1;
-  for (int i = p->nbins - 2; i >= 0; --i) p->serve[i] = p->tune[i].merges() ? p->serve[i + 1] : i;
+  merge_bins(p->tune, p->nbins, p->serve);
 }
 
 int pipe_natural_bin(const tc_pipeline* p, int64_t b) {

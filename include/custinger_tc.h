@@ -272,8 +272,8 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
  *                     occupancy limit; split threshold / split-item size 2048/1024, 1024/512,
  *                     512/256, 256/128 or 128/64 entries) or its fastest shape so far in the next
  *                     bin's graph, timed with events. Afterwards each bin keeps its fastest shape, and a
- *                     bin whose batches ran at most 3 % slower in the next bin's graph is merged into
- *                     it (its threshold dropped).
+ *                     bin is merged into the next one (its threshold dropped) where the graph that
+ *                     serves that one adds at most 3 % to its batches' time.
  * tc_pipeline_info:   bins, their capacities and the delta-kernel CTAs per SM each uses.
  * tc_pipeline_plan_get / _set: the tuned bins and shapes, to carry a tuning over to another
  *                     pipeline with the same max_batch (e.g. tuned on a copy of the graph).
