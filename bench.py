@@ -612,7 +612,7 @@ def run_ours(a, rank, world, local_rank):
     if not a.no_streaming:
         result["streaming"] = run_streaming(ctx, a.stream_sched)
         if not a.no_fixed and a.stream_sched != "fixed":
-            fx = run_streaming(ctx, "fixed", verify_every=10)
+            fx = run_streaming(ctx, "fixed")
             result["streaming"]["fixed"] = {k: fx[k] for k in ("value", "ms_total", "updates", "recount_checks",
                                                                   "scheduler", "delta_kernel_ms")}
             result["streaming"]["fixed"]["learned_over_fixed"] = round(result["streaming"]["value"] / fx["value"], 4)
@@ -720,13 +720,13 @@ def tune_pipeline(base, max_b, sched, scale, dev, per_arm=2, small_per_arm=6, sm
     return plan
 
 
-def run_streaming(ctx, sched_kind, verify_every=None):
+def run_streaming(ctx, sched_kind):
     """Update edges per second on R-MAT scale 22 (seed 4) with 200 uneven batches; the running
     count is checked against a full static recount after every batch (outside the timing)."""
     import torch
     from custingeralg_b200 import api, generators as G, native as N
     a, dev = ctx.a, ctx.dev
-    verify_every = a.stream_verify if verify_every is None else verify_every
+    verify_every = a.stream_verify
     base = rmat_graph(ctx, a.stream_scale, 16, 4)
     graph = api.Graph.from_csr(base, slack=0.25)
     pv = torch.zeros(base.n + 1, dtype=torch.int32, device=dev)
@@ -738,7 +738,7 @@ def run_streaming(ctx, sched_kind, verify_every=None):
     dbat = [(torch.from_numpy(s).to(dev), torch.from_numpy(d).to(dev), torch.from_numpy(x).to(dev))
             for s, d, x in batches]
     sched = N.default_sched()
-    sched_desc = "fixed rule (search when 16 d_long > 16 d_short (log2 d_long + 1))"
+    sched_desc = "fixed rule (every edge that no hub takes is searched)"
     if sched_kind == "learned":
         from custingeralg_b200 import sched_learn as L
         if os.path.exists(L.STREAM_WEIGHTS):

@@ -57,7 +57,8 @@ namespace {
 constexpr int kThreads = 128;      // 4 warps: a CTA's warps wait for one another at each item's end
                                    // (256 threads on the same table: 6 % slower on R-MAT 20)
 constexpr int kWarps = kThreads / kWarp;
-constexpr int kCtasPerSm = 10;     // k_count: 48 registers a thread (12 CTAs at 40 spill: R-MAT 24 + 19 %,
+constexpr int kCtasPerSm = 10;     // k_count: 48 registers a thread, 56 to 80 bytes of them spilled with
+                                   // per-vertex output (12 CTAs at 40 spill more: R-MAT 24 + 19 %,
                                    // BA n = 2^22 + 24 %; 8 CTAs: R-MAT 20 + 8 %)
 constexpr int kHashMaxBits = 11;
 constexpr int kHashMax = 1 << kHashMaxBits;  // hash slots of the CTA tier's table
@@ -118,9 +119,8 @@ constexpr int32_t kNoKey = -2;  // an entry that is not there: equals no slot's 
 constexpr int kKicks = 64;
 
 // Dynamic shared memory of k_count: the tables, then CountSmem. Tables are addressed by 32-bit
-// shared addresses and read and updated with inline ld.shared / red.shared: through C++ pointers
-// the compiler recomputes the block's shared window (a special-register read and two uniform
-// instructions) next to every few accesses.
+// shared addresses and read and updated with inline ld.shared / red.shared, so that a slot's address
+// is 32-bit arithmetic on the hash.
 constexpr int kWarpTableBytes = kTableBytes / kWarps;
 extern __shared__ __align__(16) unsigned char smem_raw[];
 
@@ -136,7 +136,7 @@ struct CountSmem {
 constexpr size_t kCountSmem = kTableBytes + sizeof(CountSmem);
 
 __device__ __forceinline__ uint32_t table_base() {
-  uint32_t base;  // kept in a register: the compiler cannot recompute a volatile result
+  uint32_t base;  // volatile, so that it is computed once
   asm volatile("mov.u32 %0, %1;" : "=r"(base) : "r"((uint32_t)__cvta_generic_to_shared(smem_raw)));
   return base;
 }
@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(256) k_find_hubs(const View g, const int32_t n
 // warps first takes hub chunks from one queue, then tiles of vertex ids from another. A hub
 // chunk is written at its own position in the hub's list; the warp that finishes a hub's last
 // chunk (a counter per hub) moves the pieces together and completes the vertex.
-constexpr int kOrientCtasPerSm = 5;  // 48 registers (6 CTAs spill: Erdos-Renyi n = 10^6 count + 1.4 %)
+constexpr int kOrientCtasPerSm = 5;  // 48 registers, 8 bytes spilled (6 CTAs: Erdos-Renyi n = 10^6 count + 1.4 %)
 template <class View, bool kWrite>
 __global__ void __launch_bounds__(256, kOrientCtasPerSm) k_orient(const View g, const int32_t n, int32_t* __restrict__ dplus,
                                                 int64_t* __restrict__ offp, int32_t* __restrict__ degv,
@@ -947,8 +947,9 @@ __global__ void __launch_bounds__(256, kOrientCtasPerSm) k_orient(const View g, 
   // N+(u) is the count carried from earlier steps (of the list that goes on into this one) plus the
   // predecessors in its segment. Bound by issue (68 % on BA n = 2^22) and by the round trip to
   // each neighbour's length. With a binary search over the lanes for the owner, one step in flight and
-  // the ranks' counters in shared memory the whole count took: R-MAT 16 215 us (now 206), Erdos-Renyi n =
-  // 10^6 1.230 ms (1.217), BA n = 2^22 5.76 ms (5.71), R-MAT 20 3.906 ms (3.895).
+  // the ranks' counters in shared memory the whole count took, both timed in one call: R-MAT 16 215 us
+  // (with it 206), Erdos-Renyi n = 10^6 1.230 ms (1.217), BA n = 2^22 5.76 ms (5.71), R-MAT 20 3.906 ms
+  // (3.895).
   constexpr int kTile = 32, kUnr = 2;
   __shared__ int32_t s_out[256 / kWarp][kTile];
   int32_t* const my_out = s_out[threadIdx.x / kWarp];

@@ -34,7 +34,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr uint64_t kSentinel = ~0ull;
-constexpr int kLongList = 2048;  // lists longer than this are rewritten by a whole CTA
+constexpr int kLongList = 2048;  // lists longer than this are rewritten in pieces, by many CTAs
 constexpr int64_t kDeltaItems = 1 << 20;  // capacity of the split-item queue
 constexpr unsigned long long kNoItem = ~0ull;
 constexpr int kGrab = 4;  // most changed edges a warp takes per grab from the delta kernel's queue
@@ -60,7 +60,7 @@ struct BatchStatus {
   unsigned long long dir_added;   // directed entries inserted (cuStinger path)
   unsigned long long dir_removed; // directed entries deleted (cuStinger path)
   unsigned long long not_fitting;
-  unsigned long long n_long;      // insertion runs whose list is long (k_long_plan)
+  unsigned long long n_long;      // insertion runs whose list is long (plan_long_run)
   unsigned long long long_scr;    // scratch entries and work items of the long-list insertion
   unsigned long long long_items;
   unsigned long long n_cmp;       // long lists compacted, their scratch entries and work items
@@ -76,7 +76,7 @@ struct BatchStatus {
   unsigned long long hub_q[2];    // work-queue heads of the hub kernel
   unsigned long long hub_items[2];  // hub work items queued
   unsigned long long n_desc[2];   // changed edges left to the per-edge kernel
-  unsigned long long e_next[2];   // work-queue heads of the delta kernel's entry and item passes
+  unsigned long long e_next[2];   // work-queue heads of the delta kernel's edges and of its split items
   unsigned long long i_next[2];
 };
 
@@ -1208,7 +1208,8 @@ __device__ __forceinline__ uint32_t delta_range(const DeltaArgs& A, const DeltaP
     // independent chains of loads in flight). Bound by the rounds of those chains and, in the
     // fused kernel, by registers: with 32 samples, 64-bit positions and 6 CTAs an SM (40
     // registers, 140 bytes spilled) 10^6 updates on R-MAT 22 took 9.89 ms a pass, with 32-bit positions
-    // 9.57, with 128 samples as well 9.45 (256: 9.74), and 1000 updates 1.56, 1.54, 1.50 (5 CTAs: 1.47).
+    // 9.57, with 128 samples as well 9.45 (256: 9.74), and 1000 updates 1.56, 1.54, 1.50 (5 CTAs: 1.47;
+    // one call's figures: the same pass takes 1.5 to 1.6 ms from call to call).
     constexpr int kS = 4;  // samples per lane
     const int32_t* const B = L + sb;
     const int32_t step = (int32_t)(((unsigned)P.lb + 32 * kS - 1) / (32 * kS));
@@ -1382,7 +1383,7 @@ __device__ __forceinline__ void batch_entries(const DeltaArgs& A, uint32_t* __re
 }
 
 // Its queued chunks, one warp per item (the second launch). An item's edge passed every check of
-// the entry pass; its endpoints' per-vertex updates and the total add up per chunk.
+// the first; its endpoints' per-vertex updates and the total add up per chunk.
 __device__ __forceinline__ void batch_items(const DeltaArgs& A, uint32_t* __restrict__ pv, const int64_t gw,
                                             const int64_t nw, unsigned long long& tri_acc) {
   const int lane = threadIdx.x & 31;
@@ -1560,7 +1561,7 @@ __device__ __forceinline__ int grid_meet(const DeltaArgs& A) {
   return s_share;
 }
 
-// Two launches: the entry pass, then the item pass (the cuStinger-style count, tc_count_batch).
+// Two launches: the edges, then the items of the split ones (the cuStinger-style count, tc_count_batch).
 // Bound by chains of dependent loads, so warps in flight count for more than the few spills that 32
 // registers cost. Both directions of present edges of R-MAT 20, counted for deletion, with 6 CTAs an SM
 // under a grid of 8 -> 8 CTAs -> and a grid of up to 32 (5 CTAs: + 3 %): 19,996 entries 158 -> 147 -> 141 us,
@@ -2533,7 +2534,8 @@ tc_status hub_grid(int* grid) {
   return TC_OK;
 }
 
-// Phases of at most this many changed edges take none of the hub kernels' four launches.
+// Phases of at most this many changed edges form no hub groups, which saves three launches (k_hub_count,
+// k_hub_alloc and k_delta_hub; k_hub_place describes the edges in any case).
 constexpr int64_t kHubBatchMin = kSmallBatch;
 
 // Hub groups and their count for one phase of a batch (deletions: phase 0, insertions: 1) on a
@@ -3015,7 +3017,7 @@ struct tc_pipeline {
   uint64_t key_ws = 0;
   int64_t key_pool_cap = 0;
   tc::SchedParams sp;
-  unsigned long long spin_ns = tc::kSpinNs;          // bound of the delta kernel's barrier wait
+  unsigned long long spin_ns = tc::kSpinNs;          // bound of the wait in which the delta kernels' CTAs meet
   unsigned bar_extra = 0;                            // (test hook: arrivals that never come)
   cudaStream_t cs = nullptr;     // capture stream
   tc::BatchStatus* h_st = nullptr;          // pinned: status of the last batch

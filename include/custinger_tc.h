@@ -62,9 +62,9 @@ enum { TC_MEM_DEVICE = 0, TC_MEM_HOST = 1 };
 typedef struct tc_sched {
   int32_t warp_max_deg;   /* static count: a centre (the edge endpoint whose N+ is hashed) with
                              out-degree up to this is counted by one warp (<= 128), above by a CTA */
-  int32_t search_ratio_x16; /* streaming delta count: edge {x,y} binary-searches the shorter list
-                               into the longer one when 16 d_long > ratio * d_short (log2 d_long + 1),
-                               else merges */
+  int32_t search_ratio_x16; /* tc_count_batch: edge {x,y} binary-searches the shorter list into the
+                               longer one when 16 d_long > ratio * d_short (log2 d_long + 1), else
+                               merges. tc_apply_batch and tc_pipeline never merge */
   int32_t blocks_per_sm;  /* persistent grid = SMs x blocks_per_sm (0 = occupancy limit) */
   int32_t chunk;          /* static count: vertices a warp claims per work-queue grab, rounded up to a
                              multiple of 32; 0 = by the graph's size (at most 16, at least two grabs
@@ -73,7 +73,8 @@ typedef struct tc_sched {
   uint8_t table[16][16];  /* strategy per cell [log2 d_a][log2 d_b]. Static count (a = the centre's
                              out-degree, b = the other endpoint's): 0 = the warp streams N+(b)
                              through the hash set, 1 = one lane walks it, 2 = packed (see
-                             packed_max_deg). Streaming: 0 = search, 1 = merge, 2 = stage (the
+                             packed_max_deg). Streaming: 0 = search, 1 = merge (tc_count_batch;
+                             tc_apply_batch and tc_pipeline search there too), 2 = stage (the
                              longer list copied into shared memory in pieces with cp.async, each
                              shorter-list entry binary-searched there) */
   int32_t shard;          /* multi-GPU work split (1 = everything): this call counts shard `shard` of */
@@ -94,7 +95,9 @@ typedef struct tc_sched {
   int32_t stream_hub_min; /* streaming delta count (tc_apply_batch, tc_pipeline): changed edges whose
                              longer-list endpoint holds at least this many of a batch phase's
                              changed edges are counted together at that endpoint, its list hashed
-                             once in shared memory (0 = never; every edge on its own) */
+                             once in shared memory (0 = never; every edge on its own). Phases of at
+                             most 2048 changed edges, in a pipeline batches of bins up to that
+                             capacity, count every edge on its own whatever the value */
 } tc_sched;
 
 typedef struct tc_graph tc_graph;
@@ -266,7 +269,8 @@ tc_status tc_count_batch(tc_graph* g, const int32_t* d_src, const int32_t* d_dst
  * tc_pipeline_prepare: reserve pool headroom for max_batch and capture every bin's graph for these
  *                     outputs now (optional; otherwise both happen on first use).
  * tc_pipeline_sync:   wait for the last batch and report it (errors of that batch surface here;
- *                     TC_ERR_TIMEOUT when the meeting of a delta kernel's CTAs ran out).
+ *                     TC_ERR_TIMEOUT when the meeting of a delta kernel's CTAs ran out; the batch
+ *                     is then applied and counted all the same).
  * tc_pipeline_autotune: explore over the next `batches` batches: each runs under one arm of its
  *                     natural bin, a candidate tile shape of the delta kernel (CTAs per SM: the
  *                     occupancy limit; split threshold / split-item size 2048/1024, 1024/512,
