@@ -44,6 +44,7 @@ constexpr unsigned long long kSpinNs = 2000000000ull;  // 2 s
 constexpr unsigned kSpinMaxIters = 1u << 24;
 
 enum : unsigned { kErrRange = 1u, kErrPool = 2u, kErrTimeout = 4u, kErrScratch = 8u };
+constexpr unsigned kLastSelfLoop = 16u;  // not an error: an entry with the sentinels' low bits (tc_insert_sorted)
 // first_del[v] between batches: no deletion marked in v's list (0x7f7f7f7f, a byte memset)
 constexpr int32_t kNoDel = 0x7f7f7f7f;
 constexpr unsigned long long kNoLongItem = ~0ull;
@@ -2057,7 +2058,8 @@ __global__ void k_unpack_dir(const uint64_t* __restrict__ keys, const int64_t b,
 // Entries with dup == 0 that are already in the graph become duplicates; the rest are packed
 // as directed insertion keys (sentinel elsewhere).
 __global__ void k_flag_present(const SlackView g, const int32_t* __restrict__ s, const int32_t* __restrict__ d,
-                               int32_t* __restrict__ dup, const int64_t b, const int L, uint64_t* __restrict__ dk) {
+                               int32_t* __restrict__ dup, const int64_t b, const int L, uint64_t* __restrict__ dk,
+                               BatchStatus* __restrict__ st) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b; i += (int64_t)gridDim.x * blockDim.x) {
     uint64_t k = kSentinel;
     if (!dup[i]) {
@@ -2067,6 +2069,7 @@ __global__ void k_flag_present(const SlackView g, const int32_t* __restrict__ s,
       const int64_t p = lower_bound(g.ind, sx, sx + lx, y);
       if (p < sx + lx && g.ind[p] == y) dup[i] = 1;
       else k = ((uint64_t)(uint32_t)x << L) | (uint32_t)y;
+      if (k == (1ull << (2 * L)) - 1) atomicOr(&st->err, kLastSelfLoop);
     }
     dk[i] = k;
   }
@@ -2876,16 +2879,19 @@ tc_status tc_insert_sorted(tc_graph* g, const int32_t* d_src, const int32_t* d_d
   // entries come sorted by (src, dst): the packed keys of the new ones stay sorted, sentinel
   // elsewhere; sort once more to push the sentinels to the end.
   const int L = bits_for(std::max(g->n, 2));
-  k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, L, w.dk);
-  size_t tb = w.cub_bytes;
-  // The caller says what is a duplicate, so a self-loop can come, and that of the last of 2^L ids has the
-  // sentinels' low 2L bits: one bit more keeps it in its vertex's run.
-  const int bits = 2 * L + (g->n == (int64_t)1 << L ? 1 : 0);
-  TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, bits, s));
-  k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.runs, w.st);
-  TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
-  TC_CUDA_TRY(cudaMemcpyAsync(&w.st_host->pool_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  TC_CUDA_TRY(cudaStreamSynchronize(s));
+  k_flag_present<<<grid_for(b, kThreads), kThreads, 0, s>>>(view, d_src, d_dst, d_dup, b, L, w.dk, w.st);
+  for (int bits = 2 * L;; ++bits) {
+    size_t tb = w.cub_bytes;
+    TC_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w.cub_tmp, tb, w.dk, w.dk2, (int)b, 0, bits, s));
+    k_dir_runs<<<grid_for(b, kThreads), kThreads, 0, s>>>(w.dk2, b, L, g->used, g->cap, g->slack_q10, w.runs, w.st);
+    TC_CUDA_TRY(cudaMemcpyAsync(w.st_host, w.st, sizeof(BatchStatus), cudaMemcpyDeviceToHost, s));
+    TC_CUDA_TRY(cudaMemcpyAsync(&w.st_host->pool_top, g->d_pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    TC_CUDA_TRY(cudaStreamSynchronize(s));
+    // The caller says what is a duplicate, so a self-loop can come, and that of the last of 2^L ids has the
+    // sentinels' low 2L bits: it may lie apart from its vertex's run. Then once more with one bit more.
+    if (!(w.st_host->err & kLastSelfLoop) || bits > 2 * L) break;
+    TC_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(BatchStatus), s));
+  }
   const BatchStatus h = *w.st_host;
   g->pool_top = (int64_t)h.pool_top;
   TC_TRY(ensure_pool(g, (int64_t)h.demand, s));
